@@ -29,25 +29,25 @@ def listed():
     return [
         # The smallest structure an edit leaves behind, at the defaults of the drop-in call: all
         # latency and launches.
-        dict(name="piece 8, fp64", kind="solve", world=1, nx=8, ny=8, nz=8, k="uniform", precision="fp64", tol=1e-6, host=False),
+        dict(name="piece 8 fp64", kind="solve", world=1, nx=8, ny=8, nz=8, k="uniform", precision="fp64", tol=1e-6, host=False),
         # The plain FP64 solve of the benchmark's small configuration.
-        dict(name="piece 32, fp64", kind="solve", world=1, nx=32, ny=32, nz=32, k="uniform", precision="fp64", tol=1e-8,
+        dict(name="piece 32 fp64", kind="solve", world=1, nx=32, ny=32, nz=32, k="uniform", precision="fp64", tol=1e-8,
              host=False),
         # A ragged building-sized piece in host arrays, as a caller without device buffers has it.
-        dict(name="piece 61x45x37, mixed", kind="solve", world=1, nx=61, ny=45, nz=37, k="lognormal", precision="mixed",
+        dict(name="piece 61x45x37 mixed", kind="solve", world=1, nx=61, ny=45, nz=37, k="lognormal", precision="mixed",
              tol=1e-8, host=True),
         # The headline piece in each precision, inputs and motions in device memory.
-        dict(name="piece 128, fp64", kind="solve", world=1, nx=128, ny=128, nz=128, k="uniform", precision="fp64", tol=1e-8,
+        dict(name="piece 128 fp64", kind="solve", world=1, nx=128, ny=128, nz=128, k="uniform", precision="fp64", tol=1e-8,
              host=False),
-        dict(name="piece 128, mixed", kind="solve", world=1, nx=128, ny=128, nz=128, k="uniform", precision="mixed", tol=1e-8,
+        dict(name="piece 128 mixed", kind="solve", world=1, nx=128, ny=128, nz=128, k="uniform", precision="mixed", tol=1e-8,
              host=False),
         # The largest piece of the range, edges that are no powers of two.
-        dict(name="piece 167x160x150, mixed", kind="solve", world=1, nx=167, ny=160, nz=150, k="lognormal", precision="mixed",
+        dict(name="piece 167x160x150 mixed", kind="solve", world=1, nx=167, ny=160, nz=150, k="lognormal", precision="mixed",
              tol=1e-8, host=False),
         # Many uneven pieces in one call, sized as the benchmark's batch draws them.
-        dict(name="batch 64, mixed", kind="batch", world=1, pieces=64, most=64, precision="mixed", tol=1e-8),
+        dict(name="batch 64 mixed", kind="batch", world=1, pieces=64, most=64, precision="mixed", tol=1e-8),
         # Forward and backward: the compliance and its gradient by every cell's stiffness.
-        dict(name="adjoint 96, fp64", kind="adjoint", world=1, nx=96, ny=96, nz=96, k="uniform", precision="fp64", tol=1e-8),
+        dict(name="adjoint 96 fp64", kind="adjoint", world=1, nx=96, ny=96, nz=96, k="uniform", precision="fp64", tol=1e-8),
         # The drop-in call for any lattice, at the reference's tolerance.
         dict(name="lattice 28", kind="motions", world=1, nx=28, ny=28, nz=28, tol=1e-6),
         # The reference's caller of it: rounds of solving and breaking until nothing breaks.
