@@ -20,10 +20,11 @@ Emitted:
                            `axis` meets (as the + face of its lesser cell, slot 2*axis+1,
                            and as the - face of its greater cell, slot 2*axis), with the
                            zero entries left out, for double and float;
-  * JAC_V / JAC_L          for each axis, V and lambda with V' M- V = I and V' M+ V = diag(lambda),
-                           M+ / M- the own blocks of slots 2*axis+1 / 2*axis: a face node's
-                           diagonal block k_A M+ + k_B M- then inverts as
-                           V diag(1 / (k_A lambda + k_B)) V'.
+  * Jac<axis>              unrolled products with V and V', and lambda, where V' M- V = I and
+                           V' M+ V = diag(lambda), M+ / M- the own blocks of slots 2*axis+1 /
+                           2*axis: a face node's diagonal block k_A M+ + k_B M- then inverts
+                           as V diag(1 / (k_A lambda + k_B)) V'. Entries that are exactly
+                           zero are left out.
 
 Run: python gen_template.py > template_gen.cuh (build() does it when the file is absent).
 """
@@ -116,21 +117,26 @@ def emit(K, fac):
     for i in range(36):
         w("  {" + ", ".join(lit(K[i, j]) for j in range(36)) + "},\n")
     w("};\n\n")
-    # Jacobi factors
-    w("static const double JAC_V_HOST[3][6][6] = {\n")
-    for V, _ in fac:
-        w("  {" + ", ".join("{" + ", ".join(lit(V[i, j]) for j in range(6)) + "}" for i in range(6)) + "},\n")
-    w("};\nstatic const double JAC_L_HOST[3][6] = {\n")
-    for _, lam in fac:
-        w("  {" + ", ".join(lit(x) for x in lam) + "},\n")
-    w("};\n")
-    w("__constant__ double JAC_V_DEV[3][6][6] = {\n")
-    for V, _ in fac:
-        w("  {" + ", ".join("{" + ", ".join(lit(V[i, j]) for j in range(6)) + "}" for i in range(6)) + "},\n")
-    w("};\n__constant__ double JAC_L_DEV[3][6] = {\n")
-    for _, lam in fac:
-        w("  {" + ", ".join(lit(x) for x in lam) + "},\n")
-    w("};\n\n")
+    # Jacobi factors: literals of the vectors' type (a table in constant memory holds doubles,
+    # which an FP32 kernel would convert entry by entry, every time)
+    w("template <int AX>\nstruct Jac;\n")
+    for ax, (V, lam) in enumerate(fac):
+        w(f"template <>\nstruct Jac<{ax}> {{\n")
+        for name, M in (("vt", V.T), ("v", V)):
+            w(f"  template <class T>\n  __device__ __forceinline__ static void {name}(const T (&x)[6], T (&y)[6]) {{\n")
+            for i in range(6):
+                w("    { T s = T(0);\n")
+                for j in range(6):
+                    if M[i, j] != 0.0:
+                        w(f"      s = fma(T({lit(M[i, j])}), x[{j}], s);\n")
+                w(f"      y[{i}] = s; }}\n")
+            w("  }\n")
+        w("  template <class T>\n  __device__ __forceinline__ static T lambda(int i) {\n")
+        w("    switch (i) {\n")
+        for i in range(5):
+            w(f"      case {i}: return T({lit(lam[i])});\n")
+        w(f"      default: return T({lit(lam[5])});\n    }}\n  }}\n}};\n")
+    w("\n")
     # stencil strips: y += sum_b T[slot][b] * xs[b], xs[b] the six node vectors of the cell
     for slot in range(6):
         w(f"// Row strip of face slot {slot}: acc[i] += sum_b sum_j TPL[6*{slot}+i][6*b+j] * x[b][j]\n")

@@ -63,26 +63,21 @@ __device__ __forceinline__ void face_macs(const T (&xs)[6][6], T (&t)[6]) {
 // kA M+ + kB M- = V^-T diag(kA lambda + kB) V^-1 (generalised eigenvectors of the two
 // face blocks, template_gen.cuh), so D^-1 v = (1/s) Dm^-1 V diag(1/(kA lambda + kB)) V' Dm^-1 v.
 // (The spacing's powers divide as products with 1/s: one division instead of nine, and
-// the same values, the spacing 1/8 being a power of two.)
+// the same values, the spacing 1/8 being a power of two.) V and lambda are literals of T:
+// read from a constant table of doubles, their 78 conversions to FP32 a part, issued at an
+// eighth of the FMAs' rate, made the FP32 smoother 92 us and the stencils that end with it
+// 173-181 us a launch on a 128^3 piece (44 and 146-155 us with literals, the same bits).
 template <int AX, class T>
 __device__ __forceinline__ void dinv(T kA, T kB, T s, const T (&v)[6], T (&y)[6]) {
     const T is = T(1) / s, is2 = is * is;
-    T vt[6] = {v[0], v[1], v[2], v[3] * is, v[4] * is, v[5] * is};
+    const T vt[6] = {v[0], v[1], v[2], v[3] * is, v[4] * is, v[5] * is};
     T w[6];
+    Jac<AX>::vt(vt, w);
 #pragma unroll
-    for (int i = 0; i < 6; i++) {
-        T acc = T(0);
+    for (int i = 0; i < 6; i++) w[i] /= fma(kA, Jac<AX>::template lambda<T>(i), kB);
+    Jac<AX>::v(w, y);
 #pragma unroll
-        for (int j = 0; j < 6; j++) acc = fma((T)JAC_V_DEV[AX][j][i], vt[j], acc);
-        w[i] = acc / fma(kA, (T)JAC_L_DEV[AX][i], kB);
-    }
-#pragma unroll
-    for (int i = 0; i < 6; i++) {
-        T acc = T(0);
-#pragma unroll
-        for (int j = 0; j < 6; j++) acc = fma((T)JAC_V_DEV[AX][i][j], w[j], acc);
-        y[i] = i < 3 ? acc * is : acc * is2;
-    }
+    for (int i = 0; i < 6; i++) y[i] *= i < 3 ? is : is2;
 }
 
 // Epilogues of the stencil (Kx is the row's K x):
