@@ -136,6 +136,8 @@ int32_t* Context::pinned_i32() {
 Context::~Context() {
     last.reset();
     partial.release();
+    red_sums.release();
+    red_count.release();
     scal.release();
     if (cub_tmp) cudaFreeAsync(cub_tmp, stream);
     mem.trim(stream);

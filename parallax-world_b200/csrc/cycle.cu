@@ -219,6 +219,8 @@ struct CgScalars {
     int64_t* iters;
     int32_t* status;
     int64_t* replaced;  // per piece: residual replacements (k_cg_verify)
+    double* beta;
+    int32_t* ndone;     // pieces done
 };
 
 __global__ void k_cg_init(int np, double tol, CgScalars s, const int32_t* __restrict__ start_done) {
@@ -248,6 +250,117 @@ __global__ void k_cg_check(int np, int64_t max_iter, CgScalars s, int32_t* ndone
     if (s.done[p]) atomicAdd(ndone, 1);
 }
 
+// The vector passes of an iteration. Each is bound by HBM on a large piece and by its own
+// lanes' chains on a small one (see Chunks); the sums' order does not depend on which.
+
+// (p, Ap) and from it alpha = rz / (p, Ap) (bodies.rs:355-356)
+template <bool SPLIT>
+__global__ void __launch_bounds__(RED_LANES) k_dot_alpha(Chunks ch, CgScalars s, const double* __restrict__ p,
+                                                         const double* __restrict__ ap) {
+    const int c = red_chunk<SPLIT>(), t = red_lane<SPLIT>(), pc = ch.piece[c];
+    if (s.done[pc]) return;
+    double pap = 0.0, none = 0.0;
+    red_chain<SPLIT ? 16 : 8>(
+        6 * ch.lo[c] + t, 6 * ch.lo[c + 1], [&](int64_t i) { return make_double2(p[i], ap[i]); },
+        [&](int64_t, const double2& v) { pap = fma(v.x, v.y, pap); });
+    if (!red_finish<SPLIT>(ch, c, t, pc, pap, none)) return;
+    s.pap[pc] = pap;
+    if (!(pap > 0.0)) {
+        s.done[pc] = 1;
+        atomicMax(s.status + pc, (int)SC_BREAKDOWN);
+        atomicAdd(s.ndone, 1);
+        return;
+    }
+    s.alpha[pc] = s.rz[pc] / pap;
+}
+
+// x += alpha p; r -= alpha Ap (bodies.rs:357-362), the FP32 V-cycle's input r32 in the same
+// pass (where given), and (r, r)
+template <bool SPLIT>
+__global__ void __launch_bounds__(RED_LANES) k_update_xr(Chunks ch, CgScalars s, double* __restrict__ x,
+                                                         const double* __restrict__ p, double* __restrict__ r,
+                                                         const double* __restrict__ ap, float* __restrict__ r32) {
+    const int c = red_chunk<SPLIT>(), t = red_lane<SPLIT>(), pc = ch.piece[c];
+    if (s.done[pc]) return;
+    const double a = s.alpha[pc];
+    double rr = 0.0, none = 0.0;
+    red_chain<SPLIT ? 12 : 6>(
+        6 * ch.lo[c] + t, 6 * ch.lo[c + 1], [&](int64_t i) { return make_double4(x[i], p[i], r[i], ap[i]); },
+        [&](int64_t i, const double4& v) {
+            x[i] = v.x + a * v.y;
+            const double rn = v.z - a * v.w;
+            r[i] = rn;
+            if (r32) r32[i] = (float)rn;
+            rr = fma(rn, rn, rr);
+        });
+    if (red_finish<SPLIT>(ch, c, t, pc, rr, none)) s.rr[pc] = rr;
+}
+
+// (r, z) and from it beta = next / rz, rz = next (bodies.rs:366-370), the iteration's count
+// and the next one's check: stop when |r| <= goal; NaN stops with BREAKDOWN (bodies.rs:352).
+// FLEX, for a preconditioner applied in lower precision (not exactly symmetric): beta takes
+// the Polak-Ribiere form (z', r' - r) / (z, r) = -alpha (z', Ap) / (z, r), which equals
+// next / rz when the preconditioner is symmetric; (z', Ap) is summed in the same pass.
+template <class Z, bool FLEX, bool SPLIT>
+__global__ void __launch_bounds__(RED_LANES) k_dots_beta(Chunks ch, CgScalars s, int64_t max_iter,
+                                                         const double* __restrict__ r, const double* __restrict__ ap,
+                                                         const Z* __restrict__ z) {
+    const int c = red_chunk<SPLIT>(), t = red_lane<SPLIT>(), pc = ch.piece[c];
+    if (s.done[pc]) return;
+    double next = 0.0, zap = 0.0;
+    red_chain<SPLIT ? 16 : 8>(
+        6 * ch.lo[c] + t, 6 * ch.lo[c + 1],
+        [&](int64_t i) { return make_double3(r[i], FLEX ? ap[i] : 0.0, (double)z[i]); },
+        [&](int64_t, const double3& v) {
+            next = fma(v.x, v.z, next);
+            if (FLEX) zap = fma(v.y, v.z, zap);
+        });
+    if (!red_finish<SPLIT>(ch, c, t, pc, next, zap)) return;
+    s.beta[pc] = FLEX ? -s.alpha[pc] * zap / s.rz[pc] : next / s.rz[pc];
+    s.rz[pc] = next;
+    s.iters[pc] += 1;
+    const double nr = sqrt(s.rr[pc]);
+    int status = -1;
+    if (nr <= s.goal[pc])
+        status = (int)SC_OK;
+    else if (!(nr == nr) || !(next == next))
+        status = (int)SC_BREAKDOWN;
+    else if (s.iters[pc] >= max_iter)
+        status = (int)SC_MAXITER;
+    if (status < 0) return;
+    s.done[pc] = 1;
+    atomicMax(s.status + pc, status);
+    atomicAdd(s.ndone, 1);
+}
+
+// p = z + beta p (bodies.rs:365-369), eight blocks a chunk. On a device-side loop (count not
+// null) it also sets the loop's condition: go on while a piece is not done and fewer than
+// `chunk` iterations ran since the launch (count is zeroed before each launch; any value it
+// holds ends the loop within chunk + 1 iterations).
+template <class Z>
+__global__ void __launch_bounds__(256) k_update_p(Chunks ch, CgScalars s, double* __restrict__ p,
+                                                  const Z* __restrict__ z, cudaGraphConditionalHandle h, int np,
+                                                  uint32_t* __restrict__ count, uint32_t chunk) {
+    if (count && blockIdx.x == 0 && threadIdx.x == 0) {
+        const uint32_t n = *count + 1u;
+        *count = n;
+        cudaGraphSetConditional(h, (*s.ndone < np && n < chunk) ? 1u : 0u);
+    }
+    const int c = blockIdx.x >> 3, pc = ch.piece[c];
+    if (s.done[pc]) return;
+    const double bt = s.beta[pc];
+    const int64_t lo = 3 * ch.lo[c] + (blockIdx.x & 7) * (3 * CHUNK / 8);  // in pairs of values
+    const int64_t end = 3 * ch.lo[c + 1], hi = lo + 3 * CHUNK / 8 < end ? lo + 3 * CHUNK / 8 : end;
+    double2* p2 = reinterpret_cast<double2*>(p);
+    using Z2 = std::conditional_t<sizeof(Z) == 8, double2, float2>;
+    const Z2* z2 = reinterpret_cast<const Z2*>(z);
+    red_chain<3>(
+        lo + threadIdx.x, hi,
+        [&](int64_t i) { return make_double4((double)z2[i].x, (double)z2[i].y, p2[i].x, p2[i].y); },
+        [&](int64_t i, const double4& v) { p2[i] = make_double2(v.x + bt * v.z, v.y + bt * v.w); });
+}
+
+// the two scalar steps on their own, for the all-FP32 conjugate gradients (pcg_mixed)
 __global__ void k_cg_alpha(int np, CgScalars s) {
     int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= np || s.done[p]) return;
@@ -261,21 +374,10 @@ __global__ void k_cg_alpha(int np, CgScalars s) {
 }
 
 // beta = next / rz; rz = next (bodies.rs:366-370); counts the iteration
-__global__ void k_cg_beta(int np, CgScalars s, double* beta) {
+__global__ void k_cg_beta(int np, CgScalars s) {
     int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= np || s.done[p]) return;
-    beta[p] = s.next[p] / s.rz[p];
-    s.rz[p] = s.next[p];
-    s.iters[p] += 1;
-}
-
-// beta for a preconditioner applied in lower precision (not exactly symmetric): the
-// Polak-Ribiere form (z', r' - r) / (z, r) = -alpha (z', Ap) / (z, r), which equals
-// next / rz when the preconditioner is symmetric; rz = next; counts the iteration
-__global__ void k_cg_beta_flex(int np, CgScalars s, const double* __restrict__ zap, double* beta) {
-    int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= np || s.done[p]) return;
-    beta[p] = -s.alpha[p] * zap[p] / s.rz[p];
+    s.beta[p] = s.next[p] / s.rz[p];
     s.rz[p] = s.next[p];
     s.iters[p] += 1;
 }
@@ -314,16 +416,6 @@ __global__ void k_floor_delta(int64_t n, const double* __restrict__ x, double* _
     delta[i] = sgn * 0x1.0p-52 * fabs(x[i]);
 }
 
-// The condition of the device-side iteration loop: go on while a piece is not done and
-// fewer than `chunk` iterations ran since the launch (count is zeroed before each launch;
-// any value it holds ends the loop within chunk + 1 iterations).
-__global__ void k_loop_more(cudaGraphConditionalHandle h, const int32_t* __restrict__ ndone, int np,
-                            uint32_t* __restrict__ count, uint32_t chunk) {
-    uint32_t c = *count + 1u;
-    *count = c;
-    cudaGraphSetConditional(h, (*ndone < np && c < chunk) ? 1u : 0u);
-}
-
 // b = a in another precision for the pieces not done, one block per chunk
 template <class A, class B>
 __global__ void __launch_bounds__(256) k_cast_chunks(const int64_t* __restrict__ chunk_lo,
@@ -335,36 +427,33 @@ __global__ void __launch_bounds__(256) k_cast_chunks(const int64_t* __restrict__
     for (int64_t i = lo + threadIdx.x; i < hi; i += blockDim.x) b[i] = (B)a[i];
 }
 
-// x += alpha p; r -= alpha Ap (bodies.rs:357-362), one block per chunk
-template <class V, class S>
+// x += alpha p; r -= alpha Ap (bodies.rs:357-362) of the all-FP32 conjugate gradients, one
+// block per chunk
 __global__ void __launch_bounds__(256) k_axpy2(const int64_t* __restrict__ chunk_lo, const int32_t* __restrict__ cpiece,
                                                const int32_t* __restrict__ done, const double* __restrict__ alpha,
-                                               S* __restrict__ x, const V* __restrict__ p, V* __restrict__ r,
-                                               const V* __restrict__ ap, float* __restrict__ r32) {
+                                               float* __restrict__ x, const float* __restrict__ p,
+                                               float* __restrict__ r, const float* __restrict__ ap) {
     int c = blockIdx.x;
     int pc = cpiece[c];
     if (done[pc]) return;
     double a = alpha[pc];
     int64_t lo = 6 * chunk_lo[c], hi = 6 * chunk_lo[c + 1];
     for (int64_t i = lo + threadIdx.x; i < hi; i += blockDim.x) {
-        x[i] += (S)(a * (double)p[i]);
-        const V rn = (V)((double)r[i] - a * (double)ap[i]);
-        r[i] = rn;
-        if (r32) r32[i] = (float)rn;  // the FP32 V-cycle's input, written in the same pass
+        x[i] += (float)(a * (double)p[i]);
+        r[i] = (float)((double)r[i] - a * (double)ap[i]);
     }
 }
 
-// p = z + beta p (bodies.rs:365-369)
-template <class V, class Z = V>
+// p = z + beta p (bodies.rs:365-369), likewise
 __global__ void __launch_bounds__(256) k_pupdate(const int64_t* __restrict__ chunk_lo, const int32_t* __restrict__ cpiece,
                                                  const int32_t* __restrict__ done, const double* __restrict__ beta,
-                                                 V* __restrict__ p, const Z* __restrict__ z) {
+                                                 float* __restrict__ p, const float* __restrict__ z) {
     int c = blockIdx.x;
     int pc = cpiece[c];
     if (done[pc]) return;
     double bt = beta[pc];
     int64_t lo = 6 * chunk_lo[c], hi = 6 * chunk_lo[c + 1];
-    for (int64_t i = lo + threadIdx.x; i < hi; i += blockDim.x) p[i] = (V)((double)z[i] + bt * (double)p[i]);
+    for (int64_t i = lo + threadIdx.x; i < hi; i += blockDim.x) p[i] = (float)((double)z[i] + bt * (double)p[i]);
 }
 
 // two dots in one pass: out_a = a.b, out_c = a.a
@@ -425,31 +514,20 @@ __global__ void k_piece_sum2(int np, const int64_t* __restrict__ piece_chunk, co
     }
 }
 
-template <class T>
-__global__ void k_copy_cast(int64_t n, const double* __restrict__ a, T* __restrict__ b) {
-    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i < n) b[i] = (T)a[i];
-}
-
-
-
-
 }  // namespace
 
 struct CgState {
-    DBuf<double> scal;  // 9 arrays of np
+    DBuf<double> scal;  // 8 arrays of np
     DBuf<int32_t> flags;
     DBuf<int64_t> iters;
     DBuf<int64_t> replaced;
     DBuf<int32_t> ndone;
     DBuf<uint32_t> loop_count;  // iterations since the device-side loop's launch
     CgScalars s{};
-    double* beta = nullptr;
-    double* zap = nullptr;  // (z, Ap) for the Polak-Ribiere beta
     int np = 0;
     void init(Context& ctx, int npieces, int32_t* status) {
         np = npieces;
-        scal.alloc(9 * (size_t)np, ctx.stream, &ctx.mem);
+        scal.alloc(8 * (size_t)np, ctx.stream, &ctx.mem);
         scal.zero();
         flags.alloc(np, ctx.stream, &ctx.mem);
         flags.zero();
@@ -467,12 +545,12 @@ struct CgState {
         s.pap = q + 4 * np;
         s.next = q + 5 * np;
         s.alpha = q + 6 * np;
-        beta = q + 7 * np;
-        zap = q + 8 * np;
+        s.beta = q + 7 * np;
         s.done = flags.get();
         s.iters = iters.get();
         s.status = status;
         s.replaced = replaced.get();
+        s.ndone = ndone.get();
     }
 };
 
@@ -486,7 +564,6 @@ static void ensure_partial(Context& ctx, const Level& L) {
     if ((int64_t)ctx.partial.size() < 2 * std::max<int64_t>(L.nchunks, 1) + 2048)
         ctx.partial.alloc(2 * (L.nchunks + 1024) + 2048, ctx.stream, &ctx.mem);
 }
-static void prepare_top(const Level&) {}
 
 // two chunked dots (a.b and a.a) per piece
 template <class T, class U = T>
@@ -621,6 +698,11 @@ static int64_t pcg(Context& ctx, Batch& b, const V* rhs, S* x, V* r, V* z, V* p,
     }
     dot2<V, P>(ctx, L, cg.s.done, r, zs, cg.s.rz, cg.s.rr);
     // one iteration (bodies.rs:351-371), ending with the next iteration's check
+    const Chunks ch = red_chunks(ctx, L);
+    // iterations one launch of the device-side loop runs at most between looks at the done
+    // count (and at the time limit)
+    const uint32_t chunk = 32;
+    bool device_loop = false;
     auto body = [&]() {
         if (L.matrix_free) {
             stencil_apply<V>(ctx, b, p, ap, nullptr, cg.s.done);
@@ -629,31 +711,26 @@ static int64_t pcg(Context& ctx, Batch& b, const V* rhs, S* x, V* r, V* z, V* p,
             spmv<V>(ctx, SPMV_Y, L.n, L.rowptr.get(), L.col.get(), VAL<V>(L), p, nullptr, ap, nullptr, nullptr,
                     L.piece.get(), nullptr, cg.s.done, L.nnzb);
         }
-        dot2<V>(ctx, L, cg.s.done, p, ap, cg.s.pap, nullptr);
-        k_cg_alpha<<<grid_for(np, 128), 128, 0, st>>>(np, cg.s);
-        SC_LAUNCH_CK();
-        if (L.nchunks > 0) {
-            k_axpy2<V, S><<<(unsigned)L.nchunks, 256, 0, st>>>(L.chunk_lo.get(), L.chunk_piece.get(), cg.s.done,
-                                                              cg.s.alpha, x, p, r, ap,
-                                                              same ? nullptr : reinterpret_cast<float*>(rp));
+        if (L.nchunks <= 0) return;  // no parts: every piece is done
+        const unsigned grid = red_grid(L.nchunks);
+        const int block = red_block(L.nchunks);
+        float* r32 = same ? nullptr : reinterpret_cast<float*>(rp);
+        auto passes = [&](auto split) {
+            constexpr bool SPLIT = decltype(split)::value;
+            k_dot_alpha<SPLIT><<<grid, block, 0, st>>>(ch, cg.s, p, ap);
             SC_LAUNCH_CK();
-        }
-        precondition();
-        dot2<V, P>(ctx, L, cg.s.done, r, zs, cg.s.next, cg.s.rr);
-        if constexpr (same) {
-            k_cg_beta<<<grid_for(np, 128), 128, 0, st>>>(np, cg.s, cg.beta);
-        } else {
-            dot2<V, P>(ctx, L, cg.s.done, ap, zs, cg.zap, nullptr);
-            k_cg_beta_flex<<<grid_for(np, 128), 128, 0, st>>>(np, cg.s, cg.zap, cg.beta);
-        }
-        SC_LAUNCH_CK();
-        if (L.nchunks > 0) {
-            k_pupdate<V, P><<<(unsigned)L.nchunks, 256, 0, st>>>(L.chunk_lo.get(), L.chunk_piece.get(), cg.s.done,
-                                                                cg.beta, p, zs);
+            k_update_xr<SPLIT><<<grid, block, 0, st>>>(ch, cg.s, x, p, r, ap, r32);
             SC_LAUNCH_CK();
-        }
-        SC_CK(cudaMemsetAsync(cg.ndone.get(), 0, sizeof(int32_t), st));
-        k_cg_check<<<grid_for(np, 128), 128, 0, st>>>(np, max_iter, cg.s, cg.ndone.get());
+            precondition();
+            k_dots_beta<P, !same, SPLIT><<<grid, block, 0, st>>>(ch, cg.s, max_iter, r, ap, zs);
+            SC_LAUNCH_CK();
+        };
+        if (red_split(L.nchunks))
+            passes(std::true_type{});
+        else
+            passes(std::false_type{});
+        k_update_p<P><<<(unsigned)(8 * L.nchunks), 256, 0, st>>>(ch, cg.s, p, zs, ctx.loop_handle, np,
+                                                                 device_loop ? cg.loop_count.get() : nullptr, chunk);
         SC_LAUNCH_CK();
     };
     // Residual replacement: r = b - K x in FP64 for the pieces whose true residual misses
@@ -707,24 +784,18 @@ static int64_t pcg(Context& ctx, Batch& b, const V* rhs, S* x, V* r, V* z, V* p,
     };
     cudaGraphExec_t exec = nullptr, loop = nullptr;
     int64_t per_iteration = 0, graph_kernels = 0;
-    // iterations one launch of the device-side loop runs at most between looks at the
-    // done count (and at the time limit)
-    const uint32_t chunk = 32;
     try {
         // Replaying a captured iteration saves ~50 launches an iteration; timing
         // individual kernels (profiling) launches them one by one instead.
         bool use_graph = ctx.prof.mask == 0 && graphs_enabled();
         if (use_graph) {
             ensure_partial(ctx, L);
-            for (auto& lv : b.levels) prepare_top(lv);
             // first choice: the iterations loop on the device, a graph whose conditional
             // WHILE node replays the iteration until every piece is done (or `chunk` ran)
             const int64_t l0 = g_launches.load();
-            loop = capture_loop(st, [&] {
-                body();
-                k_loop_more<<<1, 1, 0, st>>>(ctx.loop_handle, cg.ndone.get(), np, cg.loop_count.get(), chunk);
-                SC_LAUNCH_CK();
-            }, ctx);
+            device_loop = L.nchunks > 0;
+            if (device_loop) loop = capture_loop(st, body, ctx);
+            device_loop = loop != nullptr;
             per_iteration = g_launches.load() - l0;
             g_launches.fetch_sub(per_iteration);  // counted per iteration run, below
             if (!loop) {
@@ -1024,8 +1095,8 @@ void pcg_mixed(Context& ctx, Batch& b, const sc_options& opt, DBuf<double>& x, S
         dot2<float>(ctx, L, cg.s.done, p.get(), ap.get(), cg.s.pap, nullptr);
         k_cg_alpha<<<grid_for(np, 128), 128, 0, st>>>(np, cg.s);
         SC_LAUNCH_CK();
-        chunks(k_axpy2<float, float>, (const int32_t*)cg.s.done, (const double*)cg.s.alpha, x32.get(),
-               (const float*)p.get(), r.get(), (const float*)ap.get(), (float*)nullptr);
+        chunks(k_axpy2, (const int32_t*)cg.s.done, (const double*)cg.s.alpha, x32.get(), (const float*)p.get(),
+               r.get(), (const float*)ap.get());
     };
     // the FP64 update: fold x32 into x, r = b - K x in FP64, its verdict
     auto update = [&]() {
@@ -1048,9 +1119,9 @@ void pcg_mixed(Context& ctx, Batch& b, const sc_options& opt, DBuf<double>& x, S
     auto second = [&]() {
         cycle<float>(ctx, b, 0, r.get(), z.get(), cg.s.done);
         dot2<float>(ctx, L, cg.s.done, r.get(), z.get(), cg.s.next, cg.s.rr);
-        k_cg_beta<<<grid_for(np, 128), 128, 0, st>>>(np, cg.s, cg.beta);
+        k_cg_beta<<<grid_for(np, 128), 128, 0, st>>>(np, cg.s);
         SC_LAUNCH_CK();
-        chunks(k_pupdate<float>, (const int32_t*)cg.s.done, (const double*)cg.beta, p.get(), (const float*)z.get());
+        chunks(k_pupdate, (const int32_t*)cg.s.done, (const double*)cg.s.beta, p.get(), (const float*)z.get());
         SC_CK(cudaMemsetAsync(counts.get(), 0, sizeof(int32_t), st));
         k_mixed_check<<<grid_for(np, 128), 128, 0, st>>>(np, max_iter, cg.s, cand.get(), counts.get());
         SC_LAUNCH_CK();

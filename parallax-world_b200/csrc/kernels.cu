@@ -312,34 +312,16 @@ __global__ void __launch_bounds__(512) k_top_solve(const int32_t* __restrict__ t
     }
 }
 
-template <class T>
-__global__ void __launch_bounds__(256) k_chunk_dot(const int64_t* __restrict__ chunk_lo, const T* __restrict__ a,
-                                                   const T* __restrict__ b, double* __restrict__ partial) {
-    int64_t lo = 6 * chunk_lo[blockIdx.x], hi = 6 * chunk_lo[blockIdx.x + 1];
-    double s = 0.0;
-    for (int64_t i = lo + threadIdx.x; i < hi; i += blockDim.x) s = fma((double)a[i], (double)b[i], s);
-    __shared__ double red[256];
-    red[threadIdx.x] = s;
-    __syncthreads();
-    for (int w = 128; w > 0; w >>= 1) {
-        if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) partial[blockIdx.x] = red[0];
-}
-
-// per piece: the sum of its chunks' partials, one warp per piece (strided lanes, then a
-// shuffle tree: a fixed order)
-__global__ void k_piece_sum(int np, const int64_t* __restrict__ piece_chunk, const double* __restrict__ partial,
-                            double* __restrict__ out) {
-    const int p = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
-    const int lane = threadIdx.x & 31;
-    if (p >= np) return;
-    double s = 0.0;
-    for (int64_t c = piece_chunk[p] + lane; c < piece_chunk[p + 1]; c += 32) s += partial[c];
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-    if (lane == 0) out[p] = s;
+// out[p] = sum over piece p's parts of a.b
+template <class T, bool SPLIT>
+__global__ void __launch_bounds__(RED_LANES) k_seg_dot(Chunks ch, const T* __restrict__ a, const T* __restrict__ b,
+                                                       double* __restrict__ out) {
+    const int c = red_chunk<SPLIT>(), t = red_lane<SPLIT>(), p = ch.piece[c];
+    double s = 0.0, none = 0.0;
+    red_chain<SPLIT ? 16 : 8>(
+        6 * ch.lo[c] + t, 6 * ch.lo[c + 1], [&](int64_t i) { return make_double2((double)a[i], (double)b[i]); },
+        [&](int64_t, const double2& v) { s = fma(v.x, v.y, s); });
+    if (red_finish<SPLIT>(ch, c, t, p, s, none)) out[p] = s;
 }
 
 }  // namespace
@@ -480,16 +462,41 @@ void top_solve(Context& ctx, const Level& L, const T* r, T* z, const int32_t* do
     SC_LAUNCH_CK();
 }
 
+// The level's chunks with the context's scratch for their sums (grown here, so never inside
+// a capture).
+Chunks red_chunks(Context& ctx, const Level& L) {
+    const size_t nch = (size_t)std::max<int64_t>(L.nchunks, 1), np = L.pstart.size();
+    const size_t sums = 2 * nch + (red_split(L.nchunks) ? 2 * RED_LANES * nch : 0), counts = nch + np;
+    if (ctx.red_sums.size() < sums) ctx.red_sums.alloc(sums + 1024, ctx.stream, &ctx.mem);
+    if (ctx.red_count.size() < counts) {
+        ctx.red_count.alloc(counts + 1024, ctx.stream, &ctx.mem);
+        ctx.red_count.zero();
+    }
+    Chunks ch;
+    ch.lo = L.chunk_lo.get();
+    ch.piece = L.chunk_piece.get();
+    ch.piece_chunk = L.piece_chunk.get();
+    ch.part = ctx.red_sums.get();
+    ch.lanes = ctx.red_sums.get() + 2 * nch;
+    ch.arrived = ctx.red_count.get();
+    ch.ticket = ctx.red_count.get() + nch;
+    return ch;
+}
+
 template <class T>
 void seg_dot_t(Context& ctx, const Level& L, const T* a, const T* b, double* out) {
-    int np = (int)L.pstart.size() - 1;
-    if (ctx.partial.size() < (size_t)std::max<int64_t>(L.nchunks, 1)) ctx.partial.alloc(L.nchunks + 1024, ctx.stream, &ctx.mem);
-    if (L.nchunks > 0) {
-        k_chunk_dot<T><<<(unsigned)L.nchunks, 256, 0, ctx.stream>>>(L.chunk_lo.get(), a, b, ctx.partial.get());
-        SC_LAUNCH_CK();
-    }
-    k_piece_sum<<<grid_for((int64_t)np * 32, 128), 128, 0, ctx.stream>>>(np, L.piece_chunk.get(), ctx.partial.get(),
-                                                                        out);
+    const int np = (int)L.pstart.size() - 1;
+    bool empty = false;  // a piece without parts sums to zero
+    for (int p = 0; p < np && !empty; p++) empty = L.pstart[p] == L.pstart[p + 1];
+    if (empty) SC_CK(cudaMemsetAsync(out, 0, np * sizeof(double), ctx.stream));
+    if (L.nchunks <= 0) return;
+    const Chunks ch = red_chunks(ctx, L);
+    const unsigned grid = red_grid(L.nchunks);
+    const int block = red_block(L.nchunks);
+    if (red_split(L.nchunks))
+        k_seg_dot<T, true><<<grid, block, 0, ctx.stream>>>(ch, a, b, out);
+    else
+        k_seg_dot<T, false><<<grid, block, 0, ctx.stream>>>(ch, a, b, out);
     SC_LAUNCH_CK();
 }
 

@@ -45,7 +45,141 @@ __device__ __forceinline__ void st6(T* __restrict__ p, const T (&o)[6]) {
     }
 }
 
+// ---- reductions over a level's chunks ----------------------------------------------------
+// A sum over a piece is taken in one fixed order whatever the launch: a chunk (CHUNK parts)
+// has 256 lanes, lane t adds the chunk's values t, t + 256, ... in turn; the lanes' sums meet
+// in a halving tree (t + 128, + 64, ..., + 1); 32 strided lanes add the piece's chunks and
+// meet in a tree again.
+//
+// The order leaves each lane a serial chain of up to 96 values, and the launch decides where
+// the lanes run. WHOLE: a block a chunk. SPLIT, where that would leave most of the device
+// idle: a warp (a block of its own) 32 lanes of a chunk, 8 warps a chunk, 16 values' loads in
+// flight a lane. The last of a chunk's warps to arrive adds its lanes, the last of a piece's
+// chunks the piece, so no launch follows for the sums or for the scalars that come of them.
+constexpr int RED_LANES = 256;
+struct Chunks {
+    const int64_t* lo = nullptr;           // nchunks + 1 bounds, in parts
+    const int32_t* piece = nullptr;        // each chunk's piece
+    const int64_t* piece_chunk = nullptr;  // each piece's first chunk
+    double* part = nullptr;                // two partial sums a chunk
+    double* lanes = nullptr;               // SPLIT: two sums a lane of a chunk
+    uint32_t* arrived = nullptr;           // SPLIT: per chunk, warps that arrived (zero between kernels)
+    uint32_t* ticket = nullptr;            // per piece, chunks that arrived (zero between kernels)
+};
+// A block a chunk fills the device from about four blocks an SM on.
+constexpr int64_t RED_WHOLE = 592;
+inline bool red_split(int64_t nchunks) { return nchunks < RED_WHOLE; }
+inline unsigned red_grid(int64_t nchunks) { return (unsigned)(red_split(nchunks) ? 8 * nchunks : nchunks); }
+inline int red_block(int64_t nchunks) { return red_split(nchunks) ? 32 : RED_LANES; }
+
+// This thread's chunk and lane.
+template <bool SPLIT>
+__device__ __forceinline__ int red_chunk() {
+    return SPLIT ? (int)(blockIdx.x >> 3) : (int)blockIdx.x;
+}
+template <bool SPLIT>
+__device__ __forceinline__ int red_lane() {
+    return SPLIT ? (int)((blockIdx.x & 7) * 32 + threadIdx.x) : (int)threadIdx.x;
+}
+
+// A lane's chain: use(i, load(i)) for i = first, first + 256, ... below end, in that order, U
+// loads in flight.
+template <int U, class F, class G>
+__device__ __forceinline__ void red_chain(int64_t first, int64_t end, F&& load, G&& use) {
+    using V = decltype(load(first));
+    int64_t i = first;
+    for (; i + RED_LANES * (U - 1) < end; i += RED_LANES * U) {
+        V v[U];
+#pragma unroll
+        for (int j = 0; j < U; j++) v[j] = load(i + RED_LANES * j);
+#pragma unroll
+        for (int j = 0; j < U; j++) use(i + RED_LANES * j, v[j]);
+    }
+    V v[U];
+#pragma unroll
+    for (int j = 0; j < U; j++)
+        if (i + RED_LANES * j < end) v[j] = load(i + RED_LANES * j);
+#pragma unroll
+    for (int j = 0; j < U; j++)
+        if (i + RED_LANES * j < end) use(i + RED_LANES * j, v[j]);
+}
+
+// Every thread of the kernel comes here with its lane's sums a and b. True in one thread of
+// the last warp to arrive of the chunk's piece, with the piece's sums in a and b.
+template <bool SPLIT>
+__device__ __forceinline__ bool red_finish(const Chunks& ch, int c, int t, int p, double& a, double& b) {
+    double va[8], vb[8];
+    const int l = threadIdx.x & 31;
+    if constexpr (SPLIT) {
+        double* ln = ch.lanes + 2 * RED_LANES * (int64_t)c;
+        __stcg(ln + t, a);
+        __stcg(ln + RED_LANES + t, b);
+        __threadfence();
+        __syncwarp();
+        uint32_t n = 0;
+        if (l == 0) n = atomicAdd(ch.arrived + c, 1u);
+        if (__shfl_sync(0xffffffffu, n, 0) != 7) return false;
+        if (l == 0) ch.arrived[c] = 0;
+        __threadfence();
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            va[k] = __ldcg(ln + l + 32 * k);
+            vb[k] = __ldcg(ln + RED_LANES + l + 32 * k);
+        }
+    } else {
+        __shared__ double ra[RED_LANES], rb[RED_LANES];
+        ra[t] = a;
+        rb[t] = b;
+        __syncthreads();
+        if (t >= 32) return false;
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            va[k] = ra[l + 32 * k];
+            vb[k] = rb[l + 32 * k];
+        }
+    }
+#pragma unroll
+    for (int w = 4; w > 0; w >>= 1)
+#pragma unroll
+        for (int k = 0; k < w; k++) {
+            va[k] += va[k + w];
+            vb[k] += vb[k + w];
+        }
+    a = va[0];
+    b = vb[0];
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        a += __shfl_down_sync(0xffffffffu, a, off);
+        b += __shfl_down_sync(0xffffffffu, b, off);
+    }
+    const int64_t c0 = ch.piece_chunk[p], c1 = ch.piece_chunk[p + 1];
+    uint32_t n = 0;
+    if (l == 0) {
+        __stcg(ch.part + 2 * (int64_t)c, a);
+        __stcg(ch.part + 2 * (int64_t)c + 1, b);
+        __threadfence();
+        n = atomicAdd(ch.ticket + p, 1u);
+    }
+    if (__shfl_sync(0xffffffffu, n, 0) != (uint32_t)(c1 - c0 - 1)) return false;
+    if (l == 0) ch.ticket[p] = 0;
+    __threadfence();
+    a = b = 0.0;
+#pragma unroll 8
+    for (int64_t i = c0 + l; i < c1; i += 32) {
+        const double2 v = __ldcg(reinterpret_cast<const double2*>(ch.part) + i);
+        a += v.x;
+        b += v.y;
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        a += __shfl_xor_sync(0xffffffffu, a, off);
+        b += __shfl_xor_sync(0xffffffffu, b, off);
+    }
+    return l == 0;
+}
+
 // Host launchers (kernels.cu).
+Chunks red_chunks(Context& ctx, const Level& L);
 // nnz (the stored blocks) picks the warps a row (one when 0); see warps_per_row.
 template <class T>
 void spmv(Context& ctx, int mode, int64_t nrows, const int64_t* rowptr, const int32_t* col, const T* val, const T* x,

@@ -284,6 +284,8 @@ struct Context {
     std::string last_error;
     // scratch for reductions
     DBuf<double> partial;
+    DBuf<double> red_sums;           // the fused reductions' partial sums (Chunks)
+    DBuf<uint32_t> red_count;        // and their arrival counts
     DBuf<double> scal;
     void* cub_tmp = nullptr;
     size_t cub_bytes = 0;
