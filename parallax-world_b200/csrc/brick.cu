@@ -581,11 +581,11 @@ __global__ void __launch_bounds__(256) k_brick_jacobi(int64_t n, const float2* _
                                                       const int32_t* __restrict__ done) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
-    if (skip_row && skip_row[i]) return;
-    const int p = piece[i];
-    if (done && done[p]) return;
-    const T w = step ? (T)step[p] : T(1);
     const float2 e = __ldg(kk + i);
+    const int32_t skip = skip_row ? skip_row[i] : 0;
+    const int p = piece ? piece[i] : 0;
+    if (skip || (done && done[p])) return;
+    const T w = step ? (T)step[p] : T(1);
     const int ax = (signbit(e.x) ? 1 : 0) | (signbit(e.y) ? 2 : 0);
     const T kA = (T)fabsf(e.x), kB = (T)fabsf(e.y);
     T rv[6], d[6];
@@ -935,7 +935,8 @@ void brick_jacobi(Context& ctx, const Batch& b, const T* r, T* x, const double* 
                   const int32_t* done) {
     const Level& L = b.levels[0];
     k_brick_jacobi<T><<<grid_for(L.n, 256), 256, 0, ctx.stream>>>(L.n, b.grid.bricks.kk.get(), r, x, (T)b.grid.s,
-                                                                  L.piece.get(), step, skip_row, done);
+                                                                  b.npieces == 1 ? nullptr : L.piece.get(), step,
+                                                                  skip_row, done);
     SC_LAUNCH_CK();
 }
 template void brick_jacobi<double>(Context&, const Batch&, const double*, double*, const double*, const int32_t*,

@@ -122,28 +122,36 @@ static double transfer_bytes(const Level& L, const Level& C) {
 
 // One V-cycle from level l: z = M r (bodies.rs:377-403). Pieces whose top is level l are
 // solved directly there; the others smooth, hand the residual up, take the correction
-// back and smooth again.
+// back and smooth again. Above level 0 the first smoothing, x = step D^-1 r, is done already:
+// by the restriction that made r. On small levels each kernel is a chain of dependent loads,
+// so a single piece's kernels look up no row's piece, and a level without tops none of its
+// rows' flags (done is null for a single piece: the iterations stop with it).
 template <class T>
 static void cycle(Context& ctx, Batch& b, int l, const T* r, T* z, const int32_t* done) {
     Level& L = b.levels[l];
     bool deepest = l + 1 == (int)b.levels.size();
+    const bool one = b.npieces == 1;
+    const int32_t* piece = one ? nullptr : L.piece.get();
+    T* xc = nullptr;  // the next level's x, where that level smooths
+    if (l + 2 < (int)b.levels.size()) xc = VX<T>(b.levels[l + 1]).get();
     if (!deepest && l == 0 && L.matrix_free) {
         // level 0 of voxel pieces: smoother and both transfers matrix-free
         Level& C = b.levels[1];
         T* x = VX<T>(L).get();
-        level0_down<T>(ctx, b, r, x, VL<T>(L).get(), VT<T>(L).get(), VU<T>(L).get(), VR<T>(C).get(), done);
+        level0_down<T>(ctx, b, r, x, VL<T>(L).get(), VT<T>(L).get(), VU<T>(L).get(), VR<T>(C).get(), xc,
+                       done);
         cycle<T>(ctx, b, 1, VR<T>(C).get(), VZ<T>(C).get(), done);
         level0_up<T>(ctx, b, r, x, VT<T>(L).get(), VZ<T>(C).get(), z, done);
     } else if (!deepest) {
-        const int32_t* skip = L.top_of_part.get();
+        const int32_t* skip = L.top_h.empty() ? nullptr : L.top_of_part.get();
         T* x = VX<T>(L).get();
         T* left = VL<T>(L).get();
         bool mf = l == 0 && L.matrix_free;
         double vb = (double)sizeof(T) * 6.0 * (double)L.n;
         // x = step D^-1 r (bodies.rs:386), and any further sweeps
-        {
+        if (l == 0) {
             ProfScope ps(ctx, fam_of<T>(SC_FAM_SMOOTH64), 2 * vb + 36.0 * sizeof(T) * L.n);
-            jacobi<T>(ctx, L.n, INV<T>(L), r, x, L.step.get(), L.piece.get(), skip, done);
+            jacobi<T>(ctx, L.n, INV<T>(L), r, x, L.step.get(), piece, skip, done);
         }
         for (int sweep = 1; sweep < b.sweeps; sweep++) {
             if (mf) {
@@ -151,7 +159,7 @@ static void cycle(Context& ctx, Batch& b, int l, const T* r, T* z, const int32_t
             } else {
                 ProfScope ps(ctx, fam_of<T>(SC_FAM_SPMV64), spmv_bytes<T>(L, 3) + vb + 36.0 * sizeof(T) * L.n);
                 spmv<T>(ctx, SPMV_RES_SMOOTH, L.n, L.rowptr.get(), L.col.get(), VAL<T>(L), x, r, left, INV<T>(L),
-                        L.step.get(), L.piece.get(), skip, done, L.nnzb);
+                        L.step.get(), piece, skip, done, L.nnzb);
             }
             SC_CK(cudaMemcpyAsync(x, left, 6 * L.n * sizeof(T), cudaMemcpyDeviceToDevice, ctx.stream));
         }
@@ -161,21 +169,22 @@ static void cycle(Context& ctx, Batch& b, int l, const T* r, T* z, const int32_t
         } else {
             ProfScope ps(ctx, fam_of<T>(SC_FAM_SPMV64), spmv_bytes<T>(L, 3));
             spmv<T>(ctx, SPMV_RES, L.n, L.rowptr.get(), L.col.get(), VAL<T>(L), x, r, left, nullptr, nullptr,
-                    L.piece.get(), skip, done, L.nnzb);
+                    piece, skip, done, L.nnzb);
         }
         Level& C = b.levels[l + 1];
         // coarse = P' left (bodies.rs:388-390)
         {
-            ProfScope ps(ctx, fam_of<T>(SC_FAM_TRANSFER64), transfer_bytes<T>(L, C));
-            spmv<T>(ctx, SPMV_Y, C.n, L.tptr.get(), L.trow.get(), PTVAL<T>(L), left, nullptr, VR<T>(C).get(),
-                    nullptr, nullptr, C.piece.get(), nullptr, done, L.pnnz);
+            const double jac = xc ? (double)sizeof(T) * 42.0 * (double)C.n : 0.0;
+            ProfScope ps(ctx, fam_of<T>(SC_FAM_TRANSFER64), transfer_bytes<T>(L, C) + jac);
+            spmv<T>(ctx, xc ? SPMV_Y_JACOBI : SPMV_Y, C.n, L.tptr.get(), L.trow.get(), PTVAL<T>(L), left, nullptr,
+                    VR<T>(C).get(), INV<T>(C), C.step.get(), one ? nullptr : C.piece.get(), nullptr, done, L.pnnz, xc);
         }
         cycle<T>(ctx, b, l + 1, VR<T>(C).get(), VZ<T>(C).get(), done);
         // x += P y (bodies.rs:392-395)
         {
             ProfScope ps(ctx, fam_of<T>(SC_FAM_TRANSFER64), transfer_bytes<T>(L, C) + vb);
             spmv<T>(ctx, SPMV_ADD, L.n, L.prow.get(), L.pcol.get(), PVAL<T>(L), VZ<T>(C).get(), nullptr, x, nullptr,
-                    nullptr, L.piece.get(), skip, done, L.pnnz);
+                    nullptr, piece, skip, done, L.pnnz);
         }
         // z = x + step D^-1 (r - K x) (bodies.rs:396-401), after any further sweeps
         for (int sweep = 1; sweep < b.sweeps; sweep++) {
@@ -184,18 +193,18 @@ static void cycle(Context& ctx, Batch& b, int l, const T* r, T* z, const int32_t
             } else {
                 ProfScope ps(ctx, fam_of<T>(SC_FAM_SPMV64), spmv_bytes<T>(L, 3) + vb + 36.0 * sizeof(T) * L.n);
                 spmv<T>(ctx, SPMV_RES_SMOOTH, L.n, L.rowptr.get(), L.col.get(), VAL<T>(L), x, r, left, INV<T>(L),
-                        L.step.get(), L.piece.get(), skip, done, L.nnzb);
+                        L.step.get(), piece, skip, done, L.nnzb);
             }
             SC_CK(cudaMemcpyAsync(x, left, 6 * L.n * sizeof(T), cudaMemcpyDeviceToDevice, ctx.stream));
         }
         if (mf) {
             stencil_residual<T>(ctx, b, x, r, left, skip, done);
             ProfScope ps(ctx, fam_of<T>(SC_FAM_SMOOTH64), 3 * vb + 36.0 * sizeof(T) * L.n);
-            jacobi_add<T>(ctx, L.n, INV<T>(L), left, x, z, L.step.get(), L.piece.get(), skip, done);
+            jacobi_add<T>(ctx, L.n, INV<T>(L), left, x, z, L.step.get(), piece, skip, done);
         } else {
             ProfScope ps(ctx, fam_of<T>(SC_FAM_SPMV64), spmv_bytes<T>(L, 3) + vb + 36.0 * sizeof(T) * L.n);
             spmv<T>(ctx, SPMV_RES_SMOOTH, L.n, L.rowptr.get(), L.col.get(), VAL<T>(L), x, r, z, INV<T>(L),
-                    L.step.get(), L.piece.get(), skip, done, L.nnzb);
+                    L.step.get(), piece, skip, done, L.nnzb);
         }
     }
     if (!L.top_h.empty()) {
@@ -670,11 +679,13 @@ static int64_t pcg(Context& ctx, Batch& b, const V* rhs, S* x, V* r, V* z, V* p,
     // direction update read directly (no FP64 copy of z is made); rp, the cycle's input,
     // is written by the residual update itself.
     const P* zs = same ? reinterpret_cast<const P*>(z) : zp;
+    // one piece's kernels need no look at its done flag: the loop ends with it
+    const int32_t* done = np == 1 ? nullptr : cg.s.done;
     auto precondition = [&]() {
         if constexpr (same)
-            cycle<V>(ctx, b, 0, r, z, cg.s.done);
+            cycle<V>(ctx, b, 0, r, z, done);
         else
-            cycle<P>(ctx, b, 0, rp, zp, cg.s.done);
+            cycle<P>(ctx, b, 0, rp, zp, done);
     };
     SC_CK(cudaMemsetAsync(x, 0, n6 * sizeof(S), st));
     SC_CK(cudaMemcpyAsync(r, rhs, n6 * sizeof(V), cudaMemcpyDeviceToDevice, st));
@@ -705,11 +716,11 @@ static int64_t pcg(Context& ctx, Batch& b, const V* rhs, S* x, V* r, V* z, V* p,
     bool device_loop = false;
     auto body = [&]() {
         if (L.matrix_free) {
-            stencil_apply<V>(ctx, b, p, ap, nullptr, cg.s.done);
+            stencil_apply<V>(ctx, b, p, ap, nullptr, done);
         } else {
             ProfScope ps(ctx, fam_of<V>(SC_FAM_SPMV64), spmv_bytes<V>(L, 2));
             spmv<V>(ctx, SPMV_Y, L.n, L.rowptr.get(), L.col.get(), VAL<V>(L), p, nullptr, ap, nullptr, nullptr,
-                    L.piece.get(), nullptr, cg.s.done, L.nnzb);
+                    np == 1 ? nullptr : L.piece.get(), nullptr, done, L.nnzb);
         }
         if (L.nchunks <= 0) return;  // no parts: every piece is done
         const unsigned grid = red_grid(L.nchunks);

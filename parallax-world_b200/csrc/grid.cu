@@ -796,29 +796,62 @@ __global__ void __launch_bounds__(256) k_jacobi_mf(int64_t n, const int4* __rest
 }
 
 // rc[c] = sum over the parts k of body c of R_k' u_k, R_k' u = (u_t, u_w + r_k x u_t):
-// the rigid part P0' of the restriction (bodies.rs:239, 388-390)
+// the rigid part P0' of the restriction (bodies.rs:239, 388-390), and (xc not null) the next
+// level's pre-smoothing xc = step D^-1 rc (bodies.rs:386) while rc is at hand. A thread a
+// body adds its members in order; what bounds it is the chain member -> values, so four
+// members' loads are in flight (one at a time: 60 us on a 128^3 piece in FP32, 17 on a
+// 32^3 one in FP64; now 55 and 10, the smoothing included).
 template <class T>
-__global__ void __launch_bounds__(256) k_p0t(int64_t nc, const int64_t* __restrict__ moff,
+__global__ void __launch_bounds__(128) k_p0t(int64_t nc, const int64_t* __restrict__ moff,
                                              const int32_t* __restrict__ mem, const T* __restrict__ rvec,
                                              const T* __restrict__ u, T* __restrict__ rc,
-                                             const int32_t* __restrict__ piece_c, const int32_t* __restrict__ done) {
+                                             const int32_t* __restrict__ piece_c, const int32_t* __restrict__ done,
+                                             const T* __restrict__ inv, const double* __restrict__ step,
+                                             T* __restrict__ xc) {
     int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (c >= nc) return;
-    if (done && done[piece_c[c]]) return;
+    const int64_t t0 = moff[c], t1 = moff[c + 1];
+    const int p = piece_c ? piece_c[c] : 0;
+    if (done && done[p]) return;
     T o[6] = {T(0), T(0), T(0), T(0), T(0), T(0)};
-    for (int64_t t = moff[c]; t < moff[c + 1]; t++) {
-        int32_t k = mem[t];
-        T uv[6];
-        load6<T>(u, k, uv);
-        T r0 = rvec[3 * (int64_t)k], r1 = rvec[3 * (int64_t)k + 1], r2 = rvec[3 * (int64_t)k + 2];
-        o[0] += uv[0];
-        o[1] += uv[1];
-        o[2] += uv[2];
-        o[3] += uv[3] + (r1 * uv[2] - r2 * uv[1]);
-        o[4] += uv[4] + (r2 * uv[0] - r0 * uv[2]);
-        o[5] += uv[5] + (r0 * uv[1] - r1 * uv[0]);
+    constexpr int U = 4;
+    for (int64_t t = t0; t < t1; t += U) {
+        int32_t k[U];
+        T uv[U][6], rv[U][3];
+#pragma unroll
+        for (int j = 0; j < U; j++) k[j] = t + j < t1 ? mem[t + j] : -1;
+#pragma unroll
+        for (int j = 0; j < U; j++)
+            if (k[j] >= 0) {
+                load6<T>(u, k[j], uv[j]);
+                rv[j][0] = rvec[3 * (int64_t)k[j]];
+                rv[j][1] = rvec[3 * (int64_t)k[j] + 1];
+                rv[j][2] = rvec[3 * (int64_t)k[j] + 2];
+            }
+#pragma unroll
+        for (int j = 0; j < U; j++)
+            if (k[j] >= 0) {
+                o[0] += uv[j][0];
+                o[1] += uv[j][1];
+                o[2] += uv[j][2];
+                o[3] += uv[j][3] + (rv[j][1] * uv[j][2] - rv[j][2] * uv[j][1]);
+                o[4] += uv[j][4] + (rv[j][2] * uv[j][0] - rv[j][0] * uv[j][2]);
+                o[5] += uv[j][5] + (rv[j][0] * uv[j][1] - rv[j][1] * uv[j][0]);
+            }
     }
     store6<T>(rc, c, o);
+    if (!xc) return;
+    const T st = (T)step[p];
+    T xo[6];
+#pragma unroll
+    for (int i = 0; i < 6; i++) {
+        T d[6], s = T(0);
+        load6<T>(inv + 36 * c, i, d);
+#pragma unroll
+        for (int j = 0; j < 6; j++) s = fma(d[j], o[j], s);
+        xo[i] = s * st;
+    }
+    store6<T>(xc, c, xo);
 }
 
 // e_k = R_k z_{up[k]} = (z_t + z_w x r_k, z_w): the rigid part P0 of the prolongation
@@ -828,9 +861,8 @@ __global__ void __launch_bounds__(256) k_p0(int64_t n, const int32_t* __restrict
                                             const int32_t* __restrict__ skip_row, const int32_t* __restrict__ done) {
     int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (k >= n) return;
-    if (skip_row && skip_row[k]) return;
-    if (done && done[piece[k]]) return;
-    int32_t c = up[k];
+    const int32_t c = up[k], skip = skip_row ? skip_row[k] : 0;
+    if (skip || (done && done[piece[k]])) return;
     T zv[6];
     load6<T>(z, c, zv);
     T r0 = rvec[3 * k], r1 = rvec[3 * k + 1], r2 = rvec[3 * k + 2];
@@ -939,11 +971,11 @@ template void stencil_residual<float>(Context&, const Batch&, const float*, cons
 //   x = w D^-1 r;  left = r - K x;  t = D^-1 left;  u = left - w K t;  rc = P0' u
 // (P' = P0' (I - w K D^-1), P = (I - w D^-1 K) P0, bodies.rs:238-247).
 template <class T>
-void level0_down(Context& ctx, const Batch& b, const T* r, T* x, T* left, T* t, T* u, T* rc, const int32_t* done) {
+void level0_down(Context& ctx, const Batch& b, const T* r, T* x, T* left, T* t, T* u, T* rc, T* xc, const int32_t* done) {
     const Grid0& g = b.grid;
     const Level& L = b.levels[0];
     const Level& C = b.levels[1];
-    const int32_t* skip = L.top_of_part.get();
+    const int32_t* skip = L.top_h.empty() ? nullptr : L.top_of_part.get();
     double vb = (double)sizeof(T) * 6.0 * (double)L.n;
     {
         ProfScope ps(ctx, sizeof(T) == 8 ? SC_FAM_SMOOTH64 : SC_FAM_SMOOTH32, 2 * vb + 8.0 * L.n);
@@ -966,8 +998,10 @@ void level0_down(Context& ctx, const Batch& b, const T* r, T* x, T* left, T* t, 
         ProfScope ps(ctx, sizeof(T) == 8 ? SC_FAM_TRANSFER64 : SC_FAM_TRANSFER32, vb + (double)sizeof(T) * 3 * L.n +
                      (double)sizeof(T) * 6 * C.n);
         const T* rv = sizeof(T) == 8 ? (const T*)L.mf_r.get() : (const T*)L.mf_r32.get();
-        k_p0t<T><<<grid_for(C.n, 256), 256, 0, ctx.stream>>>(C.n, L.mem_off.get(), L.mem.get(), rv, u, rc,
-                                                             C.piece.get(), done);
+        k_p0t<T><<<grid_for(C.n, 128), 128, 0, ctx.stream>>>(C.n, L.mem_off.get(), L.mem.get(), rv, u, rc,
+                                                             b.npieces == 1 ? nullptr : C.piece.get(), done,
+                                                             sizeof(T) == 8 ? (const T*)C.inv.get() : (const T*)C.inv32.get(),
+                                                             C.step.get(), xc);
         SC_LAUNCH_CK();
     }
 }
@@ -977,7 +1011,7 @@ void level0_down(Context& ctx, const Batch& b, const T* r, T* x, T* left, T* t, 
 template <class T>
 void level0_up(Context& ctx, const Batch& b, const T* r, T* x, T* e, const T* zc, T* z, const int32_t* done) {
     const Level& L = b.levels[0];
-    const int32_t* skip = L.top_of_part.get();
+    const int32_t* skip = L.top_h.empty() ? nullptr : L.top_of_part.get();
     double vb = (double)sizeof(T) * 6.0 * (double)L.n;
     {
         ProfScope ps(ctx, sizeof(T) == 8 ? SC_FAM_TRANSFER64 : SC_FAM_TRANSFER32, vb + (double)sizeof(T) * 3 * L.n +
@@ -998,15 +1032,15 @@ void level0_up(Context& ctx, const Batch& b, const T* r, T* x, T* e, const T* zc
 template <class T>
 void level0_smooth(Context& ctx, const Batch& b, const T* r, const T* x, T* z, const int32_t* done) {
     const Level& L = b.levels[0];
-    launch_stencil<T, ST_SMOOTH>(ctx, b, x, r, z, nullptr, L.step.get(), L.top_of_part.get(), done, 3);
+    launch_stencil<T, ST_SMOOTH>(ctx, b, x, r, z, nullptr, L.step.get(), L.top_h.empty() ? nullptr : L.top_of_part.get(), done, 3);
 }
 template void level0_smooth<double>(Context&, const Batch&, const double*, const double*, double*, const int32_t*);
 template void level0_smooth<float>(Context&, const Batch&, const float*, const float*, float*, const int32_t*);
 
 template void level0_down<double>(Context&, const Batch&, const double*, double*, double*, double*, double*, double*,
-                                  const int32_t*);
+                                  double*, const int32_t*);
 template void level0_down<float>(Context&, const Batch&, const float*, float*, float*, float*, float*, float*,
-                                 const int32_t*);
+                                 float*, const int32_t*);
 template void level0_up<double>(Context&, const Batch&, const double*, double*, double*, const double*, double*,
                                 const int32_t*);
 template void level0_up<float>(Context&, const Batch&, const float*, float*, float*, const float*, float*,

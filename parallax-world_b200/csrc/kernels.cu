@@ -16,16 +16,17 @@ __global__ void __launch_bounds__(256) k_spmv(int64_t nrows, const int64_t* __re
                                               const T* __restrict__ x, const T* __restrict__ r, T* __restrict__ y,
                                               const T* __restrict__ inv, const double* __restrict__ step,
                                               const int32_t* __restrict__ piece, const int32_t* __restrict__ skip_row,
-                                              const int32_t* __restrict__ done) {
+                                              const int32_t* __restrict__ done, T* __restrict__ y2) {
     int64_t row = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     if (row >= nrows) return;
     int lane = threadIdx.x & 31;
-    if (skip_row && skip_row[row]) return;
+    // the loads that wait for nothing, before the checks that wait for some of them
+    int64_t e0 = rowptr[row], e1 = rowptr[row + 1];
+    const int32_t skip = skip_row ? skip_row[row] : 0;
     int p = piece ? piece[row] : 0;
-    if (done && done[p]) return;
+    if (skip || (done && done[p])) return;
     int g = lane >> 3, rr = lane & 7;
     T acc = T(0);
-    int64_t e0 = rowptr[row], e1 = rowptr[row + 1];
     if (rr < 6) {
         // two of the slot's blocks (e, e + 4) loaded before either is used: 8 blocks in
         // flight per warp; the lane still adds its blocks in the order e0 + g, + 4, + 8, ...
@@ -61,7 +62,7 @@ __global__ void __launch_bounds__(256) k_spmv(int64_t nrows, const int64_t* __re
     } else if (MODE == SPMV_RES) {
         if (lane < 6) y[6 * row + lane] = r[6 * row + lane] - acc;
     } else {
-        T left = (lane < 6) ? r[6 * row + lane] - acc : T(0);
+        T left = lane >= 6 ? T(0) : MODE == SPMV_Y_JACOBI ? acc : r[6 * row + lane] - acc;
         T l6[6];
 #pragma unroll
         for (int c = 0; c < 6; c++) l6[c] = __shfl_sync(0xffffffffu, left, c);
@@ -70,7 +71,12 @@ __global__ void __launch_bounds__(256) k_spmv(int64_t nrows, const int64_t* __re
             T s = T(0);
 #pragma unroll
             for (int c = 0; c < 6; c++) s = fma(d[c], l6[c], s);
-            y[6 * row + lane] = x[6 * row + lane] + (T)step[p] * s;
+            if (MODE == SPMV_Y_JACOBI) {
+                y[6 * row + lane] = acc;
+                y2[6 * row + lane] = s * (T)step[p];
+            } else {
+                y[6 * row + lane] = x[6 * row + lane] + (T)step[p] * s;
+            }
         }
     }
 }
@@ -84,21 +90,26 @@ __global__ void __launch_bounds__(32 * (WPR > 8 ? WPR : 8)) k_spmv_split(
     int64_t nrows, const int64_t* __restrict__ rowptr, const int32_t* __restrict__ col, const T* __restrict__ val,
     const T* __restrict__ x, const T* __restrict__ r, T* __restrict__ y, const T* __restrict__ inv,
     const double* __restrict__ step, const int32_t* __restrict__ piece, const int32_t* __restrict__ skip_row,
-    const int32_t* __restrict__ done) {
+    const int32_t* __restrict__ done, T* __restrict__ y2) {
     constexpr int RPC = WPR >= 8 ? 1 : 8 / WPR;  // rows per thread block
     constexpr int STRIDE = 4 * WPR;
     __shared__ T part[RPC * WPR][6];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int wr = warp % WPR;
     const int64_t row = (int64_t)blockIdx.x * RPC + warp / WPR;
-    bool active = row < nrows && !(skip_row && skip_row[row]);
-    const int p = active && piece ? piece[row] : 0;
-    if (active && done && done[p]) active = false;
+    bool active = row < nrows;
+    int64_t e0 = 0, e1 = 0;
+    int32_t skip = 0, p = 0;
+    if (active) {  // the loads that wait for nothing, before the checks that wait for some of them
+        e0 = rowptr[row], e1 = rowptr[row + 1];
+        if (skip_row) skip = skip_row[row];
+        if (piece) p = piece[row];
+        active = !(skip || (done && done[p]));
+    }
     const int g = lane >> 3, rr = lane & 7;
     T acc = T(0);
     if (active && rr < 6) {
-        const int64_t e1 = rowptr[row + 1];
-        int64_t e = rowptr[row] + 4 * wr + g;
+        int64_t e = e0 + 4 * wr + g;
         for (; e + STRIDE < e1; e += 2 * STRIDE) {
             int32_t j0 = col[e], j1 = col[e + STRIDE];
             T a0[6], x0[6], a1[6], x1[6];
@@ -136,7 +147,7 @@ __global__ void __launch_bounds__(32 * (WPR > 8 ? WPR : 8)) k_spmv_split(
     } else if (MODE == SPMV_RES) {
         if (lane < 6) y[6 * row + lane] = r[6 * row + lane] - acc;
     } else {
-        T left = (lane < 6) ? r[6 * row + lane] - acc : T(0);
+        T left = lane >= 6 ? T(0) : MODE == SPMV_Y_JACOBI ? acc : r[6 * row + lane] - acc;
         T l6[6];
 #pragma unroll
         for (int c = 0; c < 6; c++) l6[c] = __shfl_sync(0xffffffffu, left, c);
@@ -145,7 +156,12 @@ __global__ void __launch_bounds__(32 * (WPR > 8 ? WPR : 8)) k_spmv_split(
             T s = T(0);
 #pragma unroll
             for (int c = 0; c < 6; c++) s = fma(d[c], l6[c], s);
-            y[6 * row + lane] = x[6 * row + lane] + (T)step[p] * s;
+            if (MODE == SPMV_Y_JACOBI) {
+                y[6 * row + lane] = acc;
+                y2[6 * row + lane] = s * (T)step[p];
+            } else {
+                y[6 * row + lane] = x[6 * row + lane] + (T)step[p] * s;
+            }
         }
     }
 }
@@ -160,17 +176,22 @@ __global__ void __launch_bounds__(256) k_spmv_half(int64_t nrows, const int64_t*
                                                    const T* __restrict__ inv, const double* __restrict__ step,
                                                    const int32_t* __restrict__ piece,
                                                    const int32_t* __restrict__ skip_row,
-                                                   const int32_t* __restrict__ done) {
+                                                   const int32_t* __restrict__ done, T* __restrict__ y2) {
     const int64_t row = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 4;
     const int lane = threadIdx.x & 31, h = lane & 16, hl = lane & 15;
-    bool active = row < nrows && !(skip_row && skip_row[row]);
-    const int p = active && piece ? piece[row] : 0;
-    if (active && done && done[p]) active = false;
+    bool active = row < nrows;
+    int64_t e0 = 0, e1 = 0;
+    int32_t skip = 0, p = 0;
+    if (active) {
+        e0 = rowptr[row], e1 = rowptr[row + 1];
+        if (skip_row) skip = skip_row[row];
+        if (piece) p = piece[row];
+        active = !(skip || (done && done[p]));
+    }
     const int g = hl >> 3, rr = hl & 7;
     T acc = T(0);
     if (active && rr < 6) {
-        const int64_t e1 = rowptr[row + 1];
-        int64_t e = rowptr[row] + g;
+        int64_t e = e0 + g;
         for (; e + 2 < e1; e += 4) {
             int32_t j0 = col[e], j1 = col[e + 2];
             T a0[6], x0[6], a1[6], x1[6];
@@ -201,7 +222,7 @@ __global__ void __launch_bounds__(256) k_spmv_half(int64_t nrows, const int64_t*
     } else if (MODE == SPMV_RES) {
         if (active && hl < 6) y[6 * row + hl] = r[6 * row + hl] - acc;
     } else {
-        T left = (active && hl < 6) ? r[6 * row + hl] - acc : T(0);
+        T left = !(active && hl < 6) ? T(0) : MODE == SPMV_Y_JACOBI ? acc : r[6 * row + hl] - acc;
         T l6[6];
 #pragma unroll
         for (int c = 0; c < 6; c++) l6[c] = __shfl_sync(0xffffffffu, left, h + c);
@@ -210,7 +231,12 @@ __global__ void __launch_bounds__(256) k_spmv_half(int64_t nrows, const int64_t*
             T s = T(0);
 #pragma unroll
             for (int c = 0; c < 6; c++) s = fma(d[c], l6[c], s);
-            y[6 * row + hl] = x[6 * row + hl] + (T)step[p] * s;
+            if (MODE == SPMV_Y_JACOBI) {
+                y[6 * row + hl] = acc;
+                y2[6 * row + hl] = s * (T)step[p];
+            } else {
+                y[6 * row + hl] = x[6 * row + hl] + (T)step[p] * s;
+            }
         }
     }
 }
@@ -221,11 +247,11 @@ __global__ void k_jacobi(int64_t n, const T* __restrict__ inv, const T* __restri
                          const int32_t* __restrict__ skip_row, const int32_t* __restrict__ done) {
     int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (k >= n) return;
-    if (skip_row && skip_row[k]) return;
-    int p = piece ? piece[k] : 0;
-    if (done && done[p]) return;
     T rv[6], o[6];
     ld6<T>(r + 6 * k, rv);
+    const int32_t skip = skip_row ? skip_row[k] : 0;
+    int p = piece ? piece[k] : 0;
+    if (skip || (done && done[p])) return;
     T st = step ? (T)step[p] : T(1);
     const T* d = inv + 36 * k;
 #pragma unroll
@@ -262,54 +288,43 @@ __global__ void k_jacobi_add(int64_t n, const T* __restrict__ inv, const T* __re
     st6<T>(z + 6 * k, o);
 }
 
-// rc[c] = sum over P entries e in column c (fine row k) of P[e]' left[k].
+// z = Kinv r over each top piece's parts, FP64 arithmetic: row i adds A[j][i] r[j] in the
+// order of j. What bounds it is that chain and the loads it waits for (a warp alone gets one
+// load in some 55 cycles), so 32 rows are a block whose eight warps bring TOP_TILE values of j
+// to shared memory at a time and whose first warp runs the chain: a 96-row top 30 to 4.6 us, a
+// 132-row one 41 to 6.6 (before, one block a piece, each thread waiting for its own loads).
+constexpr int TOP_TILE = 128;
 template <class T>
-__global__ void __launch_bounds__(256) k_restrict(int64_t nc, const int64_t* __restrict__ tptr,
-                                                  const int64_t* __restrict__ tent, const int32_t* __restrict__ trow,
-                                                  const T* __restrict__ pval, const T* __restrict__ left,
-                                                  T* __restrict__ rc, const int32_t* __restrict__ piece_c,
-                                                  const int32_t* __restrict__ done) {
-    int64_t c = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    if (c >= nc) return;
-    int lane = threadIdx.x & 31;
-    if (done && done[piece_c[c]]) return;
-    int g = lane >> 3, rr = lane & 7;
-    T acc = T(0);
-    if (rr < 6) {
-        for (int64_t t = tptr[c] + g; t < tptr[c + 1]; t += 4) {
-            int64_t e = tent[t];
-            int32_t k = trow[t];
-            T lv[6];
-            ld6<T>(left + 6 * (int64_t)k, lv);
-            const T* b = pval + 36 * e + rr;
-#pragma unroll
-            for (int j = 0; j < 6; j++) acc = fma(b[6 * j], lv[j], acc);
-        }
-    }
-    acc += __shfl_xor_sync(0xffffffffu, acc, 8);
-    acc += __shfl_xor_sync(0xffffffffu, acc, 16);
-    if (lane < 6) rc[6 * c + lane] = acc;
-}
-
-// z = Kinv r over each top piece's parts; one block per piece, FP64 arithmetic.
-template <class T>
-__global__ void __launch_bounds__(512) k_top_solve(const int32_t* __restrict__ top, const int64_t* __restrict__ pstart,
+__global__ void __launch_bounds__(256) k_top_solve(const int32_t* __restrict__ top, const int64_t* __restrict__ pstart,
                                                    const int64_t* __restrict__ kinv_off, const double* __restrict__ kinv,
                                                    const T* __restrict__ r, T* __restrict__ z,
                                                    const int32_t* __restrict__ done) {
-    extern __shared__ double rs[];
-    int p = top[blockIdx.x];
-    if (done && done[p]) return;
-    int64_t k0 = pstart[p];
-    int n = (int)(6 * (pstart[p + 1] - k0));
-    const double* A = kinv + kinv_off[blockIdx.x];
-    for (int i = threadIdx.x; i < n; i += blockDim.x) rs[i] = (double)r[6 * k0 + i];
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        double s = 0.0;
-        for (int j = 0; j < n; j++) s = fma(A[(int64_t)j * n + i], rs[j], s);
-        z[6 * k0 + i] = (T)s;
+    __shared__ double tile[TOP_TILE][32], rs[TOP_TILE];
+    const int p = top[blockIdx.x], w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    const int64_t k0 = pstart[p], off = kinv_off[blockIdx.x];
+    const int n = (int)(6 * (pstart[p + 1] - k0)), i = blockIdx.y * 32 + l;
+    if ((done && done[p]) || (int)blockIdx.y * 32 >= n) return;
+    const double* A = kinv + off + i;
+    double s = 0.0;
+    for (int j0 = 0; j0 < n; j0 += TOP_TILE) {
+        if (j0) __syncthreads();
+        double a[TOP_TILE / 8];
+#pragma unroll
+        for (int k = 0; k < TOP_TILE / 8; k++) {
+            const int j = j0 + w + 8 * k;
+            a[k] = j < n && i < n ? __ldg(A + (int64_t)j * n) : 0.0;
+        }
+        if (threadIdx.x < TOP_TILE && j0 + (int)threadIdx.x < n) rs[threadIdx.x] = (double)r[6 * k0 + j0 + threadIdx.x];
+#pragma unroll
+        for (int k = 0; k < TOP_TILE / 8; k++) tile[w + 8 * k][l] = a[k];
+        __syncthreads();
+        if (w == 0) {
+            const int m = min(TOP_TILE, n - j0);
+#pragma unroll 16
+            for (int j = 0; j < m; j++) s = fma(tile[j][l], rs[j], s);
+        }
     }
+    if (w == 0 && i < n) z[6 * k0 + i] = (T)s;
 }
 
 // out[p] = sum over piece p's parts of a.b
@@ -329,26 +344,19 @@ __global__ void __launch_bounds__(RED_LANES) k_seg_dot(Chunks ch, const T* __res
 template <class T, int WPR>
 void launch_split(Context& ctx, int mode, int64_t nrows, const int64_t* rowptr, const int32_t* col, const T* val,
                   const T* x, const T* r, T* y, const T* inv, const double* step, const int32_t* piece,
-                  const int32_t* skip_row, const int32_t* done) {
+                  const int32_t* skip_row, const int32_t* done, T* y2) {
     constexpr int RPC = WPR >= 8 ? 1 : 8 / WPR;
     constexpr int threads = 32 * (WPR > 8 ? WPR : 8);
     const unsigned g = grid_for(nrows, RPC);
+    auto go = [&](auto kernel) {
+        kernel<<<g, threads, 0, ctx.stream>>>(nrows, rowptr, col, val, x, r, y, inv, step, piece, skip_row, done, y2);
+    };
     switch (mode) {
-        case SPMV_Y:
-            k_spmv_split<T, SPMV_Y, WPR><<<g, threads, 0, ctx.stream>>>(nrows, rowptr, col, val, x, r, y, inv, step,
-                                                                         piece, skip_row, done);
-            break;
-        case SPMV_ADD:
-            k_spmv_split<T, SPMV_ADD, WPR><<<g, threads, 0, ctx.stream>>>(nrows, rowptr, col, val, x, r, y, inv, step,
-                                                                           piece, skip_row, done);
-            break;
-        case SPMV_RES:
-            k_spmv_split<T, SPMV_RES, WPR><<<g, threads, 0, ctx.stream>>>(nrows, rowptr, col, val, x, r, y, inv, step,
-                                                                           piece, skip_row, done);
-            break;
-        default:
-            k_spmv_split<T, SPMV_RES_SMOOTH, WPR><<<g, threads, 0, ctx.stream>>>(nrows, rowptr, col, val, x, r, y, inv,
-                                                                                  step, piece, skip_row, done);
+        case SPMV_Y: go(k_spmv_split<T, SPMV_Y, WPR>); break;
+        case SPMV_ADD: go(k_spmv_split<T, SPMV_ADD, WPR>); break;
+        case SPMV_RES: go(k_spmv_split<T, SPMV_RES, WPR>); break;
+        case SPMV_Y_JACOBI: go(k_spmv_split<T, SPMV_Y_JACOBI, WPR>); break;
+        default: go(k_spmv_split<T, SPMV_RES_SMOOTH, WPR>);
     }
     SC_LAUNCH_CK();
 }
@@ -374,53 +382,31 @@ static int warps_per_row(int64_t nrows, int64_t nnz) {
 template <class T>
 void spmv(Context& ctx, int mode, int64_t nrows, const int64_t* rowptr, const int32_t* col, const T* val, const T* x,
           const T* r, T* y, const T* inv, const double* step, const int32_t* piece, const int32_t* skip_row,
-          const int32_t* done, int64_t nnz) {
+          const int32_t* done, int64_t nnz, T* y2) {
     if (nrows <= 0) return;
     const int wpr = nnz > 0 ? warps_per_row(nrows, nnz) : 1;
-    if (wpr == 0) {
-        const unsigned gh = grid_for(nrows * 16, 256);
-        switch (mode) {
-            case SPMV_Y:
-                k_spmv_half<T, SPMV_Y><<<gh, 256, 0, ctx.stream>>>(nrows, rowptr, col, val, x, r, y, inv, step, piece,
-                                                                   skip_row, done);
-                break;
-            case SPMV_ADD:
-                k_spmv_half<T, SPMV_ADD><<<gh, 256, 0, ctx.stream>>>(nrows, rowptr, col, val, x, r, y, inv, step,
-                                                                     piece, skip_row, done);
-                break;
-            case SPMV_RES:
-                k_spmv_half<T, SPMV_RES><<<gh, 256, 0, ctx.stream>>>(nrows, rowptr, col, val, x, r, y, inv, step,
-                                                                     piece, skip_row, done);
-                break;
-            default:
-                k_spmv_half<T, SPMV_RES_SMOOTH><<<gh, 256, 0, ctx.stream>>>(nrows, rowptr, col, val, x, r, y, inv,
-                                                                            step, piece, skip_row, done);
-        }
-        SC_LAUNCH_CK();
-        return;
-    }
+    auto split = [&](auto launch) {
+        launch(ctx, mode, nrows, rowptr, col, val, x, r, y, inv, step, piece, skip_row, done, y2);
+    };
     switch (wpr) {
-        case 2: return launch_split<T, 2>(ctx, mode, nrows, rowptr, col, val, x, r, y, inv, step, piece, skip_row, done);
-        case 4: return launch_split<T, 4>(ctx, mode, nrows, rowptr, col, val, x, r, y, inv, step, piece, skip_row, done);
-        case 8: return launch_split<T, 8>(ctx, mode, nrows, rowptr, col, val, x, r, y, inv, step, piece, skip_row, done);
-        case 16: return launch_split<T, 16>(ctx, mode, nrows, rowptr, col, val, x, r, y, inv, step, piece, skip_row, done);
-        case 32: return launch_split<T, 32>(ctx, mode, nrows, rowptr, col, val, x, r, y, inv, step, piece, skip_row, done);
+        case 2: return split(launch_split<T, 2>);
+        case 4: return split(launch_split<T, 4>);
+        case 8: return split(launch_split<T, 8>);
+        case 16: return split(launch_split<T, 16>);
+        case 32: return split(launch_split<T, 32>);
         default: break;
     }
-    unsigned g = grid_for(nrows * 32, 256);
+    const unsigned g = grid_for(nrows * (wpr == 0 ? 16 : 32), 256);
+    auto go = [&](auto half, auto whole) {
+        (wpr == 0 ? half : whole)<<<g, 256, 0, ctx.stream>>>(nrows, rowptr, col, val, x, r, y, inv, step, piece,
+                                                             skip_row, done, y2);
+    };
     switch (mode) {
-        case SPMV_Y:
-            k_spmv<T, SPMV_Y><<<g, 256, 0, ctx.stream>>>(nrows, rowptr, col, val, x, r, y, inv, step, piece, skip_row, done);
-            break;
-        case SPMV_ADD:
-            k_spmv<T, SPMV_ADD><<<g, 256, 0, ctx.stream>>>(nrows, rowptr, col, val, x, r, y, inv, step, piece, skip_row, done);
-            break;
-        case SPMV_RES:
-            k_spmv<T, SPMV_RES><<<g, 256, 0, ctx.stream>>>(nrows, rowptr, col, val, x, r, y, inv, step, piece, skip_row, done);
-            break;
-        default:
-            k_spmv<T, SPMV_RES_SMOOTH><<<g, 256, 0, ctx.stream>>>(nrows, rowptr, col, val, x, r, y, inv, step, piece,
-                                                                  skip_row, done);
+        case SPMV_Y: go(k_spmv_half<T, SPMV_Y>, k_spmv<T, SPMV_Y>); break;
+        case SPMV_ADD: go(k_spmv_half<T, SPMV_ADD>, k_spmv<T, SPMV_ADD>); break;
+        case SPMV_RES: go(k_spmv_half<T, SPMV_RES>, k_spmv<T, SPMV_RES>); break;
+        case SPMV_Y_JACOBI: go(k_spmv_half<T, SPMV_Y_JACOBI>, k_spmv<T, SPMV_Y_JACOBI>); break;
+        default: go(k_spmv_half<T, SPMV_RES_SMOOTH>, k_spmv<T, SPMV_RES_SMOOTH>);
     }
     SC_LAUNCH_CK();
 }
@@ -442,23 +428,14 @@ void jacobi_add(Context& ctx, int64_t n, const T* inv, const T* left, const T* x
 }
 
 template <class T>
-void restrict_t(Context& ctx, int64_t nc, const int64_t* tptr, const int64_t* tent, const int32_t* trow,
-                const T* pval, const T* left, T* rc, const int32_t* piece_c, const int32_t* done) {
-    if (nc <= 0) return;
-    k_restrict<T><<<grid_for(nc * 32, 256), 256, 0, ctx.stream>>>(nc, tptr, tent, trow, pval, left, rc, piece_c, done);
-    SC_LAUNCH_CK();
-}
-
-template <class T>
 void top_solve(Context& ctx, const Level& L, const T* r, T* z, const int32_t* done) {
     if (L.top_h.empty()) return;
     int64_t maxn = 0;
     for (int p : L.top_h) maxn = std::max<int64_t>(maxn, 6 * (L.pstart[p + 1] - L.pstart[p]));
-    size_t sm = (size_t)std::max<int64_t>(maxn, 1) * sizeof(double);
-    if (sm > 48 * 1024)
-        SC_CK(cudaFuncSetAttribute(k_top_solve<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    k_top_solve<T><<<(unsigned)L.top_h.size(), 512, sm, ctx.stream>>>(L.top.get(), L.pstart_d.get(), L.kinv_off.get(),
-                                                                       L.kinv.get(), r, z, done);
+    if (maxn <= 0) return;
+    const dim3 grid((unsigned)L.top_h.size(), grid_for(maxn, 32));
+    k_top_solve<T><<<grid, 256, 0, ctx.stream>>>(L.top.get(), L.pstart_d.get(), L.kinv_off.get(), L.kinv.get(), r, z,
+                                                 done);
     SC_LAUNCH_CK();
 }
 
@@ -506,13 +483,11 @@ void seg_dot(Context& ctx, const Level& L, const double* a, const double* b, dou
 
 #define SC_INST(T)                                                                                                 \
     template void spmv<T>(Context&, int, int64_t, const int64_t*, const int32_t*, const T*, const T*, const T*, T*, \
-                          const T*, const double*, const int32_t*, const int32_t*, const int32_t*, int64_t);       \
+                          const T*, const double*, const int32_t*, const int32_t*, const int32_t*, int64_t, T*);   \
     template void jacobi<T>(Context&, int64_t, const T*, const T*, T*, const double*, const int32_t*,              \
                             const int32_t*, const int32_t*);                                                       \
     template void jacobi_add<T>(Context&, int64_t, const T*, const T*, const T*, T*, const double*, const int32_t*, \
                                 const int32_t*, const int32_t*);                                                   \
-    template void restrict_t<T>(Context&, int64_t, const int64_t*, const int64_t*, const int32_t*, const T*,       \
-                                const T*, T*, const int32_t*, const int32_t*);                                     \
     template void top_solve<T>(Context&, const Level&, const T*, T*, const int32_t*);                             \
     template void seg_dot_t<T>(Context&, const Level&, const T*, const T*, double*);
 SC_INST(double)

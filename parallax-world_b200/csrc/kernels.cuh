@@ -5,7 +5,8 @@
 
 namespace sc {
 
-enum SpmvMode { SPMV_Y = 0, SPMV_ADD = 1, SPMV_RES = 2, SPMV_RES_SMOOTH = 3 };
+// y = A x;  y += A x;  y = r - A x;  y = x + step D^-1 (r - A x);  y = A x and y2 = step D^-1 y
+enum SpmvMode { SPMV_Y = 0, SPMV_ADD = 1, SPMV_RES = 2, SPMV_RES_SMOOTH = 3, SPMV_Y_JACOBI = 4 };
 
 __device__ __forceinline__ int64_t lower_bound_i32(const int32_t* __restrict__ a, int64_t lo, int64_t hi, int32_t v) {
     while (lo < hi) {
@@ -184,7 +185,7 @@ Chunks red_chunks(Context& ctx, const Level& L);
 template <class T>
 void spmv(Context& ctx, int mode, int64_t nrows, const int64_t* rowptr, const int32_t* col, const T* val, const T* x,
           const T* r, T* y, const T* inv, const double* step, const int32_t* piece, const int32_t* skip_row,
-          const int32_t* done, int64_t nnz = 0);
+          const int32_t* done, int64_t nnz = 0, T* y2 = nullptr);
 template <class T>
 void jacobi(Context& ctx, int64_t n, const T* inv, const T* r, T* x, const double* step, const int32_t* piece,
             const int32_t* skip_row, const int32_t* done);
@@ -192,9 +193,6 @@ void jacobi(Context& ctx, int64_t n, const T* inv, const T* r, T* x, const doubl
 template <class T>
 void jacobi_add(Context& ctx, int64_t n, const T* inv, const T* left, const T* x, T* z, const double* step,
                 const int32_t* piece, const int32_t* skip_row, const int32_t* done);
-template <class T>
-void restrict_t(Context& ctx, int64_t ncoarse, const int64_t* tptr, const int64_t* tent, const int32_t* trow,
-                const T* pval, const T* left, T* rc, const int32_t* piece_c, const int32_t* done);
 template <class T>
 void top_solve(Context& ctx, const Level& L, const T* r, T* z, const int32_t* done);
 // out[p] = sum over piece p's parts of a.b (6 values a part), deterministic.

@@ -159,7 +159,8 @@ void stencil_residual(Context& ctx, const Batch& b, const T* x, const T* r, T* y
                       const int32_t* done);
 void grid_cell_energy(Context& ctx, const Batch& b, const double* x, double* energy_cells);
 template <class T>
-void level0_down(Context& ctx, const Batch& b, const T* r, T* x, T* left, T* t, T* u, T* rc, const int32_t* done);
+void level0_down(Context& ctx, const Batch& b, const T* r, T* x, T* left, T* t, T* u, T* rc, T* xc,
+                 const int32_t* done);
 template <class T>
 void level0_up(Context& ctx, const Batch& b, const T* r, T* x, T* e, const T* zc, T* z, const int32_t* done);
 template <class T>
