@@ -517,67 +517,132 @@ __global__ void __launch_bounds__(SUM_THREADS) k_sum_products(int64_t nout, cons
     for (int r = 0; r < 6; r++) out[36 * q + 6 * r + c] = acc[r];
 }
 
-// The same for K P on a matrix-free level 0: the left block of contribution (e << 32 | f)
-// is block e of the level-0 pattern, made from the cell template (krow gives its row),
-// the right one block f of P. Thread c of a group owns column c of the output block as
-// above, but makes only row c of each template block and takes the other rows from its
-// group's lanes by shuffles, so the groups sit inside warps: five to a warp, two lanes
-// idle. Blocks stay resident, striding over the outputs (the template is staged once
-// per block).
-constexpr int K0SUM_WARPS = 6;
-constexpr int K0SUM_GROUPS = 5 * K0SUM_WARPS;
-template <class TB, class TO>
-__global__ void __launch_bounds__(32 * K0SUM_WARPS) k_sum_products_k0(int64_t nout, const int64_t* __restrict__ seg,
-                                                                     const uint64_t* __restrict__ vals,
-                                                                     const TB* __restrict__ B,
-                                                                     TO* __restrict__ out, K0View k0,
-                                                                     const int32_t* __restrict__ krow) {
-    __shared__ double T[36 * 36];
-    for (int t = threadIdx.x; t < 36 * 36; t += blockDim.x) T[t] = k0.tpl_s[t];
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int gl = min(lane / 6, 4), c = lane - 6 * gl;  // lanes 30, 31 shadow group 4's lanes 0, 1
-    const bool idle = lane >= 30;
-    const int base = 6 * gl;
-    const int g = 5 * warp + gl;
-    // the whole warp runs the same trip count, so the shuffles always find every lane
-    const int64_t first_q = (int64_t)blockIdx.x * K0SUM_GROUPS;
-    for (int64_t q0 = first_q; q0 < nout; q0 += (int64_t)gridDim.x * K0SUM_GROUPS) {
-        const int64_t q = q0 + g;
-        const bool live = !idle && q < nout;
-        int64_t i = live ? seg[q] : 0;
-        const int64_t end = live ? seg[q + 1] : 0;
-        K0Row row{};
-        if (i < end) row = k0_row(k0, krow[vals[i] >> 32]);
-        // the most contributions of any group of the warp
-        int64_t n = end - i, most = n;
-#pragma unroll
-        for (int o = 16; o; o >>= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
-        double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-        for (int64_t t = 0; t < most; t++) {
-            const bool has = t < n;
-            double bc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, ar[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-            if (has) {
-                const uint64_t v = vals[i + t];
-                const TB* bb = B + 36 * (int64_t)(v & 0xffffffffu);
-#pragma unroll
-                for (int j = 0; j < 6; j++) bc[j] = (double)bb[j * 6 + c];
-                const uint8_t d = k0.desc[v >> 32];
-#pragma unroll
-                for (int j = 0; j < 6; j++) ar[j] = k0_entry(T, row, d, c, j);  // row c of A
+// K P on a matrix-free level 0, a warp a row: K's row has at most 11 blocks (the faces of a
+// part's two cells), P's rows a few, so the row's pattern is a merge of at most 11 short
+// sorted lists, each on a lane: the least column left is the next output block, and the
+// lanes that hold it are its contributions, in K's order. FILL then makes the row's blocks
+// of K from the cell template once, in shared memory, and five groups of six lanes (lane c
+// owns column c) sum an output block each, its contributions' six products first and
+// then the addition, as the sorted sums do: the same bits, with no list of candidates made,
+// sorted or read. (By sorted candidates a contribution's block of K was made anew and its
+// rows passed on by 72 shuffles. A 128^3 piece, 112.7 M contributions: KP0NEW.)
+// KP0_BATCH output blocks are merged, then summed, at a time, whatever the row's length.
+constexpr int KP0_WARPS = 8, KP0_MOST = 11, KP0_BATCH = 20;
+template <bool FILL, class TB, class TO>
+__global__ void __launch_bounds__(32 * KP0_WARPS) k_kp0(int64_t n, K0View k0, const int64_t* __restrict__ rowptr,
+                                                        const int32_t* __restrict__ col,
+                                                        const int64_t* __restrict__ prow,
+                                                        const int32_t* __restrict__ pcol,
+                                                        const int32_t* __restrict__ up, int64_t* __restrict__ cnt,
+                                                        const int64_t* __restrict__ kprow, const TB* __restrict__ B,
+                                                        int32_t* __restrict__ kpcol, TO* __restrict__ out) {
+    constexpr int W = FILL ? KP0_WARPS : 1;  // the count needs no shared memory
+    __shared__ double T[FILL ? 36 * 36 : 1];
+    __shared__ __align__(16) double blocks[W][KP0_MOST * 36];
+    __shared__ int32_t entry[W][KP0_BATCH][KP0_MOST];
+    __shared__ uint32_t held[W][KP0_BATCH];
+    if (FILL) {
+        for (int t = threadIdx.x; t < 36 * 36; t += blockDim.x) T[t] = k0.tpl_s[t];
+        __syncthreads();
+    }
+    const int w = FILL ? threadIdx.x >> 5 : 0, lane = threadIdx.x & 31;
+    const int64_t k = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    if (k >= n) return;
+    if (up[k] < 0) {  // its piece is solved at level 0
+        if (!FILL && lane == 0) cnt[k] = 0;
+        return;
+    }
+    const int64_t e0 = rowptr[k];
+    const int ne = (int)(rowptr[k + 1] - e0);
+    const int32_t first = pcol[prow[k]];  // columns below P row k's first are not read later
+    int64_t f = 0, f1 = 0;
+    uint8_t d = 0;
+    constexpr int32_t NONE = 0x7fffffff;
+    if (lane < ne) {
+        const int32_t q = col[e0 + lane];
+        if (FILL) d = k0.desc[e0 + lane];
+        f = prow[q];
+        f1 = prow[q + 1];
+    }
+    // this lane's column and the one after it
+    int32_t cur = f < f1 ? pcol[f] : NONE, nxt = f + 1 < f1 ? pcol[f + 1] : NONE;
+    auto step = [&] {
+        f++;
+        cur = nxt;
+        nxt = f + 1 < f1 ? pcol[f + 1] : NONE;
+    };
+    while (cur < first) step();
+    if (!FILL) {
+        int64_t m = 0;
+        for (;; m++) {
+            const int32_t least = __reduce_min_sync(0xffffffffu, cur);
+            if (least == NONE) break;
+            if (cur == least) step();
+        }
+        if (lane == 0) cnt[k] = m;
+        return;
+    }
+    const K0Row row = k0_row(k0, k);
+    for (int t0 = 0; t0 < 36 * KP0_MOST; t0 += 32) {  // every lane, every time round: the shuffle needs all
+        const int t = t0 + lane, e = min(t / 36, KP0_MOST - 1), x = t % 36;
+        const uint8_t de = (uint8_t)__shfl_sync(0xffffffffu, (int)d, e);
+        if (t < 36 * KP0_MOST && e < ne) blocks[w][t] = k0_entry(T, row, de, x / 6, x % 6);
+    }
+    const int g = lane / 6, c = lane % 6;
+    for (int64_t q0 = kprow[k];; q0 += KP0_BATCH) {
+        int ns = 0;
+        for (; ns < KP0_BATCH; ns++) {
+            const int32_t least = __reduce_min_sync(0xffffffffu, cur);
+            if (least == NONE) break;
+            const bool mine = cur == least;
+            const uint32_t who = __ballot_sync(0xffffffffu, mine);
+            if (lane == 0) {
+                held[w][ns] = who;
+                kpcol[q0 + ns] = least;
             }
-            // acc(r) += sum_j A(r, j) B(j, c), row r of A from lane base + r
-#pragma unroll
-            for (int r = 0; r < 6; r++) {
-                double s = 0.0;
-#pragma unroll
-                for (int j = 0; j < 6; j++) s = fma(__shfl_sync(0xffffffffu, ar[j], base + r), bc[j], s);
-                if (has) acc[r] += s;
+            if (mine) {
+                entry[w][ns][lane] = (int32_t)f;
+                step();
             }
         }
-        if (live)
+        __syncwarp();
+        if (ns == 0) break;
+        int s = g < 5 ? g : ns;  // lanes 30 and 31 have no group
+        uint32_t who = s < ns ? held[w][s] : 0u;
+        double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+        while (s < ns) {
+            const int e = __ffs(who) - 1;
+            who &= who - 1u;
+            const TB* bb = B + 36 * (int64_t)entry[w][s][e] + c;
+            double bc[6];
 #pragma unroll
-            for (int r = 0; r < 6; r++) out[36 * q + 6 * r + c] = (TO)acc[r];
+            for (int j = 0; j < 6; j++) bc[j] = (double)bb[6 * j];
+            const double2* A = reinterpret_cast<const double2*>(blocks[w] + 36 * e);
+#pragma unroll
+            for (int r = 0; r < 6; r++) {
+                const double2 a0 = A[3 * r], a1 = A[3 * r + 1], a2 = A[3 * r + 2];
+                double v = 0.0;
+                v = fma(a0.x, bc[0], v);
+                v = fma(a0.y, bc[1], v);
+                v = fma(a1.x, bc[2], v);
+                v = fma(a1.y, bc[3], v);
+                v = fma(a2.x, bc[4], v);
+                v = fma(a2.y, bc[5], v);
+                acc[r] += v;
+            }
+            if (!who) {
+                TO* o = out + 36 * (q0 + s) + c;
+#pragma unroll
+                for (int r = 0; r < 6; r++) {
+                    o[6 * r] = (TO)acc[r];
+                    acc[r] = 0.0;
+                }
+                s += 5;
+                if (s < ns) who = held[w][s];
+            }
+        }
+        __syncwarp();
+        if (ns < KP0_BATCH) break;
     }
 }
 
@@ -1192,6 +1257,38 @@ static bool coarsen(Context& ctx, Batch& b, int l, int octree_level, const sc_op
         a.lo = lo.get();
         a.hi = hi.get();
         row_products(ctx, virt ? ROWS_K0 : ROWS_PLAIN, a, n, widest, kprow, kpcol, kpval, kpnnz, kp_cands);
+    } else if (virt) {
+        DBuf<int64_t> kcnt;
+        kcnt.alloc(n + 1, st, ms);
+        kprow.alloc(n + 1, st, ms);
+        SC_CK(cudaMemsetAsync(kcnt.get() + n, 0, sizeof(int64_t), st));
+        const unsigned nb = grid_for(n, KP0_WARPS);
+        k_kp0<false, double, double><<<nb, 32 * KP0_WARPS, 0, st>>>(n, k0, F.rowptr.get(), F.col.get(), F.prow.get(),
+                                                                   F.pcol.get(), F.up.get(), kcnt.get(), nullptr,
+                                                                   nullptr, nullptr, nullptr);
+        SC_LAUNCH_CK();
+        exclusive_scan(ctx, kcnt.get(), kprow.get(), n + 1);
+        kpnnz = d2h_i64(ctx, kprow.get() + n);
+        kpcol.alloc(std::max<int64_t>(kpnnz, 1), st, ms);
+        kp32 = opt.precision == SC_MIXED && !(fits && (gal == "rows" || kpnnz >= 12 * n));
+        auto fill = [&](auto* B, auto* out) {
+            using T = std::remove_pointer_t<decltype(B)>;
+            k_kp0<true, T, T><<<nb, 32 * KP0_WARPS, 0, st>>>(n, k0, F.rowptr.get(), F.col.get(), F.prow.get(),
+                                                             F.pcol.get(), F.up.get(), nullptr, kprow.get(), B,
+                                                             kpcol.get(), out);
+            SC_LAUNCH_CK();
+        };
+        if (kp32) {
+            // P too: both products read it, nothing after them (a matrix-free level 0
+            // transfers through its rigid part and the stencil)
+            to_float(ctx, F.pval, F.pval32);
+            F.pval.release();
+            kpval32.alloc(36 * std::max<int64_t>(kpnnz, 1), st, ms);
+            fill(F.pval32.get(), kpval32.get());
+        } else {
+            kpval.alloc(36 * std::max<int64_t>(kpnnz, 1), st, ms);
+            fill(F.pval.get(), kpval.get());
+        }
     } else {
         // one thread per block of K (its row from krow), offsets by a scan over K's entries
         const int64_t knz = F.nnzb;
@@ -1223,28 +1320,11 @@ static bool coarsen(Context& ctx, Batch& b, int l, int octree_level, const sc_op
         }
         koff.release();
         keys_to_csr_with(ctx, keys, vin, tot, n, nc, kprow, kpcol, kpnnz, seg, vals);
-        kp32 = virt && opt.precision == SC_MIXED && !(fits && (gal == "rows" || kpnnz >= 12 * n));
-        if (kp32) {
-            // P too: both products read it, nothing after them (a matrix-free level 0
-            // transfers through its rigid part and the stencil)
-            to_float(ctx, F.pval, F.pval32);
-            F.pval.release();
-            kpval32.alloc(36 * std::max<int64_t>(kpnnz, 1), st, ms);
-        } else {
-            kpval.alloc(36 * std::max<int64_t>(kpnnz, 1), st, ms);
-        }
+        kpval.alloc(36 * std::max<int64_t>(kpnnz, 1), st, ms);
         if (kpnnz > 0) {
             unsigned nb = (unsigned)((kpnnz + SUM_GROUPS - 1) / SUM_GROUPS);
-            const unsigned nb0 = std::min((unsigned)((kpnnz + K0SUM_GROUPS - 1) / K0SUM_GROUPS), 148u * 8u);
-            if (virt && kp32)
-                k_sum_products_k0<float, float><<<nb0, 32 * K0SUM_WARPS, 0, st>>>(
-                    kpnnz, seg.get(), vals.get(), F.pval32.get(), kpval32.get(), k0, krow.get());
-            else if (virt)
-                k_sum_products_k0<double, double><<<nb0, 32 * K0SUM_WARPS, 0, st>>>(
-                    kpnnz, seg.get(), vals.get(), F.pval.get(), kpval.get(), k0, krow.get());
-            else
-                k_sum_products<false, double, double><<<nb, SUM_THREADS, 0, st>>>(
-                    kpnnz, seg.get(), vals.get(), F.val.get(), F.pval.get(), kpval.get());
+            k_sum_products<false, double, double><<<nb, SUM_THREADS, 0, st>>>(kpnnz, seg.get(), vals.get(), F.val.get(),
+                                                                             F.pval.get(), kpval.get());
             SC_LAUNCH_CK();
         }
     }
