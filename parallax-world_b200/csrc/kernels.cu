@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(256) k_spmv(int64_t nrows, const int64_t* __re
             for (int c = 0; c < 6; c++) s = fma(d[c], l6[c], s);
             if (MODE == SPMV_Y_JACOBI) {
                 y[6 * row + lane] = acc;
-                y2[6 * row + lane] = s * (T)step[p];
+                y2[6 * row + lane] = s * (step ? (T)step[p] : T(1));
             } else {
                 y[6 * row + lane] = x[6 * row + lane] + (T)step[p] * s;
             }
@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(32 * (WPR > 8 ? WPR : 8)) k_spmv_split(
             for (int c = 0; c < 6; c++) s = fma(d[c], l6[c], s);
             if (MODE == SPMV_Y_JACOBI) {
                 y[6 * row + lane] = acc;
-                y2[6 * row + lane] = s * (T)step[p];
+                y2[6 * row + lane] = s * (step ? (T)step[p] : T(1));
             } else {
                 y[6 * row + lane] = x[6 * row + lane] + (T)step[p] * s;
             }
@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(256) k_spmv_half(int64_t nrows, const int64_t*
             for (int c = 0; c < 6; c++) s = fma(d[c], l6[c], s);
             if (MODE == SPMV_Y_JACOBI) {
                 y[6 * row + hl] = acc;
-                y2[6 * row + hl] = s * (T)step[p];
+                y2[6 * row + hl] = s * (step ? (T)step[p] : T(1));
             } else {
                 y[6 * row + hl] = x[6 * row + hl] + (T)step[p] * s;
             }
@@ -337,6 +337,21 @@ __global__ void __launch_bounds__(RED_LANES) k_seg_dot(Chunks ch, const T* __res
         6 * ch.lo[c] + t, 6 * ch.lo[c + 1], [&](int64_t i) { return make_double2((double)a[i], (double)b[i]); },
         [&](int64_t, const double2& v) { s = fma(v.x, v.y, s); });
     if (red_finish<SPLIT>(ch, c, t, p, s, none)) out[p] = s;
+}
+
+// The last power iteration: per piece step = 4/3 / (|w| / |v|) (bodies.rs:174, 187)
+template <bool SPLIT>
+__global__ void __launch_bounds__(RED_LANES) k_power_step(Chunks ch, const double* __restrict__ w,
+                                                          const double* __restrict__ v, double* __restrict__ step) {
+    const int c = red_chunk<SPLIT>(), t = red_lane<SPLIT>(), p = ch.piece[c];
+    double ww = 0.0, vv = 0.0;
+    red_chain<SPLIT ? 16 : 8>(
+        6 * ch.lo[c] + t, 6 * ch.lo[c + 1], [&](int64_t i) { return make_double2(w[i], v[i]); },
+        [&](int64_t, const double2& x) {
+            ww = fma(x.x, x.x, ww);
+            vv = fma(x.y, x.y, vv);
+        });
+    if (red_finish<SPLIT>(ch, c, t, p, ww, vv)) step[p] = 4.0 / 3.0 / (sqrt(ww) / sqrt(vv));
 }
 
 }  // namespace
@@ -474,6 +489,20 @@ void seg_dot_t(Context& ctx, const Level& L, const T* a, const T* b, double* out
         k_seg_dot<T, true><<<grid, block, 0, ctx.stream>>>(ch, a, b, out);
     else
         k_seg_dot<T, false><<<grid, block, 0, ctx.stream>>>(ch, a, b, out);
+    SC_LAUNCH_CK();
+}
+
+void power_step(Context& ctx, const Level& L, const double* w, const double* v, double* step) {
+    const int np = (int)L.pstart.size() - 1;
+    SC_CK(cudaMemsetAsync(step, 0xff, np * sizeof(double), ctx.stream));  // NaN where a piece has no part here
+    if (L.nchunks <= 0) return;
+    const Chunks ch = red_chunks(ctx, L);
+    const unsigned grid = red_grid(L.nchunks);
+    const int block = red_block(L.nchunks);
+    if (red_split(L.nchunks))
+        k_power_step<true><<<grid, block, 0, ctx.stream>>>(ch, w, v, step);
+    else
+        k_power_step<false><<<grid, block, 0, ctx.stream>>>(ch, w, v, step);
     SC_LAUNCH_CK();
 }
 

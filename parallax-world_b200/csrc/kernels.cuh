@@ -5,7 +5,8 @@
 
 namespace sc {
 
-// y = A x;  y += A x;  y = r - A x;  y = x + step D^-1 (r - A x);  y = A x and y2 = step D^-1 y
+// y = A x;  y += A x;  y = r - A x;  y = x + step D^-1 (r - A x);  y = A x and y2 = step D^-1 y (step
+// null: 1)
 enum SpmvMode { SPMV_Y = 0, SPMV_ADD = 1, SPMV_RES = 2, SPMV_RES_SMOOTH = 3, SPMV_Y_JACOBI = 4 };
 
 __device__ __forceinline__ int64_t lower_bound_i32(const int32_t* __restrict__ a, int64_t lo, int64_t hi, int32_t v) {
@@ -198,5 +199,8 @@ void top_solve(Context& ctx, const Level& L, const T* r, T* z, const int32_t* do
 // out[p] = sum over piece p's parts of a.b (6 values a part), deterministic.
 template <class T>
 void seg_dot_t(Context& ctx, const Level& L, const T* a, const T* b, double* out);
+
+// per piece the smoother's step from the last power iteration, w = D^-1 K v
+void power_step(Context& ctx, const Level& L, const double* w, const double* v, double* step);
 
 }  // namespace sc
