@@ -73,18 +73,6 @@ template <>
 DBuf<float>& VU<float>(Level& L) { return L.u32; }
 
 template <class T>
-void level_apply(Context& ctx, const Batch& b, int l, const T* x, T* y) {
-    const Level& L = b.levels[l];
-    if (l == 0 && L.matrix_free)
-        stencil_apply<T>(ctx, b, x, y, nullptr, nullptr);
-    else
-        spmv<T>(ctx, SPMV_Y, L.n, L.rowptr.get(), L.col.get(), VAL<T>(L), x, nullptr, y, nullptr, nullptr,
-                L.piece.get(), nullptr, nullptr, L.nnzb);
-}
-template void level_apply<double>(Context&, const Batch&, int, const double*, double*);
-template void level_apply<float>(Context&, const Batch&, int, const float*, float*);
-
-template <class T>
 static void ensure(Context& ctx, DBuf<T>& v, int64_t n) {
     if ((int64_t)v.size() < n) v.alloc(std::max<int64_t>(n, 1), ctx.stream, &ctx.mem);
 }

@@ -512,7 +512,8 @@ __global__ void __launch_bounds__(SUM_THREADS) k_sum_products(int64_t nout, cons
 // owns column c) sum an output block each, its contributions' six products first and
 // then the addition, as the sorted sums do: the same bits, with no list of candidates made,
 // sorted or read. (By sorted candidates a contribution's block of K was made anew and its
-// rows passed on by 72 shuffles. A 128^3 piece, 112.7 M contributions: KP0NEW.)
+// rows passed on by 72 shuffles. On a 128^3 piece, 112.7 M contributions, that took 30 ms
+// after 12 ms of sorting; this takes 18 and 1.3 to count.)
 // KP0_BATCH output blocks are merged, then summed, at a time, whatever the row's length.
 constexpr int KP0_WARPS = 8, KP0_MOST = 11, KP0_BATCH = 20;
 template <bool FILL, class TB, class TO>
@@ -767,7 +768,8 @@ __device__ void cholesky_inverse_block(int n, double* A, double* __restrict__ X,
 }
 
 // Every listed piece's top at once, one block per piece: A_all[off[i]..] holds the dense
-// matrix on entry and its inverse on exit; X_all is scratch of the same layout.
+// matrix on entry and its inverse on exit; X_all is scratch of the same layout. For levels
+// with a top of more than TOP_MOST rows (sc_options.few well above its default).
 __global__ void __launch_bounds__(1024) k_cholesky_inverse_all(const int32_t* __restrict__ top,
                                                                const int64_t* __restrict__ pstart,
                                                                const int64_t* __restrict__ off, double* A_all,
@@ -777,6 +779,232 @@ __global__ void __launch_bounds__(1024) k_cholesky_inverse_all(const int32_t* __
     int n = (int)(6 * (pstart[p + 1] - pstart[p]));
     if (n == 0) return;
     cholesky_inverse_block(n, A_all + off[blockIdx.x], X_all + off[blockIdx.x], status, p);
+}
+
+// The same, in the same order of additions, for tops whose panels fit shared memory: every
+// sum grows as its terms become known, instead of being taken term by term when it is
+// needed, so a column's step waits for one subtraction and division instead of a chain of
+// j products read from global memory, and the rows, or columns, of a panel run side by side.
+// Panels of 32 columns: within one, column j's entries follow from its diagonal and are added
+// to the sums of the panel's later columns; after it, the panel's 32 products go to every
+// later column's sums, kept in X until the inverse needs it. A diagonal's sum of squares has
+// an order of its own: 32 at a time in a shuffle tree, the trees in turn. One block a piece;
+// a 96-row top took 450 us column by column, tops of up to
+// 384 rows 8.5 ms (0.76 ms now).
+constexpr int TOP_THREADS = 512, TOP_LD = 33, TOP_MOST = 816;
+constexpr size_t top_smem(int64_t n) { return (size_t)n * (TOP_LD + 1) * sizeof(double); }
+
+__device__ __forceinline__ double tree32(double s) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+}
+
+__device__ void top_factor(int n, double* A, double* X, double* sm, int32_t* status, int piece) {
+    double* rs = sm + (size_t)n * TOP_LD;  // per row: its squares' sum over the panels done
+    __shared__ double dsh;
+    __shared__ int bad;
+    const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
+    auto P = [&](int i, int c) -> double& { return sm[i * TOP_LD + c]; };
+    if (tid == 0) bad = 0;
+    for (int i = tid; i < n; i += TOP_THREADS) rs[i] = 0.0;
+    for (int p0 = 0; p0 < n; p0 += 32) {
+        const int pw = min(32, n - p0), pe = p0 + pw;
+        __syncthreads();
+        // the sums so far of the panel's columns
+        for (int i = p0 + w; i < n; i += TOP_THREADS / 32)
+            if (l < pw && i >= p0 + l) P(i, l) = p0 ? X[(int64_t)i * n + p0 + l] : 0.0;
+        double a0[2] = {0.0, 0.0};
+        for (int r = 0; r < 2; r++) {
+            const int i = tid + TOP_THREADS * r;
+            if (i > p0 && i < n) a0[r] = A[(int64_t)i * n + p0];
+        }
+        double dj = tid == 0 ? A[(int64_t)p0 * n + p0] : 0.0;
+        __syncthreads();
+        for (int c = 0; c < pw; c++) {
+            const int j = p0 + c;
+            if (w == 0) {
+                const double a = l < c ? P(j, l) : 0.0;
+                const double s = tree32(fma(a, a, 0.0));
+                if (l == 0) {
+                    const double v = dj - (rs[j] + s);
+                    if (!(v > 0.0)) bad = 1;
+                    dsh = sqrt(v);
+                    P(j, c) = dsh;
+                    if (c + 1 < pw) dj = A[(int64_t)(j + 1) * n + j + 1];
+                }
+            }
+            __syncthreads();
+            const double d = dsh;
+            for (int r = 0; r < 2; r++) {
+                const int i = tid + TOP_THREADS * r;
+                if (i > j && i < n) {
+                    P(i, c) = (a0[r] - P(i, c)) / d;
+                    if (i > j + 1 && c + 1 < pw) a0[r] = A[(int64_t)i * n + j + 1];
+                }
+            }
+            __syncthreads();
+            for (int r = 0; r < 2; r++) {
+                const int i = tid + TOP_THREADS * r;
+                if (i > j && i < n) {
+                    const double a = P(i, c);
+                    const int ce = min(pw, i - p0);  // columns of the panel before row i's diagonal
+#pragma unroll 4
+                    for (int q = c + 1; q < ce; q++) P(i, q) = fma(a, P(p0 + q, c), P(i, q));
+                }
+            }
+        }
+        __syncthreads();
+        for (int i = p0 + w; i < n; i += TOP_THREADS / 32) {
+            if (l < pw && i >= p0 + l) A[(int64_t)i * n + p0 + l] = P(i, l);
+            if (i >= pe) {
+                const double a = P(i, l);
+                const double s = tree32(fma(a, a, 0.0));
+                if (l == 0) rs[i] += s;
+            }
+        }
+        // the later columns' sums: a warp takes 8 rows by 64 columns at a time
+        const int m = n - pe, nti = (m + 7) / 8, ntj = (m + 63) / 64;
+        for (int t = w; t < nti * ntj; t += TOP_THREADS / 32) {
+            const int i0 = pe + 8 * (t / ntj), j0 = pe + 64 * (t % ntj);
+            if (j0 >= i0 + 8) continue;
+            const int ja = j0 + l, jb = j0 + 32 + l;
+            double ta[8], tb[8];
+#pragma unroll
+            for (int r = 0; r < 8; r++) {
+                const int i = i0 + r;
+                ta[r] = p0 && i < n && ja < i ? X[(int64_t)i * n + ja] : 0.0;
+                tb[r] = p0 && i < n && jb < i ? X[(int64_t)i * n + jb] : 0.0;
+            }
+            const double* pa = sm + min(ja, n - 1) * TOP_LD;
+            const double* pb = sm + min(jb, n - 1) * TOP_LD;
+            const double* pi[8];
+#pragma unroll
+            for (int r = 0; r < 8; r++) pi[r] = sm + min(i0 + r, n - 1) * TOP_LD;
+#pragma unroll 4
+            for (int c = 0; c < 32; c++) {
+                const double xa = pa[c], xb = pb[c];
+#pragma unroll
+                for (int r = 0; r < 8; r++) {
+                    const double xi = pi[r][c];
+                    ta[r] = fma(xi, xa, ta[r]);
+                    tb[r] = fma(xi, xb, tb[r]);
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < 8; r++) {
+                const int i = i0 + r;
+                if (i < n && ja < i) X[(int64_t)i * n + ja] = ta[r];
+                if (i < n && jb < i) X[(int64_t)i * n + jb] = tb[r];
+            }
+        }
+    }
+    __syncthreads();
+    if (tid == 0 && bad) atomicMax(status + piece, (int)SC_NOT_SPD);
+}
+
+// X = L^-1 by panels of 32 rows, a thread a column; X's 32 x 32 blocks above the diagonal
+// ones are not written.
+__device__ void top_inverse(int n, const double* A, double* X, double* sm) {
+    constexpr int LD = 34;  // even: 16-byte loads of a row
+    double* as = sm;        // [k][row]: 32 columns of the panel's rows
+    const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
+    for (int jb = 0; jb < n; jb += TOP_THREADS) {
+        const int j = jb + tid;
+        for (int p0 = jb; p0 < n; p0 += 32) {
+            const int pw = min(32, n - p0);
+            double acc[32];
+#pragma unroll
+            for (int r = 0; r < 32; r++) acc[r] = 0.0;
+            for (int k0 = jb; k0 <= p0; k0 += 32) {
+                __syncthreads();
+                for (int r = w; r < 32; r += TOP_THREADS / 32)
+                    as[l * LD + r] = r < pw && k0 + l < n ? A[(int64_t)(p0 + r) * n + k0 + l] : 0.0;
+                __syncthreads();
+                if (j >= k0 + 32 || j >= n || k0 == p0) continue;  // (k0 == p0: the panel's own block)
+#pragma unroll 4
+                for (int k = 0; k < 32; k++) {
+                    const double x = X[(int64_t)(k0 + k) * n + j];
+                    const double2* a2 = reinterpret_cast<const double2*>(as + k * LD);
+#pragma unroll
+                    for (int r = 0; r < 16; r++) {
+                        const double2 a = a2[r];
+                        acc[2 * r] = fma(a.x, x, acc[2 * r]);
+                        acc[2 * r + 1] = fma(a.y, x, acc[2 * r + 1]);
+                    }
+                }
+            }
+            if (j < min(p0 + 32, n)) {
+#pragma unroll
+                for (int r = 0; r < 32; r++) {
+                    const int i = p0 + r;
+                    if (r < pw) {
+                        const double d = as[r * LD + r];
+                        const double x = i < j ? 0.0 : i == j ? 1.0 / d : -acc[r] / d;
+                        X[(int64_t)i * n + j] = x;
+#pragma unroll
+                        for (int q = r + 1; q < 32; q++) acc[q] = fma(as[r * LD + q], x, acc[q]);
+                    }
+                }
+            }
+        }
+        __syncthreads();
+    }
+}
+
+__global__ void __launch_bounds__(TOP_THREADS) k_top_factor(const int32_t* __restrict__ top,
+                                                            const int64_t* __restrict__ pstart,
+                                                            const int64_t* __restrict__ off, double* A_all,
+                                                            double* X_all, int32_t* __restrict__ status) {
+    extern __shared__ __align__(16) double top_sm[];
+    const int p = top[blockIdx.x];
+    const int n = (int)(6 * (pstart[p + 1] - pstart[p]));
+    if (n == 0) return;
+    double *A = A_all + off[blockIdx.x], *X = X_all + off[blockIdx.x];
+    top_factor(n, A, X, top_sm, status, p);
+    top_inverse(n, A, X, top_sm);
+}
+
+// Kinv = X' X over A, a block a 32 x 32 tile on and below the diagonal, written to both
+// sides (the products' order is the same): entry (i, j) adds X[k][i] X[k][j] over k from
+// max(i, j) on (the tile's own first rows hold the zeros above X's diagonal).
+__global__ void __launch_bounds__(256) k_top_gram(const int32_t* __restrict__ top, const int64_t* __restrict__ pstart,
+                                                  const int64_t* __restrict__ off, double* __restrict__ A_all,
+                                                  const double* __restrict__ X_all) {
+    __shared__ double xi[32][33], xj[32][33];
+    const int p = top[blockIdx.y];
+    const int n = (int)(6 * (pstart[p + 1] - pstart[p]));
+    int ti = 0, rest = blockIdx.x;
+    while (rest > ti) rest -= ++ti;  // tile (ti, rest) of the lower triangle, row by row
+    const int i0 = 32 * ti, j0 = 32 * rest;
+    if (i0 >= n) return;
+    double* A = A_all + off[blockIdx.y];
+    const double* X = X_all + off[blockIdx.y];
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    double t[4] = {0.0, 0.0, 0.0, 0.0};  // rows i0 + w + 8 q, column j0 + l
+    for (int k0 = i0; k0 < n; k0 += 32) {
+        __syncthreads();
+        for (int k = w; k < 32; k += 8) {
+            const bool in = k0 + k < n;
+            xi[k][l] = in && i0 + l < n ? X[(int64_t)(k0 + k) * n + i0 + l] : 0.0;
+            xj[k][l] = in && j0 + l < n ? X[(int64_t)(k0 + k) * n + j0 + l] : 0.0;
+        }
+        __syncthreads();
+        const int m = min(32, n - k0);
+        for (int k = 0; k < m; k++) {
+            const double b = xj[k][l];
+#pragma unroll
+            for (int q = 0; q < 4; q++) t[q] = fma(xi[k][w + 8 * q], b, t[q]);
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const int i = i0 + w + 8 * q, j = j0 + l;
+        if (i < n && j < n && j <= i) {
+            A[(int64_t)i * n + j] = t[q];
+            A[(int64_t)j * n + i] = t[q];
+        }
+    }
 }
 
 // each piece's value of a per-part flag at its first part (0 where it has no part)
@@ -1554,9 +1782,31 @@ static void build_top(Context& ctx, Batch& b, int l, const std::vector<int32_t>&
                                                                     L.kinv_off.get() + first, L.kinv.get());
         SC_LAUNCH_CK();
     }
-    k_cholesky_inverse_all<<<nt, 1024, 0, st>>>(L.top.get(), L.pstart_d.get(), L.kinv_off.get(), L.kinv.get(),
-                                                 X.get(), b.status_d.get());
+    int64_t most = 0;
+    for (int p : pieces) most = std::max<int64_t>(most, 6 * (L.pstart[p + 1] - L.pstart[p]));
+    if (most > TOP_MOST) {
+        k_cholesky_inverse_all<<<nt, 1024, 0, st>>>(L.top.get(), L.pstart_d.get(), L.kinv_off.get(), L.kinv.get(),
+                                                     X.get(), b.status_d.get());
+        SC_LAUNCH_CK();
+        return;
+    }
+    static const bool attr_set = [] {  // once (thread-safe)
+        SC_CK(cudaFuncSetAttribute(k_top_factor, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)top_smem(TOP_MOST)));
+        return true;
+    }();
+    (void)attr_set;
+    const size_t smem = std::max(top_smem(most), (size_t)32 * 34 * sizeof(double));
+    k_top_factor<<<nt, TOP_THREADS, smem, st>>>(L.top.get(), L.pstart_d.get(), L.kinv_off.get(), L.kinv.get(), X.get(),
+                                                b.status_d.get());
     SC_LAUNCH_CK();
+    const unsigned nt32 = (unsigned)((most + 31) / 32);
+    for (unsigned first = 0; first < nt; first += 65535u) {
+        const unsigned m = std::min(nt - first, 65535u);
+        k_top_gram<<<dim3(nt32 * (nt32 + 1) / 2, m), 256, 0, st>>>(L.top.get() + first, L.pstart_d.get(),
+                                                                   L.kinv_off.get() + first, L.kinv.get(), X.get());
+        SC_LAUNCH_CK();
+    }
 }
 
 template <class T>

@@ -243,8 +243,6 @@ struct SolveStats {
 void pcg_fp64(Context& ctx, Batch& b, const sc_options& opt, DBuf<double>& x, SolveStats& st);
 void pcg_mixed(Context& ctx, Batch& b, const sc_options& opt, DBuf<double>& x, SolveStats& st);
 void pcg_fp32_cycle(Context& ctx, Batch& b, const sc_options& opt, DBuf<double>& x, SolveStats& st);
-template <class T>
-void level_apply(Context& ctx, const Batch& b, int l, const T* x, T* y);
 void seg_dot(Context& ctx, const Level& L, const double* a, const double* bb, double* out_per_piece);
 
 // Per-family kernel timing with CUDA events on the context's stream.

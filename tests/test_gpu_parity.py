@@ -420,3 +420,28 @@ def test_residual_replacement_and_fp64_floor(solver, precision):
         loads, _ = z_loads(lat)
         u_ref, _ = lat.motions(loads, tol=1e-12, max_iter=20000)
         assert rel(u, u_ref) < DISP_TOL
+
+
+@pytest.mark.parametrize("shape,few", [((1, 1, 2), 64), ((3, 2, 4), 64), ((5, 5, 4), 90), ((5, 5, 5), 133),
+                                       ((6, 5, 5), 150)],
+                         ids=["few rows", "one panel", "two columns a thread", "largest in shared memory", "beyond"])
+def test_dense_tops_of_all_sizes(solver, shape, few):
+    """Pieces solved by their dense top alone (few above their parts): the factor's panels of
+    32 columns and their remainders, more than 512 rows, and more than fit shared memory,
+    against the oracle's Cholesky solve of the same level."""
+    st = np.ones(shape, np.uint8)
+    st[:, :, 0] = 2
+    k = np.random.default_rng(few).uniform(0.5, 2.0, shape).astype(np.float32)
+    _, parts = sc.grid_count(st)
+    while parts > few:  # trim corners until the piece fits
+        x, y, z = np.argwhere(st == 1)[-1]
+        st[x, y, z] = 0
+        _, parts = sc.grid_count(st)
+    lat = oracle_lattice(st, k)
+    loads, _ = z_loads(lat)
+    u_ref, ir = lat.motions(loads, tol=1e-10, few=few, hierarchy=True)
+    u, info = solver.solve_grid(st, k, sc.options(max_iter=50, tol=1e-10, few=few))
+    assert info["parts"] == ir["counts"] == [parts]
+    assert info["status"] == sc.OK
+    # one exact preconditioner: the motions agree to the top's rounding, kappa(K) eps < 1e-9
+    assert rel(u, u_ref) < 1e-9
