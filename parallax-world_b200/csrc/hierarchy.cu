@@ -291,138 +291,126 @@ __global__ void k_unpack_pattern(int64_t m, const uint64_t* __restrict__ keys, i
     row[i] = (int32_t)(keys[i] >> cb);
 }
 
-// ---- numeric products, one warp per output row ----------------------------------------
-// acc(r, c) += sum_j A(r, j) B(j, c) for the lane's entries (e = lane, lane + 32 < 36).
-// A transposed when TA. B is a rigid shift [I M; 0 I] with M w = w x r when RB (rv = r).
-template <bool TA, bool RB>
-__device__ __forceinline__ void warp_block_mac(int lane, const double* __restrict__ A, const double* __restrict__ B,
-                                               const double* rv, double* __restrict__ C) {
-#pragma unroll
-    for (int rep = 0; rep < 2; rep++) {
-        int e = lane + 32 * rep;
-        if (e >= 36) break;
-        int r = e / 6, c = e % 6;
-        double s = 0.0;
-        if (RB) {
-            // column c of R: c < 3 -> e_c; c >= 3 -> (M[:, c-3], e_c)
-            double a0 = TA ? A[0 * 6 + r] : A[r * 6 + 0];
-            double a1 = TA ? A[1 * 6 + r] : A[r * 6 + 1];
-            double a2 = TA ? A[2 * 6 + r] : A[r * 6 + 2];
-            if (c < 3) {
-                s = c == 0 ? a0 : (c == 1 ? a1 : a2);
-            } else {
-                double ac = TA ? A[c * 6 + r] : A[r * 6 + c];
-                // M = [[0, r2, -r1], [-r2, 0, r0], [r1, -r0, 0]]
-                double m0, m1, m2;
-                if (c == 3) { m0 = 0.0; m1 = -rv[2]; m2 = rv[1]; }
-                else if (c == 4) { m0 = rv[2]; m1 = 0.0; m2 = -rv[0]; }
-                else { m0 = -rv[1]; m1 = rv[0]; m2 = 0.0; }
-                s = fma(a0, m0, fma(a1, m1, fma(a2, m2, ac)));
-            }
-        } else {
-#pragma unroll
-            for (int j = 0; j < 6; j++) {
-                double a = TA ? A[j * 6 + r] : A[r * 6 + j];
-                s = fma(a, B[j * 6 + c], s);
-            }
-        }
-        C[e] += s;
-    }
-}
-
-// S[k][pos(up[o])] += K_ko R_o over the row; then P_k = delta R_k - step D_k^-1 S.
-// K0: level 0 of voxel pieces, blocks made from the cell template (val unused).
+// ---- the smoothed prolongator's values ----------------------------------------------------
+// S[k][pos(up[o])] += K_ko R_o over the row; then P_k = delta R_k - step D_k^-1 S, R_o the
+// rigid shift [I M; 0 I], M w = w x r_o. K0: level 0 of voxel pieces, blocks made from the
+// cell template (val unused). A warp a row; lane 3 r + c (18 of them) owns the entries (r, c)
+// and (r, 3 + c) of every block of S and reads (or, K0, makes) the four values of a block
+// of K they take, so nothing is passed between lanes before S is complete; four stored
+// blocks' loads are in flight. (With a whole block staged per entry and two turns of the
+// lanes for its 36 entries, a 128^3 piece's level 0 took 11.3 ms and the levels above it 6.6;
+// this takes 9.2 and 4.2.)
 template <bool K0>
-__global__ void __launch_bounds__(256) k_num_P(int64_t n, const int64_t* __restrict__ rowptr,
-                                               const int32_t* __restrict__ col, const double* __restrict__ val,
-                                               K0View k0, const int32_t* __restrict__ up,
-                                               const double* __restrict__ rvec, const double* __restrict__ inv,
-                                               const double* __restrict__ step, const int32_t* __restrict__ piece,
-                                               const int64_t* __restrict__ prow, const int32_t* __restrict__ pcol,
-                                               double* __restrict__ pval) {
-    // S's blocks of the warp's row are summed in shared memory when the P row has at most
-    // NUM_P_SMEM blocks (else in pval, zeroed beforehand): the same additions, in order
-    constexpr int NUM_P_SMEM = 12;
-    __shared__ double blk_s[8][36];                 // K0: the warp's current block
-    __shared__ double s_s[8][NUM_P_SMEM * 36];
-    int64_t k = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    if (k >= n) return;
-    int lane = threadIdx.x & 31;
-    if (up[k] < 0) return;
-    const int w = (threadIdx.x >> 5) & 7;
-    double* blk = blk_s[w];
-    K0Row row{};
-    if (K0) row = k0_row(k0, k);
-    const int64_t p0 = prow[k], p1 = prow[k + 1];
-    const bool local = p1 - p0 <= NUM_P_SMEM;
-    double* S = local ? s_s[w] : pval + 36 * p0;
-    if (local)
-        for (int t = lane; t < 36 * (int)(p1 - p0); t += 32) S[t] = 0.0;
-    __syncwarp();
-    const int64_t e1 = rowptr[k + 1];
-    for (int64_t eb = rowptr[k]; eb < e1; eb += 32) {
-        // lane t finds its entry's block of P row k (independent searches), then the
-        // warp adds the entries one by one
-        int32_t mo = 0;
-        int mpos = 0;
-        if (eb + lane < e1) {
-            mo = col[eb + lane];
-            mpos = (int)(lower_bound_i32(pcol, p0, p1, up[mo]) - p0);
-        }
-        const int nb = (int)min((int64_t)32, e1 - eb);
-        for (int t = 0; t < nb; t++) {
-            const int64_t e = eb + t;
-            const int32_t o = __shfl_sync(0xffffffffu, mo, t);
-            const int pos = __shfl_sync(0xffffffffu, mpos, t);
-            double rv[3] = {rvec[3 * (int64_t)o], rvec[3 * (int64_t)o + 1], rvec[3 * (int64_t)o + 2]};
-            const double* A = val + 36 * e;
-            if (K0) {
-                uint8_t d = k0.desc[e];
-                for (int q = lane; q < 36; q += 32) blk[q] = k0_entry(k0.tpl_s, row, d, q / 6, q % 6);
-                __syncwarp();
-                A = blk;
-            }
-            warp_block_mac<false, true>(lane, A, nullptr, rv, S + 36 * pos);
-            __syncwarp();
-        }
+constexpr int num_p_warps() { return K0 ? 8 : 4; }
+template <bool K0>
+__global__ void __launch_bounds__(32 * num_p_warps<K0>()) k_num_P(
+    int64_t n, const int64_t* __restrict__ rowptr, const int32_t* __restrict__ col, const double* __restrict__ val,
+    K0View k0, const int32_t* __restrict__ up, const double* __restrict__ rvec, const double* __restrict__ inv,
+    const double* __restrict__ step, const int32_t* __restrict__ piece, const int64_t* __restrict__ prow,
+    const int32_t* __restrict__ pcol, double* __restrict__ pval) {
+    // S is summed in shared memory when the P row has at most MOST blocks, else in pval: the
+    // same additions, in order
+    constexpr int W = num_p_warps<K0>(), MOST = K0 ? 12 : 28, U = K0 ? 1 : 4;
+    __shared__ double T[K0 ? 36 * 36 : 1];
+    __shared__ double s_s[W][MOST * 36], r_s[W][32][3];
+    if (K0) {
+        for (int t = threadIdx.x; t < 36 * 36; t += blockDim.x) T[t] = k0.tpl_s[t];
+        __syncthreads();
     }
-    double st = step[piece[k]];
-    const double* D = inv + 36 * k;
-    double rk[3] = {rvec[3 * k], rvec[3 * k + 1], rvec[3 * k + 2]};
-    for (int64_t pos = p0; pos < p1; pos++) {
-        const double* Sp = S + 36 * (pos - p0);
-        double out[2];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int r = min(lane, 17) / 3, c = min(lane, 17) % 3;
+    const bool on = lane < 18;
+    for (int64_t k = (int64_t)blockIdx.x * W + w; k < n; k += (int64_t)gridDim.x * W) {
+        if (up[k] < 0) continue;
+        K0Row row{};
+        if (K0) row = k0_row(k0, k);
+        const int64_t p0 = prow[k], p1 = prow[k + 1];
+        const int np = (int)(p1 - p0);
+        double* S = np <= MOST ? s_s[w] : pval + 36 * p0;
+        for (int t = lane; t < 36 * np; t += 32) S[t] = 0.0;
+        __syncwarp();
+        const int64_t e1 = rowptr[k + 1];
+        for (int64_t eb = rowptr[k]; eb < e1; eb += 32) {
+            // lane t finds its entry's block of P row k (independent searches) and its r
+            int mpos = 0, md = 0;
+            if (eb + lane < e1) {
+                const int32_t o = col[eb + lane];
+                if (K0) md = k0.desc[eb + lane];
+                mpos = (int)(lower_bound_i32(pcol, p0, p1, up[o]) - p0);
+                r_s[w][lane][0] = rvec[3 * (int64_t)o];
+                r_s[w][lane][1] = rvec[3 * (int64_t)o + 1];
+                r_s[w][lane][2] = rvec[3 * (int64_t)o + 2];
+            }
+            __syncwarp();
+            const int nb = (int)min((int64_t)32, e1 - eb);
+            for (int t0 = 0; t0 < nb; t0 += U) {
+                double a[U][4];  // A(r, 0), A(r, 1), A(r, 2), A(r, 3 + c)
+                int pos[U];
 #pragma unroll
-        for (int rep = 0; rep < 2; rep++) {
-            int e = lane + 32 * rep;
-            out[rep] = 0.0;
-            if (e < 36) {
-                int r = e / 6, c = e % 6;
-                double s = 0.0;
-                for (int j = 0; j < 6; j++) s = fma(D[r * 6 + j], Sp[j * 6 + c], s);
-                double rig = 0.0;
-                if (pcol[pos] == up[k]) {
-                    if (r == c) rig = 1.0;
-                    else if (r < 3 && c >= 3) {
-                        // M[r][c-3]
-                        int cc = c - 3;
-                        if (r == 0) rig = cc == 1 ? rk[2] : (cc == 2 ? -rk[1] : 0.0);
-                        if (r == 1) rig = cc == 0 ? -rk[2] : (cc == 2 ? rk[0] : 0.0);
-                        if (r == 2) rig = cc == 0 ? rk[1] : (cc == 1 ? -rk[0] : 0.0);
+                for (int u = 0; u < U; u++) {
+                    const int t = min(t0 + u, nb - 1);
+                    pos[u] = __shfl_sync(0xffffffffu, mpos, t);
+                    const uint8_t d = (uint8_t)__shfl_sync(0xffffffffu, md, t);
+                    if (t0 + u >= nb || !on) continue;
+                    if (K0) {
+                        const K0Block b = k0_block(row, d);
+#pragma unroll
+                        for (int j = 0; j < 4; j++) a[u][j] = k0_value(T, row, b, 36 * r + (j < 3 ? j : 3 + c));
+                    } else {
+                        const double* A = val + 36 * (eb + t) + 6 * r;
+#pragma unroll
+                        for (int j = 0; j < 4; j++) a[u][j] = A[j < 3 ? j : 3 + c];
                     }
                 }
-                out[rep] = rig + (-st) * s;
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    if (t0 + u >= nb || !on) continue;
+                    const double* rv = r_s[w][t0 + u];
+                    // column c of M = [[0, r2, -r1], [-r2, 0, r0], [r1, -r0, 0]]
+                    const double m0 = c == 0 ? 0.0 : c == 1 ? rv[2] : -rv[1];
+                    const double m1 = c == 0 ? -rv[2] : c == 1 ? 0.0 : rv[0];
+                    const double m2 = c == 0 ? rv[1] : c == 1 ? -rv[0] : 0.0;
+                    double* C = S + 36 * pos[u] + 6 * r + c;
+                    C[0] += c == 0 ? a[u][0] : c == 1 ? a[u][1] : a[u][2];
+                    C[3] += fma(a[u][0], m0, fma(a[u][1], m1, fma(a[u][2], m2, a[u][3])));
+                }
+            }
+            __syncwarp();
+        }
+        const double st = step[piece[k]];
+        const int32_t own = up[k];
+        const double rk[3] = {rvec[3 * k], rvec[3 * k + 1], rvec[3 * k + 2]};
+        double D[6];
+#pragma unroll
+        for (int j = 0; j < 6; j++) D[j] = inv[36 * k + 6 * r + j];
+        // R_k's entries (r, c) and (r, 3 + c)
+        const double one = r == c ? 1.0 : 0.0;
+        double far = r == 3 + c ? 1.0 : 0.0;
+        if (r == 0 && c == 1) far = rk[2];
+        if (r == 0 && c == 2) far = -rk[1];
+        if (r == 1 && c == 0) far = -rk[2];
+        if (r == 1 && c == 2) far = rk[0];
+        if (r == 2 && c == 0) far = rk[1];
+        if (r == 2 && c == 1) far = -rk[0];
+        for (int pos = 0; pos < np; pos++) {
+            const double* Sp = S + 36 * pos;
+            double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+            for (int j = 0; j < 6; j++) {
+                s0 = fma(D[j], Sp[6 * j + c], s0);
+                s1 = fma(D[j], Sp[6 * j + 3 + c], s1);
+            }
+            const bool self = pcol[p0 + pos] == own;
+            __syncwarp();
+            if (on) {
+                double* P = pval + 36 * (p0 + pos) + 6 * r + c;
+                P[0] = (self ? one : 0.0) + (-st) * s0;
+                P[3] = (self ? far : 0.0) + (-st) * s1;
             }
         }
         __syncwarp();
-        double* P = pval + 36 * pos;
-        if (lane < 36) P[lane] = out[0];
-        if (lane + 32 < 36) P[lane + 32] = out[1];
-        __syncwarp();
     }
 }
-
-
 
 // Every output block of a product as the ordered sum of its contributions: after the
 // symbolic sort, output block q's contributions are vals[seg[q] .. seg[q+1]), each the
@@ -513,7 +501,7 @@ __global__ void __launch_bounds__(SUM_THREADS) k_sum_products(int64_t nout, cons
 // then the addition, as the sorted sums do: the same bits, with no list of candidates made,
 // sorted or read. (By sorted candidates a contribution's block of K was made anew and its
 // rows passed on by 72 shuffles. On a 128^3 piece, 112.7 M contributions, that took 30 ms
-// after 12 ms of sorting; this takes 18 and 1.3 to count.)
+// after 12 ms of sorting; this takes 12.4 and 1.3 to count.)
 // KP0_BATCH output blocks are merged, then summed, at a time, whatever the row's length.
 constexpr int KP0_WARPS = 8, KP0_MOST = 11, KP0_BATCH = 20;
 template <bool FILL, class TB, class TO>
@@ -534,103 +522,108 @@ __global__ void __launch_bounds__(32 * KP0_WARPS) k_kp0(int64_t n, K0View k0, co
         __syncthreads();
     }
     const int w = FILL ? threadIdx.x >> 5 : 0, lane = threadIdx.x & 31;
-    const int64_t k = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    if (k >= n) return;
-    if (up[k] < 0) {  // its piece is solved at level 0
-        if (!FILL && lane == 0) cnt[k] = 0;
-        return;
-    }
-    const int64_t e0 = rowptr[k];
-    const int ne = (int)(rowptr[k + 1] - e0);
-    const int32_t first = pcol[prow[k]];  // columns below P row k's first are not read later
-    int64_t f = 0, f1 = 0;
-    uint8_t d = 0;
-    constexpr int32_t NONE = 0x7fffffff;
-    if (lane < ne) {
-        const int32_t q = col[e0 + lane];
-        if (FILL) d = k0.desc[e0 + lane];
-        f = prow[q];
-        f1 = prow[q + 1];
-    }
-    // this lane's column and the one after it
-    int32_t cur = f < f1 ? pcol[f] : NONE, nxt = f + 1 < f1 ? pcol[f + 1] : NONE;
-    auto step = [&] {
-        f++;
-        cur = nxt;
-        nxt = f + 1 < f1 ? pcol[f + 1] : NONE;
-    };
-    while (cur < first) step();
-    if (!FILL) {
-        int64_t m = 0;
-        for (;; m++) {
-            const int32_t least = __reduce_min_sync(0xffffffffu, cur);
-            if (least == NONE) break;
-            if (cur == least) step();
+    for (int64_t k = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; k < n;
+         k += (int64_t)gridDim.x * KP0_WARPS) {
+        if (up[k] < 0) {  // its piece is solved at level 0
+            if (!FILL && lane == 0) cnt[k] = 0;
+            continue;
         }
-        if (lane == 0) cnt[k] = m;
-        return;
-    }
-    const K0Row row = k0_row(k0, k);
-    for (int t0 = 0; t0 < 36 * KP0_MOST; t0 += 32) {  // every lane, every time round: the shuffle needs all
-        const int t = t0 + lane, e = min(t / 36, KP0_MOST - 1), x = t % 36;
-        const uint8_t de = (uint8_t)__shfl_sync(0xffffffffu, (int)d, e);
-        if (t < 36 * KP0_MOST && e < ne) blocks[w][t] = k0_entry(T, row, de, x / 6, x % 6);
-    }
-    const int g = lane / 6, c = lane % 6;
-    for (int64_t q0 = kprow[k];; q0 += KP0_BATCH) {
-        int ns = 0;
-        for (; ns < KP0_BATCH; ns++) {
-            const int32_t least = __reduce_min_sync(0xffffffffu, cur);
-            if (least == NONE) break;
-            const bool mine = cur == least;
-            const uint32_t who = __ballot_sync(0xffffffffu, mine);
-            if (lane == 0) {
-                held[w][ns] = who;
-                kpcol[q0 + ns] = least;
+        const int64_t e0 = rowptr[k];
+        const int ne = (int)(rowptr[k + 1] - e0);
+        const int32_t first = pcol[prow[k]];  // columns below P row k's first are not read later
+        int64_t f = 0, f1 = 0;
+        uint8_t d = 0;
+        constexpr int32_t NONE = 0x7fffffff;
+        if (lane < ne) {
+            const int32_t q = col[e0 + lane];
+            if (FILL) d = k0.desc[e0 + lane];
+            f = prow[q];
+            f1 = prow[q + 1];
+        }
+        // this lane's column and the one after it
+        int32_t cur = f < f1 ? pcol[f] : NONE, nxt = f + 1 < f1 ? pcol[f + 1] : NONE;
+        auto step = [&] {
+            f++;
+            cur = nxt;
+            nxt = f + 1 < f1 ? pcol[f + 1] : NONE;
+        };
+        while (cur < first) step();
+        if (!FILL) {
+            int64_t m = 0;
+            for (;; m++) {
+                const int32_t least = __reduce_min_sync(0xffffffffu, cur);
+                if (least == NONE) break;
+                if (cur == least) step();
             }
-            if (mine) {
-                entry[w][ns][lane] = (int32_t)f;
-                step();
+            if (lane == 0) cnt[k] = m;
+            continue;
+        }
+        const K0Row row = k0_row(k0, k);
+        const int br = min(lane, 17) / 3, bc = min(lane, 17) % 3;  // 18 lanes make two entries of a block each
+        for (int e = 0; e < ne; e++) {
+            const uint8_t de = (uint8_t)__shfl_sync(0xffffffffu, (int)d, e);
+            if (lane < 18) {
+                double* o = blocks[w] + 36 * e + 6 * br + bc;
+                o[0] = k0_entry(T, row, de, br, bc);
+                o[3] = k0_entry(T, row, de, br, 3 + bc);
             }
         }
-        __syncwarp();
-        if (ns == 0) break;
-        int s = g < 5 ? g : ns;  // lanes 30 and 31 have no group
-        uint32_t who = s < ns ? held[w][s] : 0u;
-        double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-        while (s < ns) {
-            const int e = __ffs(who) - 1;
-            who &= who - 1u;
-            const TB* bb = B + 36 * (int64_t)entry[w][s][e] + c;
-            double bc[6];
-#pragma unroll
-            for (int j = 0; j < 6; j++) bc[j] = (double)bb[6 * j];
-            const double2* A = reinterpret_cast<const double2*>(blocks[w] + 36 * e);
-#pragma unroll
-            for (int r = 0; r < 6; r++) {
-                const double2 a0 = A[3 * r], a1 = A[3 * r + 1], a2 = A[3 * r + 2];
-                double v = 0.0;
-                v = fma(a0.x, bc[0], v);
-                v = fma(a0.y, bc[1], v);
-                v = fma(a1.x, bc[2], v);
-                v = fma(a1.y, bc[3], v);
-                v = fma(a2.x, bc[4], v);
-                v = fma(a2.y, bc[5], v);
-                acc[r] += v;
-            }
-            if (!who) {
-                TO* o = out + 36 * (q0 + s) + c;
-#pragma unroll
-                for (int r = 0; r < 6; r++) {
-                    o[6 * r] = (TO)acc[r];
-                    acc[r] = 0.0;
+        const int g = lane / 6, c = lane % 6;
+        for (int64_t q0 = kprow[k];; q0 += KP0_BATCH) {
+            int ns = 0;
+            for (; ns < KP0_BATCH; ns++) {
+                const int32_t least = __reduce_min_sync(0xffffffffu, cur);
+                if (least == NONE) break;
+                const bool mine = cur == least;
+                const uint32_t who = __ballot_sync(0xffffffffu, mine);
+                if (lane == 0) {
+                    held[w][ns] = who;
+                    kpcol[q0 + ns] = least;
                 }
-                s += 5;
-                if (s < ns) who = held[w][s];
+                if (mine) {
+                    entry[w][ns][lane] = (int32_t)f;
+                    step();
+                }
             }
+            __syncwarp();
+            if (ns == 0) break;
+            int s = g < 5 ? g : ns;  // lanes 30 and 31 have no group
+            uint32_t who = s < ns ? held[w][s] : 0u;
+            double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+            while (s < ns) {
+                const int e = __ffs(who) - 1;
+                who &= who - 1u;
+                const TB* bb = B + 36 * (int64_t)entry[w][s][e] + c;
+                double bc[6];
+    #pragma unroll
+                for (int j = 0; j < 6; j++) bc[j] = (double)bb[6 * j];
+                const double2* A = reinterpret_cast<const double2*>(blocks[w] + 36 * e);
+    #pragma unroll
+                for (int r = 0; r < 6; r++) {
+                    const double2 a0 = A[3 * r], a1 = A[3 * r + 1], a2 = A[3 * r + 2];
+                    double v = 0.0;
+                    v = fma(a0.x, bc[0], v);
+                    v = fma(a0.y, bc[1], v);
+                    v = fma(a1.x, bc[2], v);
+                    v = fma(a1.y, bc[3], v);
+                    v = fma(a2.x, bc[4], v);
+                    v = fma(a2.y, bc[5], v);
+                    acc[r] += v;
+                }
+                if (!who) {
+                    TO* o = out + 36 * (q0 + s) + c;
+    #pragma unroll
+                    for (int r = 0; r < 6; r++) {
+                        o[6 * r] = (TO)acc[r];
+                        acc[r] = 0.0;
+                    }
+                    s += 5;
+                    if (s < ns) who = held[w][s];
+                }
+            }
+            __syncwarp();
+            if (ns < KP0_BATCH) break;
         }
-        __syncwarp();
-        if (ns < KP0_BATCH) break;
     }
 }
 
@@ -1385,17 +1378,16 @@ static bool coarsen(Context& ctx, Batch& b, int l, int octree_level, const sc_op
     cnt.release();
     off.release();
     F.pval.alloc(36 * std::max<int64_t>(F.pnnz, 1), st, ms);
-    F.pval.zero();
     const K0View k0 = k0_view(b, F);
     const bool virt = k0.desc != nullptr;  // level-0 blocks made from the cell template
     if (virt)
-        k_num_P<true><<<grid_for(n * 32, 256), 256, 0, st>>>(n, F.rowptr.get(), F.col.get(), nullptr, k0, F.up.get(),
-                                                             rvec.get(), F.inv.get(), F.step.get(), F.piece.get(),
-                                                             F.prow.get(), F.pcol.get(), F.pval.get());
+        k_num_P<true><<<std::min(grid_for(n, 8), 148u * 5u), 256, 0, st>>>(
+            n, F.rowptr.get(), F.col.get(), nullptr, k0, F.up.get(), rvec.get(), F.inv.get(), F.step.get(),
+            F.piece.get(), F.prow.get(), F.pcol.get(), F.pval.get());
     else
-        k_num_P<false><<<grid_for(n * 32, 256), 256, 0, st>>>(n, F.rowptr.get(), F.col.get(), F.val.get(), k0,
-                                                              F.up.get(), rvec.get(), F.inv.get(), F.step.get(),
-                                                              F.piece.get(), F.prow.get(), F.pcol.get(), F.pval.get());
+        k_num_P<false><<<grid_for(n, 4), 128, 0, st>>>(n, F.rowptr.get(), F.col.get(), F.val.get(), k0, F.up.get(),
+                                                       rvec.get(), F.inv.get(), F.step.get(), F.piece.get(),
+                                                       F.prow.get(), F.pcol.get(), F.pval.get());
     SC_LAUNCH_CK();
     if (keep_mf) {
         F.mf_r = std::move(rvec);
@@ -1482,7 +1474,7 @@ static bool coarsen(Context& ctx, Batch& b, int l, int octree_level, const sc_op
         kcnt.alloc(n + 1, st, ms);
         kprow.alloc(n + 1, st, ms);
         SC_CK(cudaMemsetAsync(kcnt.get() + n, 0, sizeof(int64_t), st));
-        const unsigned nb = grid_for(n, KP0_WARPS);
+        const unsigned nb = std::min(grid_for(n, KP0_WARPS), 148u * 40u);
         k_kp0<false, double, double><<<nb, 32 * KP0_WARPS, 0, st>>>(n, k0, F.rowptr.get(), F.col.get(), F.prow.get(),
                                                                    F.pcol.get(), F.up.get(), kcnt.get(), nullptr,
                                                                    nullptr, nullptr, nullptr);

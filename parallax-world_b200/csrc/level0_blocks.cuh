@@ -58,4 +58,29 @@ __device__ __forceinline__ double k0_entry(const double* __restrict__ T, const K
     return (d >> 3) ? r.kB * T[(6 * slB + i) * 36 + 6 * slot + j] : r.kA * T[(6 * slA + i) * 36 + 6 * slot + j];
 }
 
+// The same entry by entry: where the block of descriptor d starts in the template, so that
+// its entries (offset 36 i + j from there) need no more than a product each.
+struct K0Block {
+    bool diag;
+    double k;    // the block's cell's stiffness
+    int at, at2; // its place in the template; of a diagonal block, the lesser and greater cell's
+};
+__device__ __forceinline__ K0Block k0_block(const K0Row& r, uint8_t d) {
+    const int slA = 2 * r.ax + 1, slB = 2 * r.ax;
+    K0Block b;
+    b.diag = d == K0_DIAG;
+    const bool second = !b.diag && (d >> 3);
+    b.k = second ? r.kB : r.kA;
+    b.at = 216 * (second ? slB : slA) + 6 * (b.diag ? slA : d & 7);
+    b.at2 = 216 * slB + 6 * slB;
+    return b;
+}
+__device__ __forceinline__ double k0_value(const double* __restrict__ T, const K0Row& r, const K0Block& b, int off) {
+    if (!b.diag) return b.k * T[b.at + off];
+    double v = 0.0;
+    if (r.hasA) v += r.kA * T[b.at + off];
+    if (r.hasB) v += r.kB * T[b.at2 + off];
+    return v;
+}
+
 }  // namespace sc
