@@ -81,17 +81,101 @@ __global__ void __launch_bounds__(256) k_spmv(int64_t nrows, const int64_t* __re
     }
 }
 
+// A row's blocks by asynchronous copies: the sum of this lane's products over its slot's
+// blocks first + g, + stride, ... below e1 (lane = 8 g + r: slot g of 4, block row r, lanes
+// with r >= 6 idle), a warp's groups of four consecutive blocks `stride` apart.
+//
+// On levels of few, long rows the product is bound by its chain row bounds -> columns -> x
+// and by how many blocks a warp has in flight, eight with loads to registers. cp.async
+// brings blocks and x to the warp's own ring of shared memory instead, 32 blocks ahead, 16
+// bytes a lane, and the lanes add from there, in the same order: FP64 rows over four warps
+// (a 32^3 piece's levels 2 and 3) 10.5-12.9 us to 7.2-9.6, over two (a 128^3 piece's level 3)
+// 124-131 to 112-115. Where rows are many it only costs occupancy (a warp a row took 216 us for
+// 161 in FP32, 396 for 308 in FP64), and in FP32, whose blocks are half the bytes, it gains
+// nothing over two or four warps (74 us for 66, and a whole 61 x 45 x 37 solve 1 % slower):
+// those keep the loads to registers (as deep a pipeline in registers was slower still).
+constexpr int RING = 4, RING_BLOCKS = 8;  // stages of eight blocks: two of each slot
+template <class T>
+struct Ring {
+    T val[RING][RING_BLOCKS * 36];
+    T x[RING][RING_BLOCKS * 6];
+};
+__device__ __forceinline__ void cp16(void* s, const void* g) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(s)), "l"(g)
+                 : "memory");
+}
+template <class T>
+__device__ __forceinline__ T row_stream(Ring<T>& ring, int64_t first, int64_t e1, int stride,
+                                        const int32_t* __restrict__ col, const T* __restrict__ val,
+                                        const T* __restrict__ x) {
+    constexpr int PIECES = 36 * (int)sizeof(T) / 16;  // 16-byte pieces of a block
+    const int lane = threadIdx.x & 31, g = lane >> 3, rr = lane & 7;
+    T acc = T(0);
+    // the columns of a turn of the ring: lane l's block is the l-th of the warp's
+    auto block = [&](int64_t base, int l) { return base + (int64_t)stride * (l >> 2) + (l & 3); };
+    int32_t cols = block(first, lane) < e1 ? col[block(first, lane)] : 0;
+    auto issue = [&](int64_t base, int s) {  // stage s of the turn that starts at base
+        const int64_t b0 = base + 2 * (int64_t)stride * s;
+        for (int q = lane; q < RING_BLOCKS * PIECES; q += 32) {
+            const int64_t e = block(b0, q / PIECES);
+            if (e < e1)
+                cp16(reinterpret_cast<char*>(ring.val[s]) + 16 * q,
+                     reinterpret_cast<const char*>(val + 36 * e) + 16 * (q % PIECES));
+        }
+        const int32_t j = __shfl_sync(0xffffffffu, cols, 8 * s + min(lane / 3, 7));
+        if (lane < 24 && block(b0, lane / 3) < e1) {
+            cp16(ring.x[s] + 2 * lane, x + 6 * (int64_t)j + 2 * (lane % 3));
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+#pragma unroll
+    for (int s = 0; s < RING; s++) issue(first, s);
+    for (int64_t base = first; base < e1; base += 8 * (int64_t)stride) {
+        const int64_t next = base + 8 * (int64_t)stride;
+        if (next < e1) cols = block(next, lane) < e1 ? col[block(next, lane)] : 0;
+#pragma unroll
+        for (int s = 0; s < RING; s++) {
+            asm volatile("cp.async.wait_group %0;\n" ::"n"(RING - 1) : "memory");
+            __syncwarp();
+            const int64_t b0 = base + 2 * (int64_t)stride * s + g;
+            if (rr < 6) {
+#pragma unroll
+                for (int u = 0; u < 2; u++)
+                    if (b0 + (int64_t)stride * u < e1) {
+                        T a[6], xv[6];
+                        ld6<T>(ring.val[s] + 36 * (4 * u + g) + 6 * rr, a);
+                        ld6<T>(ring.x[s] + 6 * (4 * u + g), xv);
+#pragma unroll
+                        for (int c = 0; c < 6; c++) acc = fma(a[c], xv[c], acc);
+                    }
+            }
+            __syncwarp();
+            if (next < e1)
+                issue(next, s);
+            else
+                asm volatile("cp.async.commit_group;\n" ::: "memory");
+        }
+    }
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    return acc;
+}
+
 // The same with each row split over WPR warps, for levels of few, long rows (coarse
 // levels and their transfers), where one warp a row leaves the device idle. Warp w of a
-// row takes its blocks e0 + 4 w + g, then every 4 WPR, two in flight; the warps' partial
-// sums meet in shared memory and are added in warp order (a fixed order).
+// row takes its blocks e0 + 4 w + g, then every 4 WPR, streamed where that measured faster
+// (above; the rings of more than four warps would not fit), else two in flight; the warps'
+// partial sums meet in shared memory and are added in warp order (a fixed order).
+template <class T, int WPR>
+constexpr bool split_streams() { return sizeof(T) == 8 && (WPR == 2 || WPR == 4); }
+template <class T, int WPR>
+constexpr int split_warps() { return split_streams<T, WPR>() ? 4 : WPR > 8 ? WPR : 8; }
 template <class T, int MODE, int WPR>
-__global__ void __launch_bounds__(32 * (WPR > 8 ? WPR : 8)) k_spmv_split(
+__global__ void __launch_bounds__(32 * split_warps<T, WPR>()) k_spmv_split(
     int64_t nrows, const int64_t* __restrict__ rowptr, const int32_t* __restrict__ col, const T* __restrict__ val,
     const T* __restrict__ x, const T* __restrict__ r, T* __restrict__ y, const T* __restrict__ inv,
     const double* __restrict__ step, const int32_t* __restrict__ piece, const int32_t* __restrict__ skip_row,
     const int32_t* __restrict__ done, T* __restrict__ y2) {
-    constexpr int RPC = WPR >= 8 ? 1 : 8 / WPR;  // rows per thread block
+    constexpr int RPC = split_warps<T, WPR>() / WPR;  // rows per thread block
     constexpr int STRIDE = 4 * WPR;
     __shared__ T part[RPC * WPR][6];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -106,29 +190,34 @@ __global__ void __launch_bounds__(32 * (WPR > 8 ? WPR : 8)) k_spmv_split(
         if (piece) p = piece[row];
         active = !(skip || (done && done[p]));
     }
-    const int g = lane >> 3, rr = lane & 7;
     T acc = T(0);
-    if (active && rr < 6) {
-        int64_t e = e0 + 4 * wr + g;
-        for (; e + STRIDE < e1; e += 2 * STRIDE) {
-            int32_t j0 = col[e], j1 = col[e + STRIDE];
-            T a0[6], x0[6], a1[6], x1[6];
-            ld6<T>(val + 36 * e + 6 * rr, a0);
-            ld6<T>(val + 36 * (e + STRIDE) + 6 * rr, a1);
-            ld6<T>(x + 6 * (int64_t)j0, x0);
-            ld6<T>(x + 6 * (int64_t)j1, x1);
+    if constexpr (split_streams<T, WPR>()) {
+        __shared__ __align__(16) Ring<T> ring[4];
+        if (active) acc = row_stream<T>(ring[warp], e0 + 4 * wr, e1, 4 * WPR, col, val, x);
+    } else {
+        const int g = lane >> 3, rr = lane & 7;
+        if (active && rr < 6) {
+            int64_t e = e0 + 4 * wr + g;
+            for (; e + STRIDE < e1; e += 2 * STRIDE) {
+                int32_t j0 = col[e], j1 = col[e + STRIDE];
+                T a0[6], x0[6], a1[6], x1[6];
+                ld6<T>(val + 36 * e + 6 * rr, a0);
+                ld6<T>(val + 36 * (e + STRIDE) + 6 * rr, a1);
+                ld6<T>(x + 6 * (int64_t)j0, x0);
+                ld6<T>(x + 6 * (int64_t)j1, x1);
 #pragma unroll
-            for (int c = 0; c < 6; c++) acc = fma(a0[c], x0[c], acc);
+                for (int c = 0; c < 6; c++) acc = fma(a0[c], x0[c], acc);
 #pragma unroll
-            for (int c = 0; c < 6; c++) acc = fma(a1[c], x1[c], acc);
-        }
-        if (e < e1) {
-            int32_t j = col[e];
-            T a[6], xv[6];
-            ld6<T>(val + 36 * e + 6 * rr, a);
-            ld6<T>(x + 6 * (int64_t)j, xv);
+                for (int c = 0; c < 6; c++) acc = fma(a1[c], x1[c], acc);
+            }
+            if (e < e1) {
+                int32_t j = col[e];
+                T a[6], xv[6];
+                ld6<T>(val + 36 * e + 6 * rr, a);
+                ld6<T>(x + 6 * (int64_t)j, xv);
 #pragma unroll
-            for (int c = 0; c < 6; c++) acc = fma(a[c], xv[c], acc);
+                for (int c = 0; c < 6; c++) acc = fma(a[c], xv[c], acc);
+            }
         }
     }
     acc += __shfl_xor_sync(0xffffffffu, acc, 8);
@@ -360,8 +449,8 @@ template <class T, int WPR>
 void launch_split(Context& ctx, int mode, int64_t nrows, const int64_t* rowptr, const int32_t* col, const T* val,
                   const T* x, const T* r, T* y, const T* inv, const double* step, const int32_t* piece,
                   const int32_t* skip_row, const int32_t* done, T* y2) {
-    constexpr int RPC = WPR >= 8 ? 1 : 8 / WPR;
-    constexpr int threads = 32 * (WPR > 8 ? WPR : 8);
+    constexpr int RPC = split_warps<T, WPR>() / WPR;
+    constexpr int threads = 32 * split_warps<T, WPR>();
     const unsigned g = grid_for(nrows, RPC);
     auto go = [&](auto kernel) {
         kernel<<<g, threads, 0, ctx.stream>>>(nrows, rowptr, col, val, x, r, y, inv, step, piece, skip_row, done, y2);
