@@ -254,12 +254,14 @@ __global__ void k_cg_check(int np, int64_t max_iter, CgScalars s, int32_t* ndone
 template <bool SPLIT>
 __global__ void __launch_bounds__(RED_LANES) k_dot_alpha(Chunks ch, CgScalars s, const double* __restrict__ p,
                                                          const double* __restrict__ ap) {
+    extern __shared__ double sm[];
     const int c = red_chunk<SPLIT>(), t = red_lane<SPLIT>(), pc = ch.piece[c];
     if (s.done[pc]) return;
     double pap = 0.0, none = 0.0;
-    red_chain<SPLIT ? 16 : 8>(
-        6 * ch.lo[c] + t, 6 * ch.lo[c + 1], [&](int64_t i) { return make_double2(p[i], ap[i]); },
-        [&](int64_t, const double2& v) { pap = fma(v.x, v.y, pap); });
+    if (!red_run<SPLIT, 2, 8>(
+            sm, 6 * ch.lo[c] + t, 6 * ch.lo[c + 1], [&](int64_t i, double (&v)[2]) { v[0] = p[i], v[1] = ap[i]; },
+            [&](const double (&v)[2]) { pap = fma(v[0], v[1], pap); }))
+        return;
     if (!red_finish<SPLIT>(ch, c, t, pc, pap, none)) return;
     s.pap[pc] = pap;
     if (!(pap > 0.0)) {
@@ -277,19 +279,50 @@ template <bool SPLIT>
 __global__ void __launch_bounds__(RED_LANES) k_update_xr(Chunks ch, CgScalars s, double* __restrict__ x,
                                                          const double* __restrict__ p, double* __restrict__ r,
                                                          const double* __restrict__ ap, float* __restrict__ r32) {
+    extern __shared__ double sm[];
     const int c = red_chunk<SPLIT>(), t = red_lane<SPLIT>(), pc = ch.piece[c];
     if (s.done[pc]) return;
     const double a = s.alpha[pc];
+    const int64_t first = 6 * ch.lo[c] + t, end = 6 * ch.lo[c + 1];
     double rr = 0.0, none = 0.0;
-    red_chain<SPLIT ? 12 : 6>(
-        6 * ch.lo[c] + t, 6 * ch.lo[c + 1], [&](int64_t i) { return make_double4(x[i], p[i], r[i], ap[i]); },
-        [&](int64_t i, const double4& v) {
-            x[i] = v.x + a * v.y;
-            const double rn = v.z - a * v.w;
-            r[i] = rn;
-            if (r32) r32[i] = (float)rn;
+    auto update = [&](int64_t i, double xv, double pv, double rv, double av) {
+        x[i] = xv + a * pv;
+        const double rn = rv - a * av;
+        r[i] = rn;
+        if (r32) r32[i] = (float)rn;
+        return rn;
+    };
+    if constexpr (SPLIT) {
+        // eight warps update; the first sums what they leave in shared memory
+        constexpr int PER = RED_STEPS / 8;
+        const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+        double4 v[PER];
+#pragma unroll
+        for (int u = 0; u < PER; u++) {
+            const int64_t i = first + RED_LANES * (int64_t)(w + 8 * u);
+            if (i < end) v[u] = make_double4(x[i], p[i], r[i], ap[i]);
+        }
+#pragma unroll
+        for (int u = 0; u < PER; u++) {
+            const int64_t i = first + RED_LANES * (int64_t)(w + 8 * u);
+            if (i < end) sm[(w + 8 * u) * 32 + l] = update(i, v[u].x, v[u].y, v[u].z, v[u].w);
+        }
+        __syncthreads();
+        if (w != 0) return;
+        const int n = first < end ? (int)((end - first + RED_LANES - 1) / RED_LANES) : 0;
+#pragma unroll 8
+        for (int k = 0; k < n; k++) {
+            const double rn = sm[k * 32 + l];
             rr = fma(rn, rn, rr);
-        });
+        }
+    } else {
+        red_chain<6>(
+            first, end, [&](int64_t i) { return make_double4(x[i], p[i], r[i], ap[i]); },
+            [&](int64_t i, const double4& v) {
+                const double rn = update(i, v.x, v.y, v.z, v.w);
+                rr = fma(rn, rn, rr);
+            });
+    }
     if (red_finish<SPLIT>(ch, c, t, pc, rr, none)) s.rr[pc] = rr;
 }
 
@@ -302,16 +335,21 @@ template <class Z, bool FLEX, bool SPLIT>
 __global__ void __launch_bounds__(RED_LANES) k_dots_beta(Chunks ch, CgScalars s, int64_t max_iter,
                                                          const double* __restrict__ r, const double* __restrict__ ap,
                                                          const Z* __restrict__ z) {
+    extern __shared__ double sm[];
     const int c = red_chunk<SPLIT>(), t = red_lane<SPLIT>(), pc = ch.piece[c];
     if (s.done[pc]) return;
     double next = 0.0, zap = 0.0;
-    red_chain<SPLIT ? 16 : 8>(
-        6 * ch.lo[c] + t, 6 * ch.lo[c + 1],
-        [&](int64_t i) { return make_double3(r[i], FLEX ? ap[i] : 0.0, (double)z[i]); },
-        [&](int64_t, const double3& v) {
-            next = fma(v.x, v.z, next);
-            if (FLEX) zap = fma(v.y, v.z, zap);
-        });
+    if (!red_run<SPLIT, FLEX ? 3 : 2, 8>(
+            sm, 6 * ch.lo[c] + t, 6 * ch.lo[c + 1],
+            [&](int64_t i, double (&v)[FLEX ? 3 : 2]) {
+                v[0] = r[i], v[1] = (double)z[i];
+                if constexpr (FLEX) v[2] = ap[i];
+            },
+            [&](const double (&v)[FLEX ? 3 : 2]) {
+                next = fma(v[0], v[1], next);
+                if constexpr (FLEX) zap = fma(v[2], v[1], zap);
+            }))
+        return;
     if (!red_finish<SPLIT>(ch, c, t, pc, next, zap)) return;
     s.beta[pc] = FLEX ? -s.alpha[pc] * zap / s.rz[pc] : next / s.rz[pc];
     s.rz[pc] = next;
@@ -645,6 +683,19 @@ static void residual_floor(Context& ctx, Batch& b, const double* x, double* ff) 
     dot2<double>(ctx, L, nullptr, kd.get(), kd.get(), ff, nullptr);
 }
 
+template <class Z, bool FLEX, bool SPLIT>
+static void launch_dots(unsigned grid, cudaStream_t st, const Chunks& ch, const CgScalars& s, int64_t max_iter,
+                        const double* r, const double* ap, const Z* z) {
+    constexpr size_t smem = red_smem<SPLIT>(FLEX ? 3 : 2);
+    static const bool attr_set = [] {  // once per instantiation (thread-safe)
+        SC_CK(cudaFuncSetAttribute(k_dots_beta<Z, FLEX, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)smem));
+        return true;
+    }();
+    (void)attr_set;
+    k_dots_beta<Z, FLEX, SPLIT><<<grid, RED_LANES, smem, st>>>(ch, s, max_iter, r, ap, z);
+}
+
 // Times a solve may replace the residuals of pieces whose true residual missed the goal.
 constexpr int MAX_REPLACEMENTS = 8;
 
@@ -712,16 +763,15 @@ static int64_t pcg(Context& ctx, Batch& b, const V* rhs, S* x, V* r, V* z, V* p,
         }
         if (L.nchunks <= 0) return;  // no parts: every piece is done
         const unsigned grid = red_grid(L.nchunks);
-        const int block = red_block(L.nchunks);
         float* r32 = same ? nullptr : reinterpret_cast<float*>(rp);
         auto passes = [&](auto split) {
             constexpr bool SPLIT = decltype(split)::value;
-            k_dot_alpha<SPLIT><<<grid, block, 0, st>>>(ch, cg.s, p, ap);
+            k_dot_alpha<SPLIT><<<grid, RED_LANES, red_smem<SPLIT>(2), st>>>(ch, cg.s, p, ap);
             SC_LAUNCH_CK();
-            k_update_xr<SPLIT><<<grid, block, 0, st>>>(ch, cg.s, x, p, r, ap, r32);
+            k_update_xr<SPLIT><<<grid, RED_LANES, red_smem<SPLIT>(1), st>>>(ch, cg.s, x, p, r, ap, r32);
             SC_LAUNCH_CK();
             precondition();
-            k_dots_beta<P, !same, SPLIT><<<grid, block, 0, st>>>(ch, cg.s, max_iter, r, ap, zs);
+            launch_dots<P, !same, SPLIT>(grid, st, ch, cg.s, max_iter, r, ap, zs);
             SC_LAUNCH_CK();
         };
         if (red_split(L.nchunks))

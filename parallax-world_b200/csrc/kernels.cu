@@ -420,11 +420,14 @@ __global__ void __launch_bounds__(256) k_top_solve(const int32_t* __restrict__ t
 template <class T, bool SPLIT>
 __global__ void __launch_bounds__(RED_LANES) k_seg_dot(Chunks ch, const T* __restrict__ a, const T* __restrict__ b,
                                                        double* __restrict__ out) {
+    extern __shared__ double sm[];
     const int c = red_chunk<SPLIT>(), t = red_lane<SPLIT>(), p = ch.piece[c];
     double s = 0.0, none = 0.0;
-    red_chain<SPLIT ? 16 : 8>(
-        6 * ch.lo[c] + t, 6 * ch.lo[c + 1], [&](int64_t i) { return make_double2((double)a[i], (double)b[i]); },
-        [&](int64_t, const double2& v) { s = fma(v.x, v.y, s); });
+    if (!red_run<SPLIT, 2, 8>(
+            sm, 6 * ch.lo[c] + t, 6 * ch.lo[c + 1],
+            [&](int64_t i, double (&v)[2]) { v[0] = (double)a[i], v[1] = (double)b[i]; },
+            [&](const double (&v)[2]) { s = fma(v[0], v[1], s); }))
+        return;
     if (red_finish<SPLIT>(ch, c, t, p, s, none)) out[p] = s;
 }
 
@@ -432,14 +435,16 @@ __global__ void __launch_bounds__(RED_LANES) k_seg_dot(Chunks ch, const T* __res
 template <bool SPLIT>
 __global__ void __launch_bounds__(RED_LANES) k_power_step(Chunks ch, const double* __restrict__ w,
                                                           const double* __restrict__ v, double* __restrict__ step) {
+    extern __shared__ double sm[];
     const int c = red_chunk<SPLIT>(), t = red_lane<SPLIT>(), p = ch.piece[c];
     double ww = 0.0, vv = 0.0;
-    red_chain<SPLIT ? 16 : 8>(
-        6 * ch.lo[c] + t, 6 * ch.lo[c + 1], [&](int64_t i) { return make_double2(w[i], v[i]); },
-        [&](int64_t, const double2& x) {
-            ww = fma(x.x, x.x, ww);
-            vv = fma(x.y, x.y, vv);
-        });
+    if (!red_run<SPLIT, 2, 8>(
+            sm, 6 * ch.lo[c] + t, 6 * ch.lo[c + 1], [&](int64_t i, double (&x)[2]) { x[0] = w[i], x[1] = v[i]; },
+            [&](const double (&x)[2]) {
+                ww = fma(x[0], x[0], ww);
+                vv = fma(x[1], x[1], vv);
+            }))
+        return;
     if (red_finish<SPLIT>(ch, c, t, p, ww, vv)) step[p] = 4.0 / 3.0 / (sqrt(ww) / sqrt(vv));
 }
 
@@ -573,11 +578,10 @@ void seg_dot_t(Context& ctx, const Level& L, const T* a, const T* b, double* out
     if (L.nchunks <= 0) return;
     const Chunks ch = red_chunks(ctx, L);
     const unsigned grid = red_grid(L.nchunks);
-    const int block = red_block(L.nchunks);
     if (red_split(L.nchunks))
-        k_seg_dot<T, true><<<grid, block, 0, ctx.stream>>>(ch, a, b, out);
+        k_seg_dot<T, true><<<grid, RED_LANES, red_smem<true>(2), ctx.stream>>>(ch, a, b, out);
     else
-        k_seg_dot<T, false><<<grid, block, 0, ctx.stream>>>(ch, a, b, out);
+        k_seg_dot<T, false><<<grid, RED_LANES, 0, ctx.stream>>>(ch, a, b, out);
     SC_LAUNCH_CK();
 }
 
@@ -587,11 +591,10 @@ void power_step(Context& ctx, const Level& L, const double* w, const double* v, 
     if (L.nchunks <= 0) return;
     const Chunks ch = red_chunks(ctx, L);
     const unsigned grid = red_grid(L.nchunks);
-    const int block = red_block(L.nchunks);
     if (red_split(L.nchunks))
-        k_power_step<true><<<grid, block, 0, ctx.stream>>>(ch, w, v, step);
+        k_power_step<true><<<grid, RED_LANES, red_smem<true>(2), ctx.stream>>>(ch, w, v, step);
     else
-        k_power_step<false><<<grid, block, 0, ctx.stream>>>(ch, w, v, step);
+        k_power_step<false><<<grid, RED_LANES, 0, ctx.stream>>>(ch, w, v, step);
     SC_LAUNCH_CK();
 }
 

@@ -54,10 +54,12 @@ __device__ __forceinline__ void st6(T* __restrict__ p, const T (&o)[6]) {
 // meet in a tree again.
 //
 // The order leaves each lane a serial chain of up to 96 values, and the launch decides where
-// the lanes run. WHOLE: a block a chunk. SPLIT, where that would leave most of the device
-// idle: a warp (a block of its own) 32 lanes of a chunk, 8 warps a chunk, 16 values' loads in
-// flight a lane. The last of a chunk's warps to arrive adds its lanes, the last of a piece's
-// chunks the piece, so no launch follows for the sums or for the scalars that come of them.
+// the lanes run. WHOLE: a block a chunk, a thread a lane. SPLIT, where that would leave most
+// of the device idle: a block 32 lanes of a chunk, whose eight warps bring the lanes' values
+// to shared memory (a warp alone gets one load in some 55 cycles) and whose first warp runs
+// the chains from there. The last of a chunk's blocks to arrive adds its lanes, the last of
+// a piece's chunks the piece, so no launch follows for the sums or for the scalars that
+// come of them.
 constexpr int RED_LANES = 256;
 struct Chunks {
     const int64_t* lo = nullptr;           // nchunks + 1 bounds, in parts
@@ -72,7 +74,9 @@ struct Chunks {
 constexpr int64_t RED_WHOLE = 592;
 inline bool red_split(int64_t nchunks) { return nchunks < RED_WHOLE; }
 inline unsigned red_grid(int64_t nchunks) { return (unsigned)(red_split(nchunks) ? 8 * nchunks : nchunks); }
-inline int red_block(int64_t nchunks) { return red_split(nchunks) ? 32 : RED_LANES; }
+constexpr int RED_STEPS = 6 * CHUNK / RED_LANES;  // a lane's values at most
+template <bool SPLIT>
+constexpr size_t red_smem(int streams) { return SPLIT ? (size_t)streams * RED_STEPS * 32 * sizeof(double) : 0; }
 
 // This thread's chunk and lane.
 template <bool SPLIT>
@@ -81,7 +85,7 @@ __device__ __forceinline__ int red_chunk() {
 }
 template <bool SPLIT>
 __device__ __forceinline__ int red_lane() {
-    return SPLIT ? (int)((blockIdx.x & 7) * 32 + threadIdx.x) : (int)threadIdx.x;
+    return SPLIT ? (int)((blockIdx.x & 7) * 32 + (threadIdx.x & 31)) : (int)threadIdx.x;
 }
 
 // A lane's chain: use(i, load(i)) for i = first, first + 256, ... below end, in that order, U
@@ -106,7 +110,51 @@ __device__ __forceinline__ void red_chain(int64_t first, int64_t end, F&& load, 
         if (i + RED_LANES * j < end) use(i + RED_LANES * j, v[j]);
 }
 
-// Every thread of the kernel comes here with its lane's sums a and b. True in one thread of
+// This lane's values from first to end, S numbers each, in order. WHOLE: load(i, v), then
+// use(v), U values' loads in flight. SPLIT: the block's warps load, and its first warp uses;
+// false in the others, whose part ends here. sm: red_smem(S) bytes.
+template <bool SPLIT, int S, int U, class F, class G>
+__device__ __forceinline__ bool red_run(double* sm, int64_t first, int64_t end, F&& load, G&& use) {
+    if constexpr (!SPLIT) {
+        struct V {
+            double v[S];
+        };
+        red_chain<U>(
+            first, end,
+            [&](int64_t i) {
+                V x;
+                load(i, x.v);
+                return x;
+            },
+            [&](int64_t, const V& x) { use(x.v); });
+        return true;
+    } else {
+        const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+        constexpr int PER = RED_STEPS / 8;  // a warp's steps: w, w + 8, ...
+        double v[PER][S];
+#pragma unroll
+        for (int u = 0; u < PER; u++)
+            if (first + RED_LANES * (int64_t)(w + 8 * u) < end) load(first + RED_LANES * (int64_t)(w + 8 * u), v[u]);
+#pragma unroll
+        for (int u = 0; u < PER; u++)
+            if (first + RED_LANES * (int64_t)(w + 8 * u) < end)
+#pragma unroll
+                for (int q = 0; q < S; q++) sm[(q * RED_STEPS + w + 8 * u) * 32 + l] = v[u][q];
+        __syncthreads();
+        if (w != 0) return false;
+        const int n = first < end ? (int)((end - first + RED_LANES - 1) / RED_LANES) : 0;
+#pragma unroll 8
+        for (int k = 0; k < n; k++) {
+            double x[S];
+#pragma unroll
+            for (int q = 0; q < S; q++) x[q] = sm[(q * RED_STEPS + k) * 32 + l];
+            use(x);
+        }
+        return true;
+    }
+}
+
+// Every thread that red_run left going comes here with its lane's sums a and b. True in one thread of
 // the last warp to arrive of the chunk's piece, with the piece's sums in a and b.
 template <bool SPLIT>
 __device__ __forceinline__ bool red_finish(const Chunks& ch, int c, int t, int p, double& a, double& b) {
