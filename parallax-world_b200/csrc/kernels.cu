@@ -108,6 +108,7 @@ template <class T>
 __device__ __forceinline__ T row_stream(Ring<T>& ring, int64_t first, int64_t e1, int stride,
                                         const int32_t* __restrict__ col, const T* __restrict__ val,
                                         const T* __restrict__ x) {
+    static_assert(sizeof(T) == 8, "the 16-byte copies of x need 16-byte parts");
     constexpr int PIECES = 36 * (int)sizeof(T) / 16;  // 16-byte pieces of a block
     const int lane = threadIdx.x & 31, g = lane >> 3, rr = lane & 7;
     T acc = T(0);
@@ -377,23 +378,18 @@ __global__ void k_jacobi_add(int64_t n, const T* __restrict__ inv, const T* __re
     st6<T>(z + 6 * k, o);
 }
 
-// z = Kinv r over each top piece's parts, FP64 arithmetic: row i adds A[j][i] r[j] in the
-// order of j. What bounds it is that chain and the loads it waits for (a warp alone gets one
-// load in some 55 cycles), so 32 rows are a block whose eight warps bring TOP_TILE values of j
-// to shared memory at a time and whose first warp runs the chain: a 96-row top 30 to 4.6 us, a
+// z_i = sum over j of A[j][i] r_j in the order of j, FP64, for the 32 rows i from i0 on. What
+// bounds it is that chain and the loads it waits for (a warp alone gets one load in some 55
+// cycles), so 32 rows are a block whose eight warps bring TOP_TILE values of j to shared
+// memory at a time and whose first warp runs the chain: a 96-row top 30 to 4.6 us, a
 // 132-row one 41 to 6.6 (before, one block a piece, each thread waiting for its own loads).
 constexpr int TOP_TILE = 128;
 template <class T>
-__global__ void __launch_bounds__(256) k_top_solve(const int32_t* __restrict__ top, const int64_t* __restrict__ pstart,
-                                                   const int64_t* __restrict__ kinv_off, const double* __restrict__ kinv,
-                                                   const T* __restrict__ r, T* __restrict__ z,
-                                                   const int32_t* __restrict__ done) {
+__device__ __forceinline__ void dense_rows(int n, int i0, const double* __restrict__ A0, const T* __restrict__ r,
+                                           T* __restrict__ z) {
     __shared__ double tile[TOP_TILE][32], rs[TOP_TILE];
-    const int p = top[blockIdx.x], w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    const int64_t k0 = pstart[p], off = kinv_off[blockIdx.x];
-    const int n = (int)(6 * (pstart[p + 1] - k0)), i = blockIdx.y * 32 + l;
-    if ((done && done[p]) || (int)blockIdx.y * 32 >= n) return;
-    const double* A = kinv + off + i;
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31, i = i0 + l;
+    const double* A = A0 + i;
     double s = 0.0;
     for (int j0 = 0; j0 < n; j0 += TOP_TILE) {
         if (j0) __syncthreads();
@@ -403,7 +399,7 @@ __global__ void __launch_bounds__(256) k_top_solve(const int32_t* __restrict__ t
             const int j = j0 + w + 8 * k;
             a[k] = j < n && i < n ? __ldg(A + (int64_t)j * n) : 0.0;
         }
-        if (threadIdx.x < TOP_TILE && j0 + (int)threadIdx.x < n) rs[threadIdx.x] = (double)r[6 * k0 + j0 + threadIdx.x];
+        if (threadIdx.x < TOP_TILE && j0 + (int)threadIdx.x < n) rs[threadIdx.x] = (double)r[j0 + threadIdx.x];
 #pragma unroll
         for (int k = 0; k < TOP_TILE / 8; k++) tile[w + 8 * k][l] = a[k];
         __syncthreads();
@@ -413,7 +409,26 @@ __global__ void __launch_bounds__(256) k_top_solve(const int32_t* __restrict__ t
             for (int j = 0; j < m; j++) s = fma(tile[j][l], rs[j], s);
         }
     }
-    if (w == 0 && i < n) z[6 * k0 + i] = (T)s;
+    if (w == 0 && i < n) z[i] = (T)s;
+}
+
+// z = Kinv r over each top piece's parts
+template <class T>
+__global__ void __launch_bounds__(256) k_top_solve(const int32_t* __restrict__ top, const int64_t* __restrict__ pstart,
+                                                   const int64_t* __restrict__ kinv_off, const double* __restrict__ kinv,
+                                                   const T* __restrict__ r, T* __restrict__ z,
+                                                   const int32_t* __restrict__ done) {
+    const int p = top[blockIdx.x];
+    const int64_t k0 = pstart[p], off = kinv_off[blockIdx.x];
+    const int n = (int)(6 * (pstart[p + 1] - k0)), i0 = blockIdx.y * 32;
+    if ((done && done[p]) || i0 >= n) return;
+    dense_rows<T>(n, i0, kinv + off, r + 6 * k0, z + 6 * k0);
+}
+
+// x = A' b, A (n x n) row-major
+__global__ void __launch_bounds__(256) k_dense_apply(int n, const double* __restrict__ A, const double* __restrict__ b,
+                                                     double* __restrict__ x) {
+    dense_rows<double>(n, blockIdx.x * 32, A, b, x);
 }
 
 // out[p] = sum over piece p's parts of a.b
@@ -545,6 +560,12 @@ void top_solve(Context& ctx, const Level& L, const T* r, T* z, const int32_t* do
     const dim3 grid((unsigned)L.top_h.size(), grid_for(maxn, 32));
     k_top_solve<T><<<grid, 256, 0, ctx.stream>>>(L.top.get(), L.pstart_d.get(), L.kinv_off.get(), L.kinv.get(), r, z,
                                                  done);
+    SC_LAUNCH_CK();
+}
+
+void dense_apply(Context& ctx, int64_t n, const double* A, const double* b, double* x) {
+    if (n <= 0) return;
+    k_dense_apply<<<grid_for(n, 32), 256, 0, ctx.stream>>>((int)n, A, b, x);
     SC_LAUNCH_CK();
 }
 

@@ -248,6 +248,8 @@ void top_solve(Context& ctx, const Level& L, const T* r, T* z, const int32_t* do
 template <class T>
 void seg_dot_t(Context& ctx, const Level& L, const T* a, const T* b, double* out);
 
+// x = A' b, A dense (n x n, row-major)
+void dense_apply(Context& ctx, int64_t n, const double* A, const double* b, double* x);
 // per piece the smoother's step from the last power iteration, w = D^-1 K v
 void power_step(Context& ctx, const Level& L, const double* w, const double* v, double* step);
 

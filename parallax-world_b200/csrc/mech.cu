@@ -449,30 +449,51 @@ HLevel coarsen(const Fine& f, double size) {  // solve.rs:241-271
 }
 
 // ---- the device ---------------------------------------------------------------------
-// y = S x (resid: y = b - S x) over the nodes' 3x3 block rows
-__global__ void k_bsr3(int64_t n, const int64_t* __restrict__ rowptr, const int32_t* __restrict__ col,
-                       const double* __restrict__ val, const double* __restrict__ x, const double* __restrict__ b,
-                       double* __restrict__ y) {
-    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+// y = S x (b given: y = b - S x) over the nodes' 3x3 block rows, a warp a row: lane 3 b + r
+// takes row r of block b, ten blocks at a time and thirty in flight, x's three values passed
+// between a block's lanes, and lanes 0 to 2 add the blocks' terms in order. What bounds it is
+// the lines each load touches: 3 a block so, 7 where a thread, or three, take a row each and
+// every load of a warp goes to as many rows (36 us on a 40^3 piece; 29 now).
+constexpr int BSR3_WARPS = 8;
+__global__ void __launch_bounds__(32 * BSR3_WARPS) k_bsr3(int64_t n, const int64_t* __restrict__ rowptr,
+                                                          const int32_t* __restrict__ col,
+                                                          const double* __restrict__ val, const double* __restrict__ x,
+                                                          const double* __restrict__ b, double* __restrict__ y) {
+    constexpr int U = 3, SET = 10 * U;
+    __shared__ double term[BSR3_WARPS][SET][3];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t i = (int64_t)blockIdx.x * BSR3_WARPS + w;
     if (i >= n) return;
-    double a0 = 0.0, a1 = 0.0, a2 = 0.0;
-    for (int64_t e = rowptr[i]; e < rowptr[i + 1]; e++) {
-        const double* m = val + 9 * e;
-        const double* xv = x + 3 * (int64_t)col[e];
-        const double x0 = xv[0], x1 = xv[1], x2 = xv[2];
-        a0 += m[0] * x0 + m[1] * x1 + m[2] * x2;
-        a1 += m[3] * x0 + m[4] * x1 + m[5] * x2;
-        a2 += m[6] * x0 + m[7] * x1 + m[8] * x2;
+    const int blk = min(lane / 3, 9), r = lane % 3, first = 3 * blk;
+    const int64_t e1 = rowptr[i + 1];
+    double a = 0.0;
+    for (int64_t base = rowptr[i]; base < e1; base += SET) {
+        double m[U][3], xr[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int64_t e = base + 10 * u + blk;
+            m[u][0] = m[u][1] = m[u][2] = xr[u] = 0.0;
+            if (lane < 30 && e < e1) {
+                const double* mp = val + 9 * e + 3 * r;
+                m[u][0] = mp[0], m[u][1] = mp[1], m[u][2] = mp[2];
+                xr[u] = x[3 * (int64_t)col[e] + r];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const double x0 = __shfl_sync(0xffffffffu, xr[u], first), x1 = __shfl_sync(0xffffffffu, xr[u], first + 1),
+                         x2 = __shfl_sync(0xffffffffu, xr[u], first + 2);
+            if (lane < 30) term[w][10 * u + blk][r] = m[u][0] * x0 + m[u][1] * x1 + m[u][2] * x2;
+        }
+        __syncwarp();
+        if (lane < 3) {
+            const int k1 = (int)min((int64_t)SET, e1 - base);
+#pragma unroll 10
+            for (int k = 0; k < k1; k++) a += term[w][k][lane];
+        }
+        __syncwarp();
     }
-    if (b) {
-        y[3 * i] = b[3 * i] - a0;
-        y[3 * i + 1] = b[3 * i + 1] - a1;
-        y[3 * i + 2] = b[3 * i + 2] - a2;
-    } else {
-        y[3 * i] = a0;
-        y[3 * i + 1] = a1;
-        y[3 * i + 2] = a2;
-    }
+    if (lane < 3) y[3 * i + lane] = b ? b[3 * i + lane] - a : a;
 }
 
 // out = base + step * inv (v - w) per node (base, w nullable: 0; base may be out)
@@ -489,34 +510,62 @@ __global__ void k_jacobi3(int64_t n, const double* __restrict__ inv, double step
     }
 }
 
-// rb[a] = sum over a's members p of (r_t, r_w + rp x r_t); W = 3 (nodes: r_w = 0) or 6
+// rb[a] = sum over a's members p of (r_t, r_w + rp x r_t); W = 3 (nodes: r_w = 0) or 6; then
+// (xa not null) the level's first smoothing, xa = step D^-1 rb, while rb is at hand. A thread
+// a part adds its members in order, four members' loads in flight.
 template <int W>
-__global__ void k_restrict(int64_t nc, const int64_t* __restrict__ mptr, const int32_t* __restrict__ mem,
-                           const double* __restrict__ rr, const double* __restrict__ v, const double* __restrict__ w,
-                           double* __restrict__ rb) {
+__global__ void __launch_bounds__(64) k_restrict(int64_t nc, const int64_t* __restrict__ mptr,
+                                                 const int32_t* __restrict__ mem, const double* __restrict__ rr,
+                                                 const double* __restrict__ v, const double* __restrict__ w,
+                                                 double* __restrict__ rb, const double* __restrict__ inv,
+                                                 const double* __restrict__ step, double* __restrict__ xa) {
     int64_t a = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (a >= nc) return;
+    constexpr int U = 4;
     double o[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    for (int64_t t = mptr[a]; t < mptr[a + 1]; t++) {
-        const int64_t p = mem[t];
-        double f[6];
-        for (int k = 0; k < W; k++) f[k] = w ? v[W * p + k] - w[W * p + k] : v[W * p + k];
-        const double r0 = rr[3 * p], r1 = rr[3 * p + 1], r2 = rr[3 * p + 2];
-        const double t0 = r1 * f[2] - r2 * f[1], t1 = r2 * f[0] - r0 * f[2], t2 = r0 * f[1] - r1 * f[0];
-        o[0] += f[0];
-        o[1] += f[1];
-        o[2] += f[2];
-        if (W == 6) {
-            o[3] += f[3] + t0;
-            o[4] += f[4] + t1;
-            o[5] += f[5] + t2;
-        } else {
-            o[3] += t0;
-            o[4] += t1;
-            o[5] += t2;
-        }
+    const int64_t t1 = mptr[a + 1];
+    for (int64_t t = mptr[a]; t < t1; t += U) {
+        int64_t p[U];
+        double f[U][W], r[U][3];
+#pragma unroll
+        for (int u = 0; u < U; u++) p[u] = t + u < t1 ? mem[t + u] : -1;
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (p[u] >= 0) {
+#pragma unroll
+                for (int k = 0; k < W; k++) f[u][k] = w ? v[W * p[u] + k] - w[W * p[u] + k] : v[W * p[u] + k];
+#pragma unroll
+                for (int k = 0; k < 3; k++) r[u][k] = rr[3 * p[u] + k];
+            }
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (p[u] >= 0) {
+                const double r0 = r[u][0], r1 = r[u][1], r2 = r[u][2];
+                const double t0 = r1 * f[u][2] - r2 * f[u][1], t1w = r2 * f[u][0] - r0 * f[u][2],
+                             t2 = r0 * f[u][1] - r1 * f[u][0];
+                o[0] += f[u][0];
+                o[1] += f[u][1];
+                o[2] += f[u][2];
+                if constexpr (W == 6) {
+                    o[3] += f[u][3] + t0;
+                    o[4] += f[u][4] + t1w;
+                    o[5] += f[u][5] + t2;
+                } else {
+                    o[3] += t0;
+                    o[4] += t1w;
+                    o[5] += t2;
+                }
+            }
     }
     for (int k = 0; k < 6; k++) rb[6 * a + k] = o[k];
+    if (!xa) return;
+    const double st = step[0];
+    for (int i = 0; i < 6; i++) {
+        double s = 0.0;
+#pragma unroll
+        for (int k = 0; k < 6; k++) s = fma(inv[36 * a + 6 * i + k], o[k], s);
+        xa[6 * a + i] = s * st;
+    }
 }
 
 // x[p] += (e_t + e_w x r_p, e_w) of its part (W = 3: the translation only)
@@ -535,20 +584,28 @@ __global__ void k_prolong(int64_t nf, const int32_t* __restrict__ of, const doub
         for (int k = 3; k < 6; k++) x[W * p + k] += ea[k];
 }
 
-// x = A^-1 b, A^-1 (m x m) laid out as out[c * m + r]
-__global__ void k_top(int64_t m, const double* __restrict__ ainv, const double* __restrict__ b, double* __restrict__ x) {
-    for (int64_t r = threadIdx.x; r < m; r += blockDim.x) {
-        double s = 0.0;
-        for (int64_t c = 0; c < m; c++) s += ainv[c * m + r] * b[c];
-        x[r] = s;
-    }
-}
+// The PCG's scalars (solve.rs:485-538) where the iterations run on the device: the loop
+// goes on until `stop`, with `rounds` the rounds the reference would report.
+struct MechCG {
+    double rz, target, pap, alpha, beta, nx;
+    int32_t stop, round, rounds;
+    uint32_t count;   // rounds since the graph's launch
+    uint32_t ticket;  // k_mdot's blocks that arrived (zero between kernels)
+};
 
-// per-block partial sums of a . b, a fixed order
+// a . b as MDOT_BLOCKS partial sums, a fixed order. With c, the last block to arrive adds
+// them in order (as the host adds them where c is null) and takes the scalar step that
+// follows: two launches of one thread, the first waiting for one partial sum after another,
+// came after each dot before.
+// STEP 0, after p'Ap: a round that meets p'Ap <= 0 stops (and counts), else alpha = rz / p'Ap.
+// STEP 1, after r'z: beta = r'z / rz, rz = r'z, the round done, and the next round's tests
+// (solve.rs: the cap stops, rz < 0 gives None, rz <= target stops).
 constexpr int MDOT_BLOCKS = 256;
+template <int STEP>
 __global__ void __launch_bounds__(256) k_mdot(int64_t n, const double* __restrict__ a, const double* __restrict__ b,
-                                              double* __restrict__ part) {
+                                              double* part, MechCG* c) {
     __shared__ double red[256];
+    __shared__ bool last;
     const int64_t per = (n + MDOT_BLOCKS - 1) / MDOT_BLOCKS;
     const int64_t lo = blockIdx.x * per, hi = min(n, lo + per);
     double s = 0.0;
@@ -559,41 +616,38 @@ __global__ void __launch_bounds__(256) k_mdot(int64_t n, const double* __restric
         if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
         __syncthreads();
     }
-    if (threadIdx.x == 0) part[blockIdx.x] = red[0];
-}
-
-// The PCG's scalars (solve.rs:485-538) where the iterations run on the device: the loop
-// goes on until `stop`, with `rounds` the rounds the reference would report.
-struct MechCG {
-    double rz, target, pap, alpha, beta, nx;
-    int32_t stop, round, rounds;
-    uint32_t count;  // rounds since the graph's launch
-};
-
-// *out = the partial sums of k_mdot, added in order (as the host adds them)
-__global__ void k_mdot_sum(const double* __restrict__ part, double* __restrict__ out) {
-    double s = 0.0;
-    for (int i = 0; i < MDOT_BLOCKS; i++) s += part[i];
-    *out = s;
-}
-
-// after p'Ap: a round that meets p'Ap <= 0 stops (and counts), else alpha = rz / p'Ap
-__global__ void k_mcg_alpha(MechCG* c) {
-    if (c->stop) return;
-    if (c->pap <= 0.0) {
-        c->rounds = c->round;
-        c->stop = 1;
-    } else {
-        c->alpha = c->rz / c->pap;
+    if (threadIdx.x == 0) {
+        __stcg(part + blockIdx.x, red[0]);
+        if (c) {
+            __threadfence();
+            last = atomicAdd(&c->ticket, 1u) == MDOT_BLOCKS - 1;
+        }
     }
-}
-
-// after r'z: beta = r'z / rz, rz = r'z, the round done, and the next round's tests
-// (solve.rs: the cap stops, rz < 0 gives None, rz <= target stops)
-__global__ void k_mcg_beta(MechCG* c) {
+    if (!c) return;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    red[threadIdx.x] = __ldcg(part + threadIdx.x);
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    c->ticket = 0;
+    s = 0.0;
+#pragma unroll 16
+    for (int i = 0; i < MDOT_BLOCKS; i++) s += red[i];
+    if (STEP == 0) c->pap = s;
+    else c->nx = s;
     if (c->stop) return;
-    c->beta = c->nx / c->rz;
-    c->rz = c->nx;
+    if (STEP == 0) {
+        if (s <= 0.0) {
+            c->rounds = c->round;
+            c->stop = 1;
+        } else {
+            c->alpha = c->rz / s;
+        }
+        return;
+    }
+    c->beta = s / c->rz;
+    c->rz = s;
     c->round += 1;
     if (c->round >= MECH_ROUNDS) {  // the cap ends the loop before its tests
         c->rounds = MECH_ROUNDS;
@@ -607,26 +661,26 @@ __global__ void k_mcg_beta(MechCG* c) {
     }
 }
 
-// the loop's condition: on while not stopped and fewer than `chunk` rounds ran since the
-// launch (so the host looks in now and then)
-__global__ void k_mcg_more(cudaGraphConditionalHandle h, MechCG* c, uint32_t chunk) {
-    const uint32_t n = c->count + 1u;
-    c->count = n;
-    cudaGraphSetConditional(h, (!c->stop && n < chunk) ? 1u : 0u);
-}
-
-// k_mupdate with the step from the device's scalars; nothing once stopped
-__global__ void k_mupdate_d(int64_t n, int update, const MechCG* __restrict__ c, double* __restrict__ x,
-                            double* __restrict__ r, const double* __restrict__ p, const double* __restrict__ ap) {
-    if (c->stop) return;
-    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
+// update 0: x += alpha p, r -= alpha Ap; 1: x = r + beta x (x = p, r = z), and the device-side
+// loop's condition (loop): on while not stopped and fewer than `chunk` rounds ran since the
+// launch (so the host looks in now and then). Nothing once stopped.
+__global__ void k_mupdate_d(int64_t n, int update, MechCG* __restrict__ c, double* __restrict__ x,
+                            double* __restrict__ r, const double* __restrict__ p, const double* __restrict__ ap,
+                            bool loop, cudaGraphConditionalHandle h, uint32_t chunk) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const bool stop = c->stop;
+    if (loop && i == 0) {
+        const uint32_t k = c->count + 1u;
+        c->count = k;
+        cudaGraphSetConditional(h, (!stop && k < chunk) ? 1u : 0u);
+    }
+    if (stop || i >= n) return;
     if (update == 0) {
         const double s = c->alpha;
         x[i] = x[i] + p[i] * s;
         r[i] = r[i] - ap[i] * s;
     } else {
-        x[i] = r[i] + x[i] * c->beta;  // x = p, r = z
+        x[i] = r[i] + x[i] * c->beta;
     }
 }
 
@@ -639,7 +693,7 @@ struct MechSolver {
     MechSolver(Context& c, MechLevels& m) : ctx(c), M(m) {}
 
     double dot(const double* a, const double* b, int64_t n) {
-        k_mdot<<<MDOT_BLOCKS, 256, 0, ctx.stream>>>(n, a, b, part.get());
+        k_mdot<0><<<MDOT_BLOCKS, 256, 0, ctx.stream>>>(n, a, b, part.get(), nullptr);
         SC_LAUNCH_CK();
         part.download(hpart.data(), MDOT_BLOCKS);
         SC_CK(cudaStreamSynchronize(ctx.stream));
@@ -647,40 +701,43 @@ struct MechSolver {
         for (int i = 0; i < MDOT_BLOCKS; i++) s += hpart[i];
         return s;
     }
-    // *out = a . b on the device (the same partial sums, added in the same order, as dot)
-    void dot_d(const double* a, const double* b, int64_t n, double* out) {
-        k_mdot<<<MDOT_BLOCKS, 256, 0, ctx.stream>>>(n, a, b, part.get());
-        SC_LAUNCH_CK();
-        k_mdot_sum<<<1, 1, 0, ctx.stream>>>(part.get(), out);
+    // a . b on the device (the same partial sums, added in the same order, as dot) and the
+    // scalar step after it
+    template <int STEP>
+    void dot_step(const double* a, const double* b, int64_t n, MechCG* c) {
+        k_mdot<STEP><<<MDOT_BLOCKS, 256, 0, ctx.stream>>>(n, a, b, part.get(), c);
         SC_LAUNCH_CK();
     }
     void times(const double* x, double* y, const double* b = nullptr) {
-        k_bsr3<<<grid_for(M.n0, 128), 128, 0, ctx.stream>>>(M.n0, M.rowptr0.get(), M.col0.get(), M.val0.get(), x, b,
-                                                             y);
+        k_bsr3<<<grid_for(M.n0, BSR3_WARPS), 32 * BSR3_WARPS, 0, ctx.stream>>>(M.n0, M.rowptr0.get(), M.col0.get(),
+                                                                               M.val0.get(), x, b, y);
         SC_LAUNCH_CK();
     }
-    // x = V-cycle of level l for its b (solve.rs:403-447)
+    // level l's b from the finer residual v (- w), and where the level smooths, its first x
+    template <int W>
+    void restrict_to(size_t l, const double* v, const double* w) {
+        MechLevel& U = M.lv[l];
+        k_restrict<W><<<grid_for(U.n, 64), 64, 0, ctx.stream>>>(U.n, U.mptr.get(), U.mem.get(), U.r.get(), v, w,
+                                                                U.b.get(), U.inv.get(), U.step.get(),
+                                                                U.direct ? nullptr : U.x.get());
+        SC_LAUNCH_CK();
+    }
+    // x = V-cycle of level l for its b, its first smoothing done (solve.rs:403-447)
     void cycle(size_t l) {
         MechLevel& L = M.lv[l];
         if (L.direct) {
-            k_top<<<1, 256, 0, ctx.stream>>>(6 * L.n, L.top_inv.get(), L.b.get(), L.x.get());
-            SC_LAUNCH_CK();
+            dense_apply(ctx, 6 * L.n, L.top_inv.get(), L.b.get(), L.x.get());
             return;
         }
         MechLevel& U = M.lv[l + 1];
-        jacobi<double>(ctx, L.n, L.inv.get(), L.b.get(), L.x.get(), L.step.get(), nullptr, nullptr, nullptr);
         spmv<double>(ctx, SPMV_RES, L.n, L.rowptr.get(), L.col.get(), L.val.get(), L.x.get(), L.b.get(), L.res.get(),
                      nullptr, nullptr, nullptr, nullptr, nullptr, L.nnzb);
-        k_restrict<6><<<grid_for(U.n, 128), 128, 0, ctx.stream>>>(U.n, U.mptr.get(), U.mem.get(), U.r.get(),
-                                                                   L.res.get(), nullptr, U.b.get());
-        SC_LAUNCH_CK();
+        restrict_to<6>(l + 1, L.res.get(), nullptr);
         cycle(l + 1);
         k_prolong<6><<<grid_for(L.n, 256), 256, 0, ctx.stream>>>(L.n, U.of.get(), U.r.get(), U.x.get(), L.x.get());
         SC_LAUNCH_CK();
-        spmv<double>(ctx, SPMV_RES, L.n, L.rowptr.get(), L.col.get(), L.val.get(), L.x.get(), L.b.get(), L.res.get(),
-                     nullptr, nullptr, nullptr, nullptr, nullptr, L.nnzb);
-        jacobi_add<double>(ctx, L.n, L.inv.get(), L.res.get(), L.x.get(), L.t.get(), L.step.get(), nullptr, nullptr,
-                           nullptr);
+        spmv<double>(ctx, SPMV_RES_SMOOTH, L.n, L.rowptr.get(), L.col.get(), L.val.get(), L.x.get(), L.b.get(),
+                     L.t.get(), L.inv.get(), L.step.get(), nullptr, nullptr, nullptr, L.nnzb);
         std::swap(L.x, L.t);
     }
     // out = the preconditioner of b (solve.rs:450-476); scratch: 3 n0
@@ -690,9 +747,7 @@ struct MechSolver {
         SC_LAUNCH_CK();
         times(out, scratch);
         MechLevel& U = M.lv[0];
-        k_restrict<3><<<grid_for(U.n, 128), 128, 0, ctx.stream>>>(U.n, U.mptr.get(), U.mem.get(), U.r.get(), b,
-                                                                   scratch, U.b.get());
-        SC_LAUNCH_CK();
+        restrict_to<3>(0, b, scratch);
         cycle(0);
         k_prolong<3><<<g, 256, 0, ctx.stream>>>(M.n0, U.of.get(), U.r.get(), U.x.get(), out);
         SC_LAUNCH_CK();
@@ -981,25 +1036,22 @@ static int device_rounds(Context& ctx, MechSolver& S, int64_t m, double rz, doub
     cg.upload(&c0, 1);
     MechCG* c = cg.get();
     const unsigned g = grid_for(m, 256);
+    const uint32_t chunk = 64;
+    cudaGraphConditionalHandle h = 0;
+    bool loop = true;  // the round being launched is the device-side loop's
     auto round = [&] {
         S.times(p, ap);
-        S.dot_d(p, ap, m, &c->pap);
-        k_mcg_alpha<<<1, 1, 0, st>>>(c);
-        SC_LAUNCH_CK();
-        k_mupdate_d<<<g, 256, 0, st>>>(m, 0, c, x, r, p, ap);
+        S.dot_step<0>(p, ap, m, c);
+        k_mupdate_d<<<g, 256, 0, st>>>(m, 0, c, x, r, p, ap, false, h, chunk);
         SC_LAUNCH_CK();
         S.precondition(r, z, scratch);
-        S.dot_d(r, z, m, &c->nx);
-        k_mcg_beta<<<1, 1, 0, st>>>(c);
-        SC_LAUNCH_CK();
-        k_mupdate_d<<<g, 256, 0, st>>>(m, 1, c, p, z, nullptr, nullptr);
+        S.dot_step<1>(r, z, m, c);
+        k_mupdate_d<<<g, 256, 0, st>>>(m, 1, c, p, z, nullptr, nullptr, loop, h, chunk);
         SC_LAUNCH_CK();
     };
-    const uint32_t chunk = 64;
     cudaGraphExec_t exec = nullptr;
     {
         cudaGraph_t graph = nullptr;
-        cudaGraphConditionalHandle h = 0;
         cudaGraphNodeParams prm = {};
         prm.type = cudaGraphNodeTypeConditional;
         prm.conditional.type = cudaGraphCondTypeWhile;
@@ -1013,8 +1065,6 @@ static int device_rounds(Context& ctx, MechSolver& S, int64_t m, double rz, doub
             cudaGraph_t body = nullptr;
             try {
                 round();
-                k_mcg_more<<<1, 1, 0, st>>>(h, c, chunk);
-                SC_LAUNCH_CK();
             } catch (...) {
                 cudaStreamEndCapture(st, &body);
                 cudaGraphDestroy(graph);
@@ -1026,6 +1076,7 @@ static int device_rounds(Context& ctx, MechSolver& S, int64_t m, double rz, doub
         cudaGetLastError();
         if (graph) cudaGraphDestroy(graph);
     }
+    loop = false;
     MechCG now{};
     try {
         for (;;) {
