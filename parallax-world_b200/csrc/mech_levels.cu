@@ -169,41 +169,56 @@ __global__ void k_pair_ends(int64_t np, const uint32_t* __restrict__ pi, const u
 }
 
 // y = S x over B-vectors (solve.rs:63-73, 306-317): the diagonal block's terms, then each
-// pair touching the row in pair order
+// pair touching the row in pair order. LANES lanes a row, one of its B values each, so that
+// a block's rows are read side by side (a thread a row: 56 us a product on the levels of a
+// 40^3 piece, 13 now), two pairs' loads in flight.
+template <int B>
+constexpr int inc_lanes() { return B == 3 ? 4 : 8; }
 template <int B>
 __global__ void k_incidence_apply(int64_t n, const int64_t* __restrict__ ptr, const uint64_t* __restrict__ ent,
                                   const double* __restrict__ diag, const double* __restrict__ pm,
                                   const uint32_t* __restrict__ pi, const uint32_t* __restrict__ pj,
                                   const double* __restrict__ x, double* __restrict__ y) {
+    const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t i = tid / inc_lanes<B>();
+    const int r = (int)(tid % inc_lanes<B>());
+    if (i >= n || r >= B) return;
+    constexpr int U = 2;
+    double yv = 0.0;
+    for (int c = 0; c < B; c++) yv += diag[(int64_t)B * B * i + B * r + c] * x[(int64_t)B * i + c];
+    const int64_t t1 = ptr[i + 1];
+    for (int64_t t = ptr[i]; t < t1; t += U) {
+        double m[U][B], xv[U][B];
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (t + u < t1) {
+                const uint64_t e = ent[t + u];
+                const int64_t q = (int64_t)(e >> 1);
+                const bool turned = e & 1;  // the block's transpose
+                const double* mp = pm + (int64_t)B * B * q + (turned ? r : B * r);
+                const double* xj = x + (int64_t)B * (turned ? pi[q] : pj[q]);
+#pragma unroll
+                for (int c = 0; c < B; c++) {
+                    m[u][c] = mp[turned ? B * c : c];
+                    xv[u][c] = xj[c];
+                }
+            }
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (t + u < t1) {
+                double a = 0.0;
+#pragma unroll
+                for (int c = 0; c < B; c++) a += m[u][c] * xv[u][c];
+                yv += a;
+            }
+    }
+    y[(int64_t)B * i + r] = yv;
+}
+
+// v = w / norm
+__global__ void k_over_norm(int64_t n, const double* __restrict__ w, double norm, double* __restrict__ v) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double yv[B];
-    for (int r = 0; r < B; r++) {
-        double acc = 0.0;
-        for (int c = 0; c < B; c++) acc += diag[(int64_t)B * B * i + B * r + c] * x[(int64_t)B * i + c];
-        yv[r] = acc;
-    }
-    for (int64_t t = ptr[i]; t < ptr[i + 1]; t++) {
-        const uint64_t e = ent[t];
-        const int64_t q = (int64_t)(e >> 1);
-        const double* m = pm + (int64_t)B * B * q;
-        if ((e & 1) == 0) {
-            const double* xj = x + (int64_t)B * pj[q];
-            for (int r = 0; r < B; r++) {
-                double a = 0.0;
-                for (int c = 0; c < B; c++) a += m[B * r + c] * xj[c];
-                yv[r] += a;
-            }
-        } else {
-            const double* xj = x + (int64_t)B * pi[q];
-            for (int r = 0; r < B; r++) {
-                double a = 0.0;
-                for (int c = 0; c < B; c++) a += m[B * c + r] * xj[c];
-                yv[r] += a;
-            }
-        }
-    }
-    for (int r = 0; r < B; r++) y[(int64_t)B * i + r] = yv[r];
+    if (i < n) v[i] = w[i] / norm;
 }
 
 // y = inv x, part by part
@@ -423,17 +438,12 @@ __global__ void k_row_fill(int64_t n, int64_t m, const uint64_t* __restrict__ sk
     col[t] = (int32_t)(skey[t] & 0xffffffffull);
     const int64_t s = ssrc[t];
     double* out = val + (int64_t)B * B * t;
-    if (s < 0) {
-        const double* d = diag + (int64_t)B * B * (-1 - s);
-        for (int k = 0; k < B * B; k++) out[k] = d[k];
+    const double* p = s < 0 ? diag + (int64_t)B * B * (-1 - s) : pm + (int64_t)B * B * (s >> 1);
+    if (s >= 0 && (s & 1)) {
+        for (int x = 0; x < B; x++)
+            for (int y = 0; y < B; y++) out[B * x + y] = p[B * y + x];
     } else {
-        const double* p = pm + (int64_t)B * B * (s >> 1);
-        if (s & 1) {
-            for (int x = 0; x < B; x++)
-                for (int y = 0; y < B; y++) out[B * x + y] = p[B * y + x];
-        } else {
-            for (int k = 0; k < B * B; k++) out[k] = p[k];
-        }
+        for (int k = 0; k < B * B; k++) out[k] = p[k];
     }
 }
 
@@ -483,33 +493,46 @@ double host_norm(const std::vector<double>& v) {
 }
 
 // 4/3 over the largest eigenvalue of inv S, ten power steps from the reference's start
-// (solve.rs:274-296): the products on the device, the norms on the host in order
+// (solve.rs:274-296): the products and the scaling on the device, the norms, sums in the
+// order of the values, on the host from a copy. The estimate is the last step's |w| / |v|, so
+// only the last step needs |v| -- unless w vanishes, when the steps run again with both.
 template <int B>
 double power_step(Context& ctx, const DevSys& s, const DevIncidence& I, const double* inv) {
     cudaStream_t st = ctx.stream;
     MemStats* ms = &ctx.mem;
     const int64_t n = s.n;
+    constexpr int STEPS = 10;
     std::vector<double> v((size_t)(B * n)), w((size_t)(B * n));
-    for (int64_t k = 0; k < n; k++)
-        for (int q = 0; q < B; q++) v[(size_t)(B * k + q)] = 1.0 + (double)((7 * k + 3 * q) % 11) / 11.0;
     DBuf<double> dv, da, dw;
     dv.alloc(B * n, st, ms);
     da.alloc(B * n, st, ms);
     dw.alloc(B * n, st, ms);
-    double most = 1.0;
-    for (int it = 0; it < 10; it++) {
+    auto run = [&](bool both, double& most) {
+        for (int64_t k = 0; k < n; k++)
+            for (int q = 0; q < B; q++) v[(size_t)(B * k + q)] = 1.0 + (double)((7 * k + 3 * q) % 11) / 11.0;
         dv.upload(v.data(), v.size());
-        k_incidence_apply<B><<<grid_for(n, LT), LT, 0, st>>>(n, I.ptr.get(), I.ent.get(), s.diag.get(), s.pm.get(),
-                                                            s.pi.get(), s.pj.get(), dv.get(), da.get());
-        SC_LAUNCH_CK();
-        k_block_over<B><<<grid_for(n, LT), LT, 0, st>>>(n, inv, da.get(), dw.get());
-        SC_LAUNCH_CK();
-        dw.download(w.data(), w.size());
-        SC_CK(cudaStreamSynchronize(st));
-        const double nw = host_norm(w), nv = host_norm(v);
-        if (nw == 0.0) break;
-        most = nw / nv;
-        for (size_t k = 0; k < v.size(); k++) v[k] = w[k] / nw;
+        for (int it = 0; it < STEPS; it++) {
+            k_incidence_apply<B><<<grid_for(inc_lanes<B>() * n, LT), LT, 0, st>>>(
+                n, I.ptr.get(), I.ent.get(), s.diag.get(), s.pm.get(), s.pi.get(), s.pj.get(), dv.get(), da.get());
+            SC_LAUNCH_CK();
+            k_block_over<B><<<grid_for(n, LT), LT, 0, st>>>(n, inv, da.get(), dw.get());
+            SC_LAUNCH_CK();
+            dw.download(w.data(), w.size());
+            const bool need_v = both || it + 1 == STEPS;
+            if (need_v) dv.download(v.data(), v.size());
+            SC_CK(cudaStreamSynchronize(st));
+            const double nw = host_norm(w);
+            if (nw == 0.0) return false;
+            if (need_v) most = nw / host_norm(v);
+            k_over_norm<<<grid_for(B * n, LT), LT, 0, st>>>(B * n, dw.get(), nw, dv.get());
+            SC_LAUNCH_CK();
+        }
+        return true;
+    };
+    double most = 1.0;
+    if (!run(false, most)) {
+        most = 1.0;
+        run(true, most);
     }
     return 4.0 / 3.0 / most;
 }
