@@ -312,7 +312,8 @@ void check_lattice(const sc_lattice& lat) {
 // motions (bodies.rs:429-468) of a lattice into out (6 per node, device), zeros for held
 // and gone nodes; returns the solve's status (the hierarchy stays as ctx.last)
 sc_status lattice_motions(Context& c, const sc_lattice& lat, const uint8_t* alive, const uint8_t* gone,
-                          const double* loads, const sc_options& opt, double* out, sc_solve_info* info) {
+                          const double* loads, const sc_options& opt, double* out, sc_solve_info* info,
+                          const LatticeOnDevice* dev) {
     auto b = std::make_unique<Batch>();
     c.last.reset();  // the previous solve's hierarchy is not kept through this one
     // Every node held or gone: nothing to solve, every motion zero (the reference's CG
@@ -331,7 +332,7 @@ sc_status lattice_motions(Context& c, const sc_lattice& lat, const uint8_t* aliv
     }
     SC_CK(cudaStreamSynchronize(c.stream));
     c.mem.peak = c.mem.now;
-    lattice_level0(c, *b, lat, alive, gone, loads);
+    lattice_level0(c, *b, lat, alive, gone, loads, dev);
     DBuf<double> x;
     SolveStats st;
     double solve_ms = 0;

@@ -224,42 +224,47 @@ int bits_for2(int64_t v) {
 }  // namespace
 
 void lattice_level0(Context& ctx, Batch& b, const sc_lattice& Lt, const uint8_t* alive_h, const uint8_t* gone_h,
-                    const double* loads_h) {
+                    const double* loads_h, const LatticeOnDevice* dev) {
     cudaStream_t st = ctx.stream;
     MemStats* ms = &ctx.mem;
     int64_t nn = Lt.n_nodes, nb = Lt.n_bonds;
     b.npieces = 1;
     b.base_level = Lt.level;
-    auto up = [&](auto* host, size_t count, auto& buf) {
-        buf.alloc(std::max<size_t>(count, 1), st, ms);
-        if (host) buf.upload(host, count);
-    };
     DBuf<double> x, p, n, a, d, e, g, loads;
     DBuf<int64_t> bi, bj, around;
     DBuf<uint8_t> held, alive, gone;
-    up(Lt.x, 3 * nn, x);
-    up(Lt.bond_p, 3 * nb, p);
-    up(Lt.bond_n, 3 * nb, n);
-    up(Lt.bond_a, nb, a);
-    up(Lt.bond_d, nb, d);
-    up(Lt.bond_e, nb, e);
-    up(Lt.bond_g, nb, g);
-    up(Lt.bond_i, nb, bi);
-    up(Lt.bond_j, nb, bj);
-    up(Lt.around, 6 * nn, around);
-    up(Lt.held, nn, held);
-    up(loads_h, 6 * nn, loads);
-    if (alive_h) up(alive_h, nb, alive);
-    if (gone_h) up(gone_h, nn, gone);
-    const uint8_t* al = alive_h ? alive.get() : nullptr;
-    const uint8_t* gn = gone_h ? gone.get() : nullptr;
-    BondsD B{bi.get(), bj.get(), p.get(), n.get(), a.get(), d.get(), e.get(), g.get(), x.get()};
+    LatticeOnDevice D{};
+    if (dev) {
+        D = *dev;
+    } else {
+        auto up = [&](const auto* host, size_t count, auto& buf) {
+            buf.alloc(std::max<size_t>(count, 1), st, ms);
+            if (host) buf.upload(host, count);
+            return buf.get();
+        };
+        D.x = up(Lt.x, 3 * nn, x);
+        D.p = up(Lt.bond_p, 3 * nb, p);
+        D.n = up(Lt.bond_n, 3 * nb, n);
+        D.a = up(Lt.bond_a, nb, a);
+        D.d = up(Lt.bond_d, nb, d);
+        D.e = up(Lt.bond_e, nb, e);
+        D.g = up(Lt.bond_g, nb, g);
+        D.bi = up(Lt.bond_i, nb, bi);
+        D.bj = up(Lt.bond_j, nb, bj);
+        D.around = up(Lt.around, 6 * nn, around);
+        D.held = up(Lt.held, nn, held);
+        D.loads = up(loads_h, 6 * nn, loads);
+        D.alive = alive_h ? up(alive_h, nb, alive) : nullptr;
+        D.gone = gone_h ? up(gone_h, nn, gone) : nullptr;
+    }
+    const uint8_t *al = D.alive, *gn = D.gone;
+    BondsD B{D.bi, D.bj, D.p, D.n, D.a, D.d, D.e, D.g, D.x};
     // parts
     DBuf<int64_t> isp, before;
     isp.alloc(nn + 1, st, ms);
     before.alloc(nn + 1, st, ms);
     SC_CK(cudaMemsetAsync(isp.get() + nn, 0, sizeof(int64_t), st));
-    k_part_flags<<<grid_for(nn, 256), 256, 0, st>>>(nn, held.get(), gn, isp.get());
+    k_part_flags<<<grid_for(nn, 256), 256, 0, st>>>(nn, D.held, gn, isp.get());
     SC_LAUNCH_CK();
     size_t tb = 0;
     cub::DeviceScan::ExclusiveSum(nullptr, tb, isp.get(), before.get(), nn + 1, st);
@@ -287,7 +292,7 @@ void lattice_level0(Context& ctx, Batch& b, const sc_lattice& Lt, const uint8_t*
     L.site.alloc(3 * nparts, st, ms);
     L.piece.alloc(nparts, st, ms);
     b.loads.alloc(6 * nparts, st, ms);
-    k_part_geom<<<grid_for(nparts, 256), 256, 0, st>>>(nparts, b.part_node.get(), x.get(), around.get(), loads.get(),
+    k_part_geom<<<grid_for(nparts, 256), 256, 0, st>>>(nparts, b.part_node.get(), D.x, D.around, D.loads,
                                                        L.centre.get(), L.site.get(), b.loads.get(), L.piece.get());
     SC_LAUNCH_CK();
     // block entries

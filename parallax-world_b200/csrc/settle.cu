@@ -108,13 +108,15 @@ __global__ void k_break_beams(int64_t nbeams, const double* __restrict__ used, c
     }
 }
 
-// the lattice's node positions, held flags and bonds (with strengths) on the device
+// the lattice's nodes, weights and bonds (with strengths) on the device: what a round's solve
+// and the use of its bonds read, uploaded once for all rounds
 struct DeviceLattice {
     int64_t n = 0, nb = 0;
     DBuf<double> x, p, nrm, a, d, e, g, ft, fc, fs;
-    DBuf<int64_t> bi, bj;
+    DBuf<int64_t> bi, bj, around;
     DBuf<uint8_t> held;
-    void load(Context& c, const sc_lattice& L, const sc_strength& S) {
+    DBuf<double> loads;
+    void load(Context& c, const sc_lattice& L, const sc_strength& S, const std::vector<double>& weights) {
         cudaStream_t st = c.stream;
         n = L.n_nodes;
         nb = L.n_bonds;
@@ -124,6 +126,8 @@ struct DeviceLattice {
         };
         up(x, L.x, 3 * n);
         up(held, L.held, n);
+        up(around, L.around, 6 * n);
+        up(loads, weights.data(), 6 * n);
         up(bi, L.bond_i, nb);
         up(bj, L.bond_j, nb);
         up(p, L.bond_p, 3 * nb);
@@ -167,21 +171,22 @@ void drop_unheld(Context& c, const DeviceLattice& D, const uint8_t* alive, uint8
     SC_LAUNCH_CK();
 }
 
-// forces under the weights and their use of the bonds' strengths, for the given alive /
+// the motions under the weights, the bonds' forces and their use of the bonds' strengths, for
+// the given alive /
 // gone flags (device); the solve's status
-sc_status round_used(Context& c, const sc_lattice& L, const DeviceLattice& D, const std::vector<double>& weights,
-                     const uint8_t* alive_d, const uint8_t* gone_d, const sc_options& opt, double* used_d,
-                     sc_solve_info* info, double& work) {
+sc_status round_used(Context& c, const sc_lattice& L, const DeviceLattice& D, const uint8_t* alive_d,
+                     const uint8_t* gone_d, const sc_options& opt, double* used_d, sc_solve_info* info, double& work) {
     cudaStream_t st = c.stream;
-    std::vector<uint8_t> alive_h(std::max<int64_t>(D.nb, 1)), gone_h(D.n);
-    if (D.nb) SC_CK(cudaMemcpyAsync(alive_h.data(), alive_d, D.nb, cudaMemcpyDeviceToHost, st));
+    std::vector<uint8_t> gone_h(D.n);
     SC_CK(cudaMemcpyAsync(gone_h.data(), gone_d, D.n, cudaMemcpyDeviceToHost, st));
     SC_CK(cudaStreamSynchronize(st));
     DBuf<double> u;
     u.alloc(6 * D.n, st, &c.mem);
     sc_solve_info local{};
     sc_solve_info* inf = info ? info : &local;
-    sc_status s = lattice_motions(c, L, alive_h.data(), gone_h.data(), weights.data(), opt, u.get(), inf);
+    const LatticeOnDevice dev{D.x.get(),  D.p.get(),  D.nrm.get(),    D.a.get(),    D.d.get(), D.e.get(), D.g.get(),
+                              D.loads.get(), D.bi.get(), D.bj.get(), D.around.get(), D.held.get(), alive_d,   gone_d};
+    sc_status s = lattice_motions(c, L, nullptr, gone_h.data(), nullptr, opt, u.get(), inf, &dev);
     work += inf->work;
     if (D.nb > 0) {
         k_bond_used<<<grid_for(D.nb, 256), 256, 0, st>>>(D.nb, D.view(), D.x.get(), u.get(), alive_d, gone_d, used_d);
@@ -202,7 +207,7 @@ sc_status used_standing(Context& c, const sc_lattice& L, const sc_strength& S, c
                         sc_solve_info* info) {
     cudaStream_t st = c.stream;
     DeviceLattice D;
-    D.load(c, L, S);
+    D.load(c, L, S, weights_of(L, S));
     DBuf<uint8_t> alive, gone;
     alive.alloc(std::max<int64_t>(D.nb, 1), st, &c.mem);
     SC_CK(cudaMemsetAsync(alive.get(), 1, std::max<int64_t>(D.nb, 1), st));
@@ -212,7 +217,7 @@ sc_status used_standing(Context& c, const sc_lattice& L, const sc_strength& S, c
     DBuf<double> u;
     u.alloc(std::max<int64_t>(D.nb, 1), st, &c.mem);
     double work = 0;
-    sc_status s = round_used(c, L, D, weights_of(L, S), alive.get(), gone.get(), opt, u.get(), info, work);
+    sc_status s = round_used(c, L, D, alive.get(), gone.get(), opt, u.get(), info, work);
     if (D.nb) u.download(used, D.nb);
     SC_CK(cudaStreamSynchronize(st));
     return s;
@@ -222,8 +227,7 @@ sc_status settle(Context& c, const sc_lattice& L, const sc_strength& S, const sc
                  sc_settle_info* out) {
     cudaStream_t st = c.stream;
     DeviceLattice D;
-    D.load(c, L, S);
-    const std::vector<double> w = weights_of(L, S);
+    D.load(c, L, S, weights_of(L, S));
     DBuf<uint8_t> alive, gone;
     alive.alloc(std::max<int64_t>(D.nb, 1), st, &c.mem);
     SC_CK(cudaMemsetAsync(alive.get(), 1, std::max<int64_t>(D.nb, 1), st));
@@ -241,7 +245,7 @@ sc_status settle(Context& c, const sc_lattice& L, const sc_strength& S, const sc
     for (;;) {
         rounds += 1;
         drop_unheld(c, D, alive.get(), gone.get());
-        sc_status s = round_used(c, L, D, w, alive.get(), gone.get(), opt, used.get(), nullptr, work);
+        sc_status s = round_used(c, L, D, alive.get(), gone.get(), opt, used.get(), nullptr, work);
         worst = std::max(worst, s);
         broke.zero();
         const int64_t nbeams = D.nb / PER_BEAM;

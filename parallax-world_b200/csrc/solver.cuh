@@ -180,8 +180,16 @@ void brick_jacobi(Context& ctx, const Batch& b, const T* r, T* x, const double* 
                   const int32_t* done);
 
 // --- lattice.cu -----------------------------------------------------------------------
+// A lattice's arrays where they lie on the device already (settle's rounds), as sc_lattice
+// has them, with the bonds alive, the nodes gone and the loads.
+struct LatticeOnDevice {
+    const double *x, *p, *n, *a, *d, *e, *g, *loads;
+    const int64_t *bi, *bj, *around;
+    const uint8_t *held, *alive, *gone;
+};
+// dev: read these instead of uploading L's arrays, alive, gone and loads
 void lattice_level0(Context& ctx, Batch& b, const sc_lattice& L, const uint8_t* alive, const uint8_t* gone,
-                    const double* loads);
+                    const double* loads, const LatticeOnDevice* dev = nullptr);
 
 // --- mech.cu: the engine's solver (mechanics/src/solve.rs) -----------------------------
 int mech_solve(Context& ctx, int64_t n, const int64_t* sites, const double* at, const double* diag, int64_t npairs,
@@ -218,7 +226,8 @@ void gather_full(const sc_material& m, double* out);
 // --- capi.cu / settle.cu -----------------------------------------------------------------
 // motions of a lattice into out_dev (6 per node, device); the solve's status
 sc_status lattice_motions(Context& ctx, const sc_lattice& L, const uint8_t* alive, const uint8_t* gone,
-                          const double* loads, const sc_options& opt, double* out_dev, sc_solve_info* info);
+                          const double* loads, const sc_options& opt, double* out_dev, sc_solve_info* info,
+                          const LatticeOnDevice* dev = nullptr);
 sc_status used_standing(Context& ctx, const sc_lattice& L, const sc_strength& S, const sc_options& opt,
                         double* used, sc_solve_info* info);
 sc_status settle(Context& ctx, const sc_lattice& L, const sc_strength& S, const sc_options& opt, uint8_t* gone,
