@@ -53,9 +53,12 @@ constexpr int NBOX = XB0 + XB1 + XB2;
 constexpr int KB = (BX + 1) * (BY + 1) * (BZ + 1);  // cells lo-1 .. hi-1
 constexpr int NNB = 13;                             // the brick and the twelve it reads from
 constexpr int HKX = BY * BZ, HKY = BX * BZ, HKZ = BX * BY, HK = HKX + HKY + HKZ;  // halo cells
-constexpr int BRICK_THREADS = 256;
+// Threads a brick: 256, two parts a thread in turn, where several bricks share an SM; 512
+// where the bricks are fewer than the SMs, and a brick's own time, not their throughput, is
+// what a stencil takes (a 32^3 FP64 solve, 122 bricks: 15.75 to 15.44 ms).
+constexpr int BRICK_THREADS = 256, BRICK_THREADS_FEW = 512, BRICK_FEW = 148;
 static_assert(NSLOT < 4096, "slot indices take 12 bits (halo_table)");
-static_assert(BRICK_THREADS == BCELLS, "the k box is filled a cell a thread");
+static_assert(BRICK_THREADS >= BCELLS, "the k box is filled a cell a thread");
 
 // The bricks a brick reads from, as offsets in brick units: itself, its six face
 // neighbours, and the six edge neighbours one step back along one axis and one step
@@ -491,15 +494,15 @@ __device__ __forceinline__ int own_entry(uint32_t c) {
 // Resident blocks an SM the register cap aims at: five in FP32 (shared memory allows
 // five), four where the epilogue applies the block-Jacobi factor (more registers, which
 // five blocks would spill), three in FP64 (shared memory allows three).
-template <class T, int MODE>
+template <class T, int MODE, int TH>
 constexpr int brick_min_blocks() {
-    return sizeof(T) == 8 ? 3 : (MODE == ST_RES_JAC || MODE == ST_PROLONG || MODE == ST_SMOOTH) ? 4 : 5;
+    return TH > BRICK_THREADS ? 1 : sizeof(T) == 8 ? 3 : (MODE == ST_RES_JAC || MODE == ST_PROLONG || MODE == ST_SMOOTH) ? 4 : 5;
 }
 
 // Level 0 applied over bricks, one thread block a brick (see the file's head). The same
 // epilogues as grid.cu's k_stencil: y = Kx, r - Kx, ... (ST_* in level0.cuh).
-template <class T, int MODE>
-__global__ void __launch_bounds__(BRICK_THREADS, brick_min_blocks<T, MODE>()) k_brick_stencil(BrickView v, const T* __restrict__ x,
+template <class T, int MODE, int TH>
+__global__ void __launch_bounds__(TH, brick_min_blocks<T, MODE, TH>()) k_brick_stencil(BrickView v, const T* __restrict__ x,
                                                                  const T* __restrict__ r, T* __restrict__ y,
                                                                  T* __restrict__ y2, T s,
                                                                  const double* __restrict__ step,
@@ -520,7 +523,7 @@ __global__ void __launch_bounds__(BRICK_THREADS, brick_min_blocks<T, MODE>()) k_
     {
         constexpr int N16 = (int)(sizeof(T) * 6 * NBOX / 16);
         float4* z = reinterpret_cast<float4*>(box);
-        for (int i = threadIdx.x; i < N16; i += BRICK_THREADS) z[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int i = threadIdx.x; i < N16; i += TH) z[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
     __syncthreads();
     // The box is filled by asynchronous copies (cp.async: global memory straight to shared
@@ -528,20 +531,20 @@ __global__ void __launch_bounds__(BRICK_THREADS, brick_min_blocks<T, MODE>()) k_
     // parts, their run read in order, each to its face's entry (by its part_code, kept for
     // the part phase), and the halo parts of its resolved list (bricks_build).
     const bool vec16 = sizeof(T) == 8 && ((reinterpret_cast<uintptr_t>(x) & 15) == 0);
-    for (int t = threadIdx.x; t < cnt; t += BRICK_THREADS) {
+    for (int t = threadIdx.x; t < cnt; t += TH) {
         const uint32_t c = __ldg(v.code + start + t);
         codes[t] = (uint16_t)c;
         copy_part<T>(box + 6 * own_entry(c), x + 6 * ((int64_t)start + t), vec16);
     }
     {
         const int32_t h0 = __ldg(v.hstart + b), h1 = __ldg(v.hstart + b + 1);
-        for (int32_t h = h0 + threadIdx.x; h < h1; h += BRICK_THREADS)
+        for (int32_t h = h0 + threadIdx.x; h < h1; h += TH)
             copy_part<T>(box + 6 * (int)__ldg(v.hent + h), x + 6 * (int64_t)__ldg(v.hsrc + h), vec16);
     }
     // k of the brick's cells and of the single layers before it (-x, -y, -z)
     {
-        const int t = threadIdx.x;  // BRICK_THREADS == BCELLS: one cell of the brick a thread
-        kbox[kbox_index(t / (BY * BZ), t / BZ % BY, t % BZ)] = __ldg(v.kd + (int64_t)b * BCELLS + t);
+        const int t = threadIdx.x;
+        if (t < BCELLS) kbox[kbox_index(t / (BY * BZ), t / BZ % BY, t % BZ)] = __ldg(v.kd + (int64_t)b * BCELLS + t);
         if (t < HK) {
             int h0, h1, h2;
             if (t < HKX) {
@@ -560,7 +563,7 @@ __global__ void __launch_bounds__(BRICK_THREADS, brick_min_blocks<T, MODE>()) k_
     const T* rb = r ? r + 6 * (int64_t)start : nullptr;
     T* yb = y + 6 * (int64_t)start;
     T* y2b = y2 ? y2 + 6 * (int64_t)start : nullptr;
-    for (int t = threadIdx.x; t < cnt; t += BRICK_THREADS) {
+    for (int t = threadIdx.x; t < cnt; t += TH) {
         const uint32_t c = codes[t];
         const int a = (c >> 12) & 3, l0 = (c >> 8) & 7, l1 = (c >> 4) & 15, l2 = c & 15;
         if (a == 0)
@@ -903,14 +906,23 @@ void brick_stencil(Context& ctx, const Batch& b, const T* x, const T* r, T* y, T
     const Bricks& K = b.grid.bricks;
     if (K.n_bricks <= 0) return;
     constexpr size_t smem = brick_smem<T>();
+    auto go = [&](auto kernel, int threads) {
+        kernel<<<(unsigned)K.n_bricks, threads, smem, ctx.stream>>>(view_of(K), x, r, y, y2, (T)b.grid.s, step, skip_row,
+                                                                   done);
+        SC_LAUNCH_CK();
+    };
     static const bool attr_set = [] {  // once per instantiation (thread-safe)
-        SC_CK(cudaFuncSetAttribute(k_brick_stencil<T, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        SC_CK(cudaFuncSetAttribute(k_brick_stencil<T, MODE, BRICK_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)smem));
+        SC_CK(cudaFuncSetAttribute(k_brick_stencil<T, MODE, BRICK_THREADS_FEW>,
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         return true;
     }();
     (void)attr_set;
-    k_brick_stencil<T, MODE><<<(unsigned)K.n_bricks, BRICK_THREADS, smem, ctx.stream>>>(
-        view_of(K), x, r, y, y2, (T)b.grid.s, step, skip_row, done);
-    SC_LAUNCH_CK();
+    if (K.n_bricks <= BRICK_FEW)
+        go(k_brick_stencil<T, MODE, BRICK_THREADS_FEW>, BRICK_THREADS_FEW);
+    else
+        go(k_brick_stencil<T, MODE, BRICK_THREADS>, BRICK_THREADS);
 }
 
 #define SC_BRICK_MODES(T)                                                                                            \
