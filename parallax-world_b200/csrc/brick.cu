@@ -45,10 +45,13 @@ constexpr int BCELLS = BX * BY * BZ;
 constexpr int NS0 = (BX + 1) * BY * BZ, NS1 = BX * (BY + 1) * BZ, NS2 = BX * BY * (BZ + 1);
 constexpr int NSLOT = NS0 + NS1 + NS2;
 constexpr int MW = (NSLOT + 31) / 32;  // mask words a brick
-// the box of axis-a faces a brick reads: positions lo-1 .. hi along a, lo-1 .. hi-1
-// along the other two
-constexpr int XB0 = (BX + 2) * (BY + 1) * (BZ + 1), XB1 = (BX + 1) * (BY + 2) * (BZ + 1),
-              XB2 = (BX + 1) * (BY + 1) * (BZ + 2);
+// The box of axis-a faces a brick reads: positions lo-1 .. hi along a, lo-1 .. hi-1 along the
+// other two. Rows of BZ + 2 entries and planes alike modulo 16 on the three axes: a part's
+// twelve reads then lie at entries a fixed distance from its own face's modulo 16, and lanes
+// whose own faces differ there meet no bank conflict in any of them (see k_part_codes).
+constexpr int BOX_ROW = BZ + 2, BOX_PLANE0 = (BY + 1) * BOX_ROW, BOX_PLANE1 = (BY + 2) * BOX_ROW + 6;
+static_assert(BOX_PLANE0 % 16 == BOX_PLANE1 % 16, "planes alike modulo 16");
+constexpr int XB0 = (BX + 2) * BOX_PLANE0, XB1 = (BX + 1) * BOX_PLANE1, XB2 = (BX + 1) * BOX_PLANE0;
 constexpr int NBOX = XB0 + XB1 + XB2;
 constexpr int KB = (BX + 1) * (BY + 1) * (BZ + 1);  // cells lo-1 .. hi-1
 constexpr int NNB = 13;                             // the brick and the twelve it reads from
@@ -91,10 +94,11 @@ __host__ __device__ inline int slot_of(int a, int l0, int l1, int l2) {
     return slot_off(a) + (l0 * slot_ext(a, 1) + l1) * slot_ext(a, 2) + l2;
 }
 __host__ __device__ constexpr int box_ext(int a, int d) { return slot_ext(a, d) + 1; }
+__host__ __device__ constexpr int box_plane(int a) { return a == 1 ? BOX_PLANE1 : BOX_PLANE0; }
 __host__ __device__ constexpr int box_off(int a) { return a == 0 ? 0 : a == 1 ? XB0 : XB0 + XB1; }
 // box entry of axis-a face position c (brick-local cell coordinates, -1 .. B)
-__device__ __forceinline__ int box_index(int a, int c0, int c1, int c2) {
-    return box_off(a) + ((c0 + 1) * box_ext(a, 1) + (c1 + 1)) * box_ext(a, 2) + (c2 + 1);
+__host__ __device__ constexpr int box_index(int a, int c0, int c1, int c2) {
+    return box_off(a) + (c0 + 1) * box_plane(a) + (c1 + 1) * BOX_ROW + (c2 + 1);
 }
 __device__ __forceinline__ int kbox_index(int c0, int c1, int c2) {
     return ((c0 + 1) * (BY + 1) + (c1 + 1)) * (BZ + 1) + (c2 + 1);
@@ -115,19 +119,30 @@ struct BrickView {
     const int32_t* nbr;    // NNB a brick: the bricks of NB_OFF_H, -1 where none
     const float* kd;       // BCELLS a brick: each cell's k, 0 where not free
     const BrickGeo* geo;   // per piece
-    const uint16_t* code;  // per part (brick order): its part_code
+    const uint16_t* code;  // per part, 32 a group from its brick's first: the part_codes (k_part_codes)
     const int32_t* hstart; // n_bricks + 1: each brick's halo list
     const uint16_t* hent;  // per halo item: the box entry it fills
     const int32_t* hsrc;   // per halo item: the part (brick order) it comes from
     const float* hk;       // per brick, HK values: the k of the cells of its -x, -y, -z layers
 };
 
-// A part's slot as the part phase reads it: axis (bits 12-13), brick-local face position
-// l (l0 bits 8-10, l1 bits 4-7, l2 bits 0-3).
-__host__ __device__ constexpr uint32_t part_code(int a, int l0, int l1, int l2) {
-    return ((uint32_t)a << 12) | ((uint32_t)l0 << 8) | ((uint32_t)l1 << 4) | (uint32_t)l2;
+// A part as the part phase reads it: its place in its group of 32 (bits 11-15), its axis a
+// (bits 9-10), whether its face lies on the + plane of extra slots (bit 8: l_a is a's extent,
+// its field 0), and its brick-local face position l (l0 bits 6-7, l1 bits 3-5, l2 bits 0-2).
+__host__ __device__ constexpr uint32_t part_code(int at, int a, int l0, int l1, int l2) {
+    const uint32_t plane = (a == 0 ? l0 / BX : a == 1 ? l1 / BY : l2 / BZ) & 1;
+    return ((uint32_t)at << 11) | ((uint32_t)a << 9) | (plane << 8) | ((uint32_t)(l0 % BX) << 6) |
+           ((uint32_t)(l1 % BY) << 3) | (uint32_t)(l2 % BZ);
 }
-static_assert(BX + 1 < 8 && BY + 1 < 16 && BZ + 1 < 16, "part_code fields");
+static_assert(BX == 4 && BY == 8 && BZ == 8, "part_code fields");
+struct PartAt {
+    int a, l0, l1, l2;
+};
+__device__ __forceinline__ PartAt part_at(uint32_t c) {
+    const int a = (c >> 9) & 3, plane = (c >> 8) & 1;
+    return {a, (int)((c >> 6) & 3) + (a == 0 ? BX * plane : 0), (int)((c >> 3) & 7) + (a == 1 ? BY * plane : 0),
+            (int)(c & 7) + (a == 2 ? BZ * plane : 0)};
+}
 
 // The entries of a brick's box that other bricks hold, the same for every brick (the
 // brick's own parts go to the box straight from their run, by their part_code). Entry i
@@ -142,12 +157,9 @@ std::vector<uint2> halo_table() {
     std::vector<uint2> t;
     constexpr CodeTable code = make_code_table();
     const int B[3] = {BX, BY, BZ};
-    for (int i = 0; i < NBOX; i++) {
-        const int a = i < XB0 ? 0 : i < XB0 + XB1 ? 1 : 2;
-        const int rem = i - box_off(a);
-        const int e2 = box_ext(a, 2), e1 = box_ext(a, 1);
-        const int c[3] = {rem / (e2 * e1) - 1, rem / e2 % e1 - 1, rem % e2 - 1};
-        if ((c[0] < 0) + (c[1] < 0) + (c[2] < 0) > 1) continue;  // read by no part
+    auto entry = [&](int a, const int (&c)[3]) {
+        const int i = box_index(a, c[0], c[1], c[2]);
+        if ((c[0] < 0) + (c[1] < 0) + (c[2] < 0) > 1) return;  // read by no part
         int o[3], l[3], oa[3], la[3];
         for (int d = 0; d < 3; d++) {
             if (c[d] < 0) {
@@ -165,12 +177,16 @@ std::vector<uint2> halo_table() {
         }
         const int q = code.v[(o[0] + 1) * 9 + (o[1] + 1) * 3 + (o[2] + 1)];
         const int qa = code.v[(oa[0] + 1) * 9 + (oa[1] + 1) * 3 + (oa[2] + 1)];
-        if (q == 0) continue;  // an own slot
+        if (q == 0) return;  // an own slot
         const bool plane = c[a] >= B[a];
         t.push_back(make_uint2(((uint32_t)q << 27) | ((uint32_t)a << 25) | ((plane ? 1u : 0u) << 24) |
                                    ((uint32_t)i << 12) | (uint32_t)slot_of(a, l[0], l[1], l[2]),
                                ((uint32_t)qa << 27) | (uint32_t)slot_of(a, la[0], la[1], la[2])));
-    }
+    };
+    for (int a = 0; a < 3; a++)
+        for (int c0 = -1; c0 < box_ext(a, 0) - 1; c0++)
+            for (int c1 = -1; c1 < box_ext(a, 1) - 1; c1++)
+                for (int c2 = -1; c2 < box_ext(a, 2) - 1; c2++) entry(a, {c0, c1, c2});
     return t;
 }
 
@@ -479,7 +495,7 @@ __device__ __forceinline__ void copy_part(T* dst, const T* src, bool vec16) {
 }
 
 // Shared memory of one brick: the x box (NBOX faces, 6 values each), the k box and the
-// brick's parts' part_codes in storage order.
+// brick's parts' part_codes.
 template <class T>
 constexpr size_t brick_smem() {
     return sizeof(T) * 6 * NBOX + sizeof(float) * KB + sizeof(uint16_t) * (NSLOT + 8);
@@ -487,8 +503,8 @@ constexpr size_t brick_smem() {
 
 // the box entry of an own part's face, from its part_code
 __device__ __forceinline__ int own_entry(uint32_t c) {
-    const int a = (c >> 12) & 3, l0 = (c >> 8) & 7, l1 = (c >> 4) & 15, l2 = c & 15;
-    return a == 0 ? box_index(0, l0, l1, l2) : a == 1 ? box_index(1, l0, l1, l2) : box_index(2, l0, l1, l2);
+    const PartAt p = part_at(c);
+    return box_index(p.a, p.l0, p.l1, p.l2);
 }
 
 // Resident blocks an SM the register cap aims at: five in FP32 (shared memory allows
@@ -528,13 +544,13 @@ __global__ void __launch_bounds__(TH, brick_min_blocks<T, MODE, TH>()) k_brick_s
     __syncthreads();
     // The box is filled by asynchronous copies (cp.async: global memory straight to shared
     // memory, no registers in between) issued together and awaited once: the brick's own
-    // parts, their run read in order, each to its face's entry (by its part_code, kept for
-    // the part phase), and the halo parts of its resolved list (bricks_build).
+    // parts, a warp a group of 32 of its run, each to its face's entry (by its part_code, kept
+    // for the part phase), and the halo parts of its resolved list (bricks_build).
     const bool vec16 = sizeof(T) == 8 && ((reinterpret_cast<uintptr_t>(x) & 15) == 0);
     for (int t = threadIdx.x; t < cnt; t += TH) {
         const uint32_t c = __ldg(v.code + start + t);
         codes[t] = (uint16_t)c;
-        copy_part<T>(box + 6 * own_entry(c), x + 6 * ((int64_t)start + t), vec16);
+        copy_part<T>(box + 6 * own_entry(c), x + 6 * ((int64_t)start + (t & ~31) + (int)(c >> 11)), vec16);
     }
     {
         const int32_t h0 = __ldg(v.hstart + b), h1 = __ldg(v.hstart + b + 1);
@@ -559,19 +575,20 @@ __global__ void __launch_bounds__(TH, brick_min_blocks<T, MODE, TH>()) k_brick_s
     }
     cp_async_wait_all();
     __syncthreads();
-    // the brick's parts, in storage order (their vectors from the brick's first part on)
+    // the brick's parts, a warp a group (their vectors from the brick's first part on)
     const T* rb = r ? r + 6 * (int64_t)start : nullptr;
     T* yb = y + 6 * (int64_t)start;
     T* y2b = y2 ? y2 + 6 * (int64_t)start : nullptr;
     for (int t = threadIdx.x; t < cnt; t += TH) {
         const uint32_t c = codes[t];
-        const int a = (c >> 12) & 3, l0 = (c >> 8) & 7, l1 = (c >> 4) & 15, l2 = c & 15;
-        if (a == 0)
-            brick_part<0, T, MODE>(box, kbox, l0, l1, l2, t, rb, yb, y2b, s, w);
-        else if (a == 1)
-            brick_part<1, T, MODE>(box, kbox, l0, l1, l2, t, rb, yb, y2b, s, w);
+        const PartAt p = part_at(c);
+        const int q = (t & ~31) + (int)(c >> 11);
+        if (p.a == 0)
+            brick_part<0, T, MODE>(box, kbox, p.l0, p.l1, p.l2, q, rb, yb, y2b, s, w);
+        else if (p.a == 1)
+            brick_part<1, T, MODE>(box, kbox, p.l0, p.l1, p.l2, q, rb, yb, y2b, s, w);
         else
-            brick_part<2, T, MODE>(box, kbox, l0, l1, l2, t, rb, yb, y2b, s, w);
+            brick_part<2, T, MODE>(box, kbox, p.l0, p.l1, p.l2, q, rb, yb, y2b, s, w);
     }
 }
 
@@ -682,21 +699,37 @@ BrickView view_of(const Bricks& K) {
     return v;
 }
 
-// each brick-ordered part's part_code, from its sort key's slot
-__global__ void k_part_codes(int64_t n, const uint64_t* __restrict__ key, uint16_t* __restrict__ code) {
-    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    int e = (int)(key[i] % NSLOT);
-    int a = 0;
-    if (e >= NS0 + NS1) {
-        a = 2;
-        e -= NS0 + NS1;
-    } else if (e >= NS0) {
-        a = 1;
-        e -= NS0;
+// The part_codes of each brick's parts, from their sort keys' slots, in the order in which the
+// stencil's lanes take them. A warp takes the 32 parts of a group (its global accesses are those
+// of parts in order); within it, parts of one axis whose box entries are equal modulo 16 would
+// meet in the same banks, so lanes take first one part of each residue, then the next of each,
+// and so on: each half of the warp (FP32: 24 bytes an entry in 8-byte loads; FP64: a quarter,
+// 16-byte loads) reads distinct residues as far as the group has them. Counted on a 64^3 piece
+// the box's reads take 250 k wavefronts instead of 308 k of at least 165 k (FP32), 450 k instead
+// of 567 k of 315 k (FP64); ordering all of a brick would leave 200 k and 363 k but spread a
+// warp's 24 bytes a part over 10.4 lines instead of 5.8. At 128^3 the mixed solve 387.1 to 383.6
+// ms, FP64 524.4 to 520.8. A block a brick.
+__global__ void __launch_bounds__(256) k_part_codes(const int32_t* __restrict__ start, const uint64_t* __restrict__ key,
+                                                    uint16_t* __restrict__ code) {
+    const int32_t s0 = start[blockIdx.x], cnt = start[blockIdx.x + 1] - s0;
+    const int lane = threadIdx.x & 31;
+    for (int t0 = threadIdx.x - lane; t0 < cnt; t0 += blockDim.x) {
+        const bool in = t0 + lane < cnt;
+        int a = 3, l0 = 0, l1 = 0, l2 = 0, residue = 0;
+        if (in) {
+            const int slot = (int)(key[s0 + t0 + lane] % NSLOT);
+            a = slot < NS0 ? 0 : slot < NS0 + NS1 ? 1 : 2;
+            const int e = slot - slot_off(a), e1 = slot_ext(a, 1), e2 = slot_ext(a, 2);
+            l0 = e / (e2 * e1), l1 = e / e2 % e1, l2 = e % e2;
+            residue = box_index(a, l0, l1, l2) % 16;
+        }
+        const unsigned alike = __match_any_sync(0xffffffffu, a * 16 + residue);
+        const int rank = __popc(alike & ((1u << lane) - 1u));
+        const int order = (a * 32 + rank) * 16 + residue;  // no two lanes' alike but those past the end
+        int at = 0;
+        for (int j = 0; j < 32; j++) at += __shfl_sync(0xffffffffu, order, j) < order;
+        if (in) code[s0 + t0 + at] = (uint16_t)part_code(lane, a, l0, l1, l2);
     }
-    const int e2 = slot_ext(a, 2), e1 = slot_ext(a, 1);
-    code[i] = (uint16_t)part_code(a, e / (e2 * e1), e / e2 % e1, e % e2);
 }
 
 }  // namespace
@@ -786,8 +819,10 @@ void bricks_build(Context& ctx, Batch& b) {
         SC_LAUNCH_CK();
     }
     K.code.alloc(n, st, ms);
-    k_part_codes<<<grid_for(n, 256), 256, 0, st>>>(n, key_s.get(), K.code.get());
-    SC_LAUNCH_CK();
+    if (nb > 0) {
+        k_part_codes<<<nb, 256, 0, st>>>(K.start.get(), key_s.get(), K.code.get());
+        SC_LAUNCH_CK();
+    }
     // each brick's halo list and the k of its neighbours' boundary cells
     K.hstart.alloc(nb1 + 1, st, ms);
     K.hk.alloc(nb1 * HK, st, ms);

@@ -33,7 +33,7 @@ struct Bricks {
     DBuf<uint8_t> geo;          // per piece: dimensions, brick grid, first cell and brick
     DBuf<uint8_t> halo;         // the entries of a brick's shared-memory box its neighbours fill
     int32_t nhalo = 0;
-    DBuf<uint16_t> code;        // per brick-ordered part: its axis and brick-local position
+    DBuf<uint16_t> code;        // per part, 32 a group in the lanes' order: its place, axis and brick-local position
     DBuf<int32_t> hstart;       // n_bricks + 1: each brick's halo list
     DBuf<uint16_t> hent;        // per halo item: the box entry it fills
     DBuf<int32_t> hsrc;         // per halo item: the brick-ordered part it comes from
