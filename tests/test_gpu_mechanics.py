@@ -55,3 +55,29 @@ def test_mech_solve_rejects_bad_pairs(solver):
     bad["pi"][0] = bad["pj"][0]  # a pair with itself
     with pytest.raises(sc.StaticsError):
         solver.mech_solve(bad)
+
+
+@pytest.mark.parametrize("n", [2, 30, 31, 32, 70])
+def test_mech_solve_long_rows(solver, n):
+    """Every node joined to every other by a spring along their line: rows of n blocks with the
+    diagonal, about and past the thirty that a warp takes at a time, against the oracle at
+    the bounds of the voxel pieces above."""
+    rng = np.random.default_rng(n)
+    sites = np.array([(i % 5, i // 5 % 5, i // 25) for i in range(n)], np.int64)
+    at = 0.125 * sites
+    diag = np.tile(np.eye(3), (n, 1, 1))
+    pi, pj = (np.ascontiguousarray(v, np.uint32) for v in np.triu_indices(n, 1))
+    d = at[pj] - at[pi]
+    d /= np.linalg.norm(d, axis=1)[:, None]
+    k = rng.uniform(0.5, 2.0, len(pi))[:, None, None] * d[:, :, None] * d[:, None, :]
+    for i, j, b in zip(pi, pj, k):
+        diag[i] += b
+        diag[j] += b
+    s = {"sites": sites, "at": at, "diag": diag, "pi": pi, "pj": pj, "pb": -k, "b": rng.standard_normal((n, 3)),
+         "h": 0.125}
+    _, r_ref, sizes, _ = M.solve(s, tol=1e-8)
+    x_tight, _, _, _ = M.solve(s, tol=1e-12)
+    x, rounds, levels = solver.mech_solve(s, tol=1e-8)
+    assert levels == len(sizes)
+    assert abs(rounds - r_ref) <= 2
+    assert np.linalg.norm(x - x_tight) <= 1e-7 * np.linalg.norm(x_tight)

@@ -445,3 +445,44 @@ def test_dense_tops_of_all_sizes(solver, shape, few):
     assert info["status"] == sc.OK
     # one exact preconditioner: the motions agree to the top's rounding, kappa(K) eps < 1e-9
     assert rel(u, u_ref) < 1e-9
+
+
+@pytest.mark.parametrize("shape", [(16, 40, 48), (20, 48, 48)], ids=["fewer bricks than SMs", "more"])
+def test_brick_stencil_by_brick_count(solver, shape):
+    """The stencil's two block shapes (4 x 5 x 6 = 120 bricks take 512 threads each, 5 x 6 x 6 =
+    180 take 256), against the oracle's operator at the bounds of the shapes above."""
+    st, k = piece(0, 3, shape=shape)
+    lat = oracle_lattice(st, k)
+    _, parts = sc.grid_count(st)
+    x = np.random.default_rng(3).standard_normal((parts, 6))
+    want = lat.level0_apply(x)
+    got = solver.grid_apply(st, k, x, sc.FP64)
+    assert rel(got, want) < OP_TOL64
+    assert np.abs(got - want).max() <= 1e-12 * np.abs(want).max()
+    assert rel(solver.grid_apply(st, k, x, sc.MIXED), want) < OP_TOL32
+
+
+@pytest.mark.parametrize("precision", [sc.FP64, sc.MIXED])
+def test_reductions_with_empty_and_tiny_pieces(solver, precision):
+    """The reductions' chunks of 4096 parts: a piece with no part at all, one of a single free
+    cell, one just over a chunk, one of two and one of seven, in one batch, each against the
+    oracle."""
+    shapes = [(1, 1, 2), (10, 12, 12), (12, 12, 12), (24, 20, 20)]
+    pieces = []
+    for i, shape in enumerate(shapes):
+        st = np.ones(shape, np.uint8)
+        st[:, :, 0] = 2
+        pieces.append((st, np.random.default_rng(i).uniform(0.5, 2.0, shape).astype(np.float32)))
+    empty = np.zeros((3, 3, 3), np.uint8)
+    empty[:, :, 0] = 2
+    pieces.insert(2, (empty, np.zeros(empty.shape, np.float32)))
+    outs, infos = solver.solve_grid_batch(pieces, sc.options(max_iter=5000, tol=1e-8, precision=precision))
+    for (st, k), u, info in zip(pieces, outs, infos):
+        if not (st == 1).any():
+            assert u.size == 0 and info["iterations"] == 0
+            continue
+        lat = oracle_lattice(st, k)
+        loads, _ = z_loads(lat)
+        u_ref, _ = lat.motions(loads, tol=1e-12)
+        assert info["status"] == sc.OK and info["residual"] <= 1e-8 * 1.0001
+        assert rel(u, u_ref) < DISP_TOL
