@@ -528,18 +528,32 @@ __global__ void __launch_bounds__(TH, brick_min_blocks<T, MODE, TH>()) k_brick_s
     T* box = reinterpret_cast<T*>(brick_sm);
     float* kbox = reinterpret_cast<float*>(box + 6 * NBOX);
     uint16_t* codes = reinterpret_cast<uint16_t*>(kbox + KB);
-    const int b = blockIdx.x;
-    const int4 inf = v.info[b];
-    if (done && done[inf.x]) return;
-    const int32_t start = v.start[b], cnt = v.start[b + 1] - start;
-    if (cnt == 0) return;                            // only cells: nothing of its own to write
-    if (skip_row && skip_row[start]) return;         // the piece is solved at level 0
+    const int b = blockIdx.x, t = threadIdx.x;
+    // Two trips to memory before the copies, not a trip a line: what hangs on the brick alone,
+    // then what hangs on that (the mixed 128^3 solve 385.2 to 382.6 ms, FP64 519.0 to 516.4).
+    const int4 inf = __ldg(v.info + b);
+    const int32_t start = __ldg(v.start + b), cnt = __ldg(v.start + b + 1) - start;
+    const int32_t h0 = __ldg(v.hstart + b), nh = __ldg(v.hstart + b + 1) - h0;
+    if (cnt == 0) return;  // only cells: nothing of its own to write
+    const bool off = done && done[inf.x];
+    const bool top = skip_row && skip_row[start];  // the piece is solved at level 0
     const T w = step ? (T)step[inf.x] : T(0);
+    uint32_t c[2], he[2];
+    int32_t hs[2];
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+        c[j] = t + TH * j < cnt ? __ldg(v.code + start + t + TH * j) : 0;
+        he[j] = t + TH * j < nh ? __ldg(v.hent + h0 + t + TH * j) : 0;
+        hs[j] = t + TH * j < nh ? __ldg(v.hsrc + h0 + t + TH * j) : 0;
+    }
+    const float kd = t < BCELLS ? __ldg(v.kd + (int64_t)b * BCELLS + t) : 0.0f;
+    const float hk = t < HK ? __ldg(v.hk + (int64_t)b * HK + t) : 0.0f;
+    if (off || top) return;
     // the box starts at zero: faces that are no part stay so
     {
         constexpr int N16 = (int)(sizeof(T) * 6 * NBOX / 16);
         float4* z = reinterpret_cast<float4*>(box);
-        for (int i = threadIdx.x; i < N16; i += TH) z[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int i = t; i < N16; i += TH) z[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
     __syncthreads();
     // The box is filled by asynchronous copies (cp.async: global memory straight to shared
@@ -547,31 +561,30 @@ __global__ void __launch_bounds__(TH, brick_min_blocks<T, MODE, TH>()) k_brick_s
     // parts, a warp a group of 32 of its run, each to its face's entry (by its part_code, kept
     // for the part phase), and the halo parts of its resolved list (bricks_build).
     const bool vec16 = sizeof(T) == 8 && ((reinterpret_cast<uintptr_t>(x) & 15) == 0);
-    for (int t = threadIdx.x; t < cnt; t += TH) {
-        const uint32_t c = __ldg(v.code + start + t);
-        codes[t] = (uint16_t)c;
-        copy_part<T>(box + 6 * own_entry(c), x + 6 * ((int64_t)start + (t & ~31) + (int)(c >> 11)), vec16);
+    auto own = [&](int i, uint32_t ci) {
+        codes[i] = (uint16_t)ci;
+        copy_part<T>(box + 6 * own_entry(ci), x + 6 * ((int64_t)start + (i & ~31) + (int)(ci >> 11)), vec16);
+    };
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+        if (t + TH * j < cnt) own(t + TH * j, c[j]);
+        if (t + TH * j < nh) copy_part<T>(box + 6 * (int)he[j], x + 6 * (int64_t)hs[j], vec16);
     }
-    {
-        const int32_t h0 = __ldg(v.hstart + b), h1 = __ldg(v.hstart + b + 1);
-        for (int32_t h = h0 + threadIdx.x; h < h1; h += TH)
-            copy_part<T>(box + 6 * (int)__ldg(v.hent + h), x + 6 * (int64_t)__ldg(v.hsrc + h), vec16);
-    }
+    for (int i = t + 2 * TH; i < cnt; i += TH) own(i, __ldg(v.code + start + i));
+    for (int i = t + 2 * TH; i < nh; i += TH)
+        copy_part<T>(box + 6 * (int)__ldg(v.hent + h0 + i), x + 6 * (int64_t)__ldg(v.hsrc + h0 + i), vec16);
     // k of the brick's cells and of the single layers before it (-x, -y, -z)
-    {
-        const int t = threadIdx.x;
-        if (t < BCELLS) kbox[kbox_index(t / (BY * BZ), t / BZ % BY, t % BZ)] = __ldg(v.kd + (int64_t)b * BCELLS + t);
-        if (t < HK) {
-            int h0, h1, h2;
-            if (t < HKX) {
-                h0 = -1, h1 = t / BZ, h2 = t % BZ;
-            } else if (t < HKX + HKY) {
-                h0 = (t - HKX) / BZ, h1 = -1, h2 = (t - HKX) % BZ;
-            } else {
-                h0 = (t - HKX - HKY) / BY, h1 = (t - HKX - HKY) % BY, h2 = -1;
-            }
-            kbox[kbox_index(h0, h1, h2)] = __ldg(v.hk + (int64_t)b * HK + t);
+    if (t < BCELLS) kbox[kbox_index(t / (BY * BZ), t / BZ % BY, t % BZ)] = kd;
+    if (t < HK) {
+        int i0, i1, i2;
+        if (t < HKX) {
+            i0 = -1, i1 = t / BZ, i2 = t % BZ;
+        } else if (t < HKX + HKY) {
+            i0 = (t - HKX) / BZ, i1 = -1, i2 = (t - HKX) % BZ;
+        } else {
+            i0 = (t - HKX - HKY) / BY, i1 = (t - HKX - HKY) % BY, i2 = -1;
         }
+        kbox[kbox_index(i0, i1, i2)] = hk;
     }
     cp_async_wait_all();
     __syncthreads();
@@ -579,10 +592,10 @@ __global__ void __launch_bounds__(TH, brick_min_blocks<T, MODE, TH>()) k_brick_s
     const T* rb = r ? r + 6 * (int64_t)start : nullptr;
     T* yb = y + 6 * (int64_t)start;
     T* y2b = y2 ? y2 + 6 * (int64_t)start : nullptr;
-    for (int t = threadIdx.x; t < cnt; t += TH) {
-        const uint32_t c = codes[t];
-        const PartAt p = part_at(c);
-        const int q = (t & ~31) + (int)(c >> 11);
+    for (int i = t; i < cnt; i += TH) {
+        const uint32_t ci = codes[i];
+        const PartAt p = part_at(ci);
+        const int q = (i & ~31) + (int)(ci >> 11);
         if (p.a == 0)
             brick_part<0, T, MODE>(box, kbox, p.l0, p.l1, p.l2, q, rb, yb, y2b, s, w);
         else if (p.a == 1)
