@@ -248,7 +248,11 @@ __global__ void k_cg_check(int np, int64_t max_iter, CgScalars s, int32_t* ndone
 }
 
 // The vector passes of an iteration. Each is bound by HBM on a large piece and by its own
-// lanes' chains on a small one (see Chunks); the sums' order does not depend on which.
+// lanes' chains on a small one (see Chunks); the sums' order does not depend on which. x is
+// advanced with p, which both need then, and not with r: at 128^3 172 + 58 us become 87 + 111.
+// A piece that this iteration finishes still has that to come, so its done is LAST until the next
+// iteration's k_dot_alpha (every other reader takes any value but zero as done).
+constexpr int32_t DONE = 1, LAST = 2;
 
 // (p, Ap) and from it alpha = rz / (p, Ap) (bodies.rs:355-356)
 template <bool SPLIT>
@@ -256,7 +260,10 @@ __global__ void __launch_bounds__(RED_LANES) k_dot_alpha(Chunks ch, CgScalars s,
                                                          const double* __restrict__ ap) {
     extern __shared__ double sm[];
     const int c = red_chunk<SPLIT>(), t = red_lane<SPLIT>(), pc = ch.piece[c];
-    if (s.done[pc]) return;
+    if (s.done[pc]) {
+        if (t == 0 && c == ch.piece_chunk[pc]) s.done[pc] = DONE;
+        return;
+    }
     double pap = 0.0, none = 0.0;
     if (!red_run<SPLIT, 2, 8>(
             sm, 6 * ch.lo[c] + t, 6 * ch.lo[c + 1], [&](int64_t i, double (&v)[2]) { v[0] = p[i], v[1] = ap[i]; },
@@ -273,20 +280,18 @@ __global__ void __launch_bounds__(RED_LANES) k_dot_alpha(Chunks ch, CgScalars s,
     s.alpha[pc] = s.rz[pc] / pap;
 }
 
-// x += alpha p; r -= alpha Ap (bodies.rs:357-362), the FP32 V-cycle's input r32 in the same
-// pass (where given), and (r, r)
+// r -= alpha Ap (bodies.rs:357-362), the FP32 V-cycle's input r32 in the same pass (where
+// given), and (r, r)
 template <bool SPLIT>
-__global__ void __launch_bounds__(RED_LANES) k_update_xr(Chunks ch, CgScalars s, double* __restrict__ x,
-                                                         const double* __restrict__ p, double* __restrict__ r,
-                                                         const double* __restrict__ ap, float* __restrict__ r32) {
+__global__ void __launch_bounds__(RED_LANES) k_update_r(Chunks ch, CgScalars s, double* __restrict__ r,
+                                                        const double* __restrict__ ap, float* __restrict__ r32) {
     extern __shared__ double sm[];
     const int c = red_chunk<SPLIT>(), t = red_lane<SPLIT>(), pc = ch.piece[c];
     if (s.done[pc]) return;
     const double a = s.alpha[pc];
     const int64_t first = 6 * ch.lo[c] + t, end = 6 * ch.lo[c + 1];
     double rr = 0.0, none = 0.0;
-    auto update = [&](int64_t i, double xv, double pv, double rv, double av) {
-        x[i] = xv + a * pv;
+    auto update = [&](int64_t i, double rv, double av) {
         const double rn = rv - a * av;
         r[i] = rn;
         if (r32) r32[i] = (float)rn;
@@ -296,16 +301,16 @@ __global__ void __launch_bounds__(RED_LANES) k_update_xr(Chunks ch, CgScalars s,
         // eight warps update; the first sums what they leave in shared memory
         constexpr int PER = RED_STEPS / 8;
         const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-        double4 v[PER];
+        double2 v[PER];
 #pragma unroll
         for (int u = 0; u < PER; u++) {
             const int64_t i = first + RED_LANES * (int64_t)(w + 8 * u);
-            if (i < end) v[u] = make_double4(x[i], p[i], r[i], ap[i]);
+            if (i < end) v[u] = make_double2(r[i], ap[i]);
         }
 #pragma unroll
         for (int u = 0; u < PER; u++) {
             const int64_t i = first + RED_LANES * (int64_t)(w + 8 * u);
-            if (i < end) sm[(w + 8 * u) * 32 + l] = update(i, v[u].x, v[u].y, v[u].z, v[u].w);
+            if (i < end) sm[(w + 8 * u) * 32 + l] = update(i, v[u].x, v[u].y);
         }
         __syncthreads();
         if (w != 0) return;
@@ -316,10 +321,10 @@ __global__ void __launch_bounds__(RED_LANES) k_update_xr(Chunks ch, CgScalars s,
             rr = fma(rn, rn, rr);
         }
     } else {
-        red_chain<6>(
-            first, end, [&](int64_t i) { return make_double4(x[i], p[i], r[i], ap[i]); },
-            [&](int64_t i, const double4& v) {
-                const double rn = update(i, v.x, v.y, v.z, v.w);
+        red_chain<8>(
+            first, end, [&](int64_t i) { return make_double2(r[i], ap[i]); },
+            [&](int64_t i, const double2& v) {
+                const double rn = update(i, v.x, v.y);
                 rr = fma(rn, rn, rr);
             });
     }
@@ -363,18 +368,18 @@ __global__ void __launch_bounds__(RED_LANES) k_dots_beta(Chunks ch, CgScalars s,
     else if (s.iters[pc] >= max_iter)
         status = (int)SC_MAXITER;
     if (status < 0) return;
-    s.done[pc] = 1;
+    s.done[pc] = LAST;
     atomicMax(s.status + pc, status);
     atomicAdd(s.ndone, 1);
 }
 
-// p = z + beta p (bodies.rs:365-369), eight blocks a chunk. On a device-side loop (count not
+// x += alpha p, p = z + beta p (bodies.rs:357-369), eight blocks a chunk. On a device-side loop (count not
 // null) it also sets the loop's condition: go on while a piece is not done and fewer than
 // `chunk` iterations ran since the launch (count is zeroed before each launch; any value it
 // holds ends the loop within chunk + 1 iterations).
 template <class Z>
-__global__ void __launch_bounds__(256) k_update_p(Chunks ch, CgScalars s, double* __restrict__ p,
-                                                  const Z* __restrict__ z, cudaGraphConditionalHandle h, int np,
+__global__ void __launch_bounds__(256) k_update_xp(Chunks ch, CgScalars s, double* __restrict__ x,
+                                                   double* __restrict__ p, const Z* __restrict__ z, cudaGraphConditionalHandle h, int np,
                                                   uint32_t* __restrict__ count, uint32_t chunk) {
     if (count && blockIdx.x == 0 && threadIdx.x == 0) {
         const uint32_t n = *count + 1u;
@@ -382,17 +387,23 @@ __global__ void __launch_bounds__(256) k_update_p(Chunks ch, CgScalars s, double
         cudaGraphSetConditional(h, (*s.ndone < np && n < chunk) ? 1u : 0u);
     }
     const int c = blockIdx.x >> 3, pc = ch.piece[c];
-    if (s.done[pc]) return;
-    const double bt = s.beta[pc];
+    if (s.done[pc] == DONE) return;
+    const double a = s.alpha[pc], bt = s.beta[pc];
     const int64_t lo = 3 * ch.lo[c] + (blockIdx.x & 7) * (3 * CHUNK / 8);  // in pairs of values
     const int64_t end = 3 * ch.lo[c + 1], hi = lo + 3 * CHUNK / 8 < end ? lo + 3 * CHUNK / 8 : end;
-    double2* p2 = reinterpret_cast<double2*>(p);
+    double2 *p2 = reinterpret_cast<double2*>(p), *x2 = reinterpret_cast<double2*>(x);
     using Z2 = std::conditional_t<sizeof(Z) == 8, double2, float2>;
     const Z2* z2 = reinterpret_cast<const Z2*>(z);
+    struct Three {
+        double2 x, p;
+        Z2 z;
+    };
     red_chain<3>(
-        lo + threadIdx.x, hi,
-        [&](int64_t i) { return make_double4((double)z2[i].x, (double)z2[i].y, p2[i].x, p2[i].y); },
-        [&](int64_t i, const double4& v) { p2[i] = make_double2(v.x + bt * v.z, v.y + bt * v.w); });
+        lo + threadIdx.x, hi, [&](int64_t i) { return Three{x2[i], p2[i], z2[i]}; },
+        [&](int64_t i, const Three& v) {
+            x2[i] = make_double2(v.x.x + a * v.p.x, v.x.y + a * v.p.y);
+            p2[i] = make_double2((double)v.z.x + bt * v.p.x, (double)v.z.y + bt * v.p.y);
+        });
 }
 
 // the two scalar steps on their own, for the all-FP32 conjugate gradients (pcg_mixed)
@@ -768,7 +779,7 @@ static int64_t pcg(Context& ctx, Batch& b, const V* rhs, S* x, V* r, V* z, V* p,
             constexpr bool SPLIT = decltype(split)::value;
             k_dot_alpha<SPLIT><<<grid, RED_LANES, red_smem<SPLIT>(2), st>>>(ch, cg.s, p, ap);
             SC_LAUNCH_CK();
-            k_update_xr<SPLIT><<<grid, RED_LANES, red_smem<SPLIT>(1), st>>>(ch, cg.s, x, p, r, ap, r32);
+            k_update_r<SPLIT><<<grid, RED_LANES, red_smem<SPLIT>(1), st>>>(ch, cg.s, r, ap, r32);
             SC_LAUNCH_CK();
             precondition();
             launch_dots<P, !same, SPLIT>(grid, st, ch, cg.s, max_iter, r, ap, zs);
@@ -778,8 +789,8 @@ static int64_t pcg(Context& ctx, Batch& b, const V* rhs, S* x, V* r, V* z, V* p,
             passes(std::true_type{});
         else
             passes(std::false_type{});
-        k_update_p<P><<<(unsigned)(8 * L.nchunks), 256, 0, st>>>(ch, cg.s, p, zs, ctx.loop_handle, np,
-                                                                 device_loop ? cg.loop_count.get() : nullptr, chunk);
+        k_update_xp<P><<<(unsigned)(8 * L.nchunks), 256, 0, st>>>(ch, cg.s, x, p, zs, ctx.loop_handle, np,
+                                                                  device_loop ? cg.loop_count.get() : nullptr, chunk);
         SC_LAUNCH_CK();
     };
     // Residual replacement: r = b - K x in FP64 for the pieces whose true residual misses
