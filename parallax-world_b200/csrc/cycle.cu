@@ -249,7 +249,7 @@ __global__ void k_cg_check(int np, int64_t max_iter, CgScalars s, int32_t* ndone
 
 // The vector passes of an iteration. Each is bound by HBM on a large piece and by its own
 // lanes' chains on a small one (see Chunks); the sums' order does not depend on which. x is
-// advanced with p, which both need then, and not with r: at 128^3 172 + 58 us become 87 + 111.
+// advanced with p, which both need then, and not with r: at 128^3 172 + 58 us became 105 + 106.
 // A piece that this iteration finishes still has that to come, so its done is LAST until the next
 // iteration's k_dot_alpha (every other reader takes any value but zero as done).
 constexpr int32_t DONE = 1, LAST = 2;
