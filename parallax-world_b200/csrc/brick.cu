@@ -955,18 +955,11 @@ void brick_stencil(Context& ctx, const Batch& b, const T* x, const T* r, T* y, T
     if (K.n_bricks <= 0) return;
     constexpr size_t smem = brick_smem<T>();
     auto go = [&](auto kernel, int threads) {
+        ctx.shared_most(kernel, smem);
         kernel<<<(unsigned)K.n_bricks, threads, smem, ctx.stream>>>(view_of(K), x, r, y, y2, (T)b.grid.s, step, skip_row,
                                                                    done);
         SC_LAUNCH_CK();
     };
-    static const bool attr_set = [] {  // once per instantiation (thread-safe)
-        SC_CK(cudaFuncSetAttribute(k_brick_stencil<T, MODE, BRICK_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)smem));
-        SC_CK(cudaFuncSetAttribute(k_brick_stencil<T, MODE, BRICK_THREADS_FEW>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        return true;
-    }();
-    (void)attr_set;
     if (K.n_bricks <= BRICK_FEW)
         go(k_brick_stencil<T, MODE, BRICK_THREADS_FEW>, BRICK_THREADS_FEW);
     else

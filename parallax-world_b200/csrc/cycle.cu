@@ -695,16 +695,11 @@ static void residual_floor(Context& ctx, Batch& b, const double* x, double* ff) 
 }
 
 template <class Z, bool FLEX, bool SPLIT>
-static void launch_dots(unsigned grid, cudaStream_t st, const Chunks& ch, const CgScalars& s, int64_t max_iter,
+static void launch_dots(Context& ctx, unsigned grid, const Chunks& ch, const CgScalars& s, int64_t max_iter,
                         const double* r, const double* ap, const Z* z) {
     constexpr size_t smem = red_smem<SPLIT>(FLEX ? 3 : 2);
-    static const bool attr_set = [] {  // once per instantiation (thread-safe)
-        SC_CK(cudaFuncSetAttribute(k_dots_beta<Z, FLEX, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)smem));
-        return true;
-    }();
-    (void)attr_set;
-    k_dots_beta<Z, FLEX, SPLIT><<<grid, RED_LANES, smem, st>>>(ch, s, max_iter, r, ap, z);
+    ctx.shared_most(k_dots_beta<Z, FLEX, SPLIT>, smem);
+    k_dots_beta<Z, FLEX, SPLIT><<<grid, RED_LANES, smem, ctx.stream>>>(ch, s, max_iter, r, ap, z);
 }
 
 // Times a solve may replace the residuals of pieces whose true residual missed the goal.
@@ -782,7 +777,7 @@ static int64_t pcg(Context& ctx, Batch& b, const V* rhs, S* x, V* r, V* z, V* p,
             k_update_r<SPLIT><<<grid, RED_LANES, red_smem<SPLIT>(1), st>>>(ch, cg.s, r, ap, r32);
             SC_LAUNCH_CK();
             precondition();
-            launch_dots<P, !same, SPLIT>(grid, st, ch, cg.s, max_iter, r, ap, zs);
+            launch_dots<P, !same, SPLIT>(ctx, grid, ch, cg.s, max_iter, r, ap, zs);
             SC_LAUNCH_CK();
         };
         if (red_split(L.nchunks))

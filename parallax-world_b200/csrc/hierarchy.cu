@@ -1788,12 +1788,7 @@ static void build_top(Context& ctx, Batch& b, int l, const std::vector<int32_t>&
         SC_LAUNCH_CK();
         return;
     }
-    static const bool attr_set = [] {  // once (thread-safe)
-        SC_CK(cudaFuncSetAttribute(k_top_factor, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)top_smem(TOP_MOST)));
-        return true;
-    }();
-    (void)attr_set;
+    ctx.shared_most(k_top_factor, top_smem(TOP_MOST));
     const size_t smem = std::max(top_smem(most), (size_t)32 * 34 * sizeof(double));
     k_top_factor<<<nt, TOP_THREADS, smem, st>>>(L.top.get(), L.pstart_d.get(), L.kinv_off.get(), L.kinv.get(), X.get(),
                                                 b.status_d.get());

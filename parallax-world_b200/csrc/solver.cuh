@@ -12,6 +12,7 @@
 
 #include <chrono>
 #include <memory>
+#include <set>
 #include <vector>
 
 #include "common.cuh"
@@ -300,7 +301,17 @@ struct Context {
     std::unique_ptr<Batch> last;     // the last solve's hierarchy (parity queries)
     int32_t* pinned = nullptr;       // 16 bytes of pinned host memory for small reads
     cudaGraphConditionalHandle loop_handle = 0;  // the device-side CG loop's condition
+    std::set<const void*> raised;    // kernels whose shared-memory limit this context has raised
     void* cub_scratch(size_t bytes);
+    // Before a launch with dynamic shared memory: raises the kernel's limit to `most`, its
+    // largest ever. The runtime keeps the limit a device, so each context raises it once.
+    template <class K>
+    void shared_most(K* kernel, size_t most) {
+        const void* f = reinterpret_cast<const void*>(kernel);
+        if (raised.count(f)) return;
+        SC_CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+        raised.insert(f);
+    }
     int32_t* pinned_i32();
     ~Context();
 };
