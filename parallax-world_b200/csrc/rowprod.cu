@@ -380,6 +380,8 @@ __global__ void k_upper_windows(int64_t nc, const int32_t* __restrict__ cpiece, 
     hi[c] = (int32_t)cpstart[cpiece[c] + 1];
 }
 
+constexpr int ROWS_SLOTS = 256;  // a tile's output blocks: 72 KB
+
 // staged A entries: first B entry and value block (8 bytes each), count and prefix
 size_t meta_bytes(int meta) { return (size_t)meta * 2 * sizeof(int64_t) + (size_t)(2 * meta + 2) * sizeof(int); }
 
@@ -387,9 +389,12 @@ template <int MODE, int TH, bool AREG>
 void launch_fill_th(Context& ctx, int64_t nrows, const RowArgs& a, const int64_t* first, const int64_t* crow,
                     int32_t* ccol, double* cval, int S, int ntiles, int nwmax, int meta) {
     meta = std::min(meta, 2 * TH);
-    size_t smem = (size_t)S * 36 * sizeof(double) + (MODE == ROWS_K0 ? 36 * 36 * sizeof(double) : 0) +
-                  72 * sizeof(double) + meta_bytes(meta) + 2 * (size_t)nwmax * sizeof(uint32_t);
-    SC_CK(cudaFuncSetAttribute(k_rows_fill<MODE, TH, AREG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    auto bytes = [](int slots, int staged, int words) {
+        return (size_t)slots * 36 * sizeof(double) + (MODE == ROWS_K0 ? 36 * 36 * sizeof(double) : 0) +
+               72 * sizeof(double) + meta_bytes(staged) + 2 * (size_t)words * sizeof(uint32_t);
+    };
+    const size_t smem = bytes(S, meta, nwmax);
+    ctx.shared_most(k_rows_fill<MODE, TH, AREG>, bytes(ROWS_SLOTS, 2 * TH, (int)(ROWS_MAX_WIDTH / 32)));
     k_rows_fill<MODE, TH, AREG><<<dim3((unsigned)nrows, (unsigned)ntiles), TH, smem, ctx.stream>>>(
         nrows, a, first, crow, ccol, cval, S, nwmax, meta);
     SC_LAUNCH_CK();
@@ -460,10 +465,10 @@ void row_products(Context& ctx, int mode, const RowArgs& a, int64_t nrows, int64
     ccol.alloc(std::max<int64_t>(cnnz, 1), st, ms);
     cval.alloc(36 * std::max<int64_t>(cnnz, 1), st, ms);
     if (cnnz == 0) return;
-    // slots summed by one block: the widest row, at most 256 blocks (72 KB); wider rows
+    // slots summed by one block: the widest row, at most ROWS_SLOTS blocks; wider rows
     // go in several tiles, one block each. SC_ROWS_SLOTS and SC_ROWS_META shrink the
     // tiles and the staged entries (to test the tiling).
-    int cap = 256, meta = RP_META;
+    int cap = ROWS_SLOTS, meta = RP_META;
     if (const char* v = std::getenv("SC_ROWS_SLOTS")) cap = std::max(1, std::min(cap, std::atoi(v)));
     if (const char* v = std::getenv("SC_ROWS_META")) meta = std::max(1, std::min(meta, std::atoi(v)));
     const int S = (int)std::min<int64_t>(cap, (h[1] + 7) / 8 * 8);

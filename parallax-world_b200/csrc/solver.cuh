@@ -304,7 +304,8 @@ struct Context {
     std::set<const void*> raised;    // kernels whose shared-memory limit this context has raised
     void* cub_scratch(size_t bytes);
     // Before a launch with dynamic shared memory: raises the kernel's limit to `most`, its
-    // largest ever. The runtime keeps the limit a device, so each context raises it once.
+    // largest ever. The runtime keeps the limit a device, so each context raises it once,
+    // and never to what a launch needs, which could take it from another thread's launch.
     template <class K>
     void shared_most(K* kernel, size_t most) {
         const void* f = reinterpret_cast<const void*>(kernel);

@@ -5,7 +5,6 @@ import subprocess
 import sys
 import textwrap
 
-import numpy as np
 import pytest
 
 import statics_cuda as sc
@@ -59,3 +58,53 @@ def test_a_new_device_context_solves_as_the_first(name, precision):
     ended, which one device is enough to check: the same call in a fresh solver, the same
     bits."""
     run_script(TWICE, name, str(precision))
+
+
+SHIM = r"""
+#include <dlfcn.h>
+#include <stdio.h>
+static struct { const void* f; int most; } seen[4096];
+static int n;
+int cudaFuncSetAttribute(const void* f, int attr, int value) {
+    static int (*next)(const void*, int, int);
+    if (!next)  /* the runtime's own: it is loaded already, in the library's scope */
+        next = (int (*)(const void*, int, int))dlsym(dlopen("libcudart.so.12", RTLD_NOW | RTLD_NOLOAD),
+                                                     "cudaFuncSetAttribute");
+    if (!next) return 999;
+    if (attr == 8) {  /* cudaFuncAttributeMaxDynamicSharedMemorySize */
+        int i = 0;
+        while (i < n && seen[i].f != f) i++;
+        if (i == n && n < 4096) seen[n++].f = f;
+        if (i < n) {
+            if (value < seen[i].most) {
+                fprintf(stderr, "limit lowered from %d to %d\n", seen[i].most, value);
+                return 1;  /* cudaErrorInvalidValue */
+            }
+            seen[i].most = value;
+        }
+    }
+    return next(f, attr, value);
+}
+"""
+
+BOTH = """
+    import statics_cuda as sc
+    from helpers import piece
+
+    opt = sc.options(max_iter=5000, tol=1e-8)
+    for shape in ((31, 29, 37), (9, 8, 7), (24, 24, 24), (12, 20, 9)):
+        solver = sc.Solver(0)
+        _, info = solver.solve_grid(*piece(0, 3, shape=shape), opt)
+        assert info["status"] == sc.OK
+        solver.close()
+"""
+
+
+def test_no_limit_is_ever_lowered(tmp_path):
+    """A kernel's limit is the device's, so every thread's: lowered to what one launch needs, it
+    fails another thread's launch that needs more and was about to run. Here the call that
+    sets it is stood in for, and refuses to lower one: large and small pieces in turn solve."""
+    (tmp_path / "shim.c").write_text(SHIM)
+    shim = str(tmp_path / "shim.so")
+    subprocess.run(["gcc", "-shared", "-fPIC", "-O1", "-o", shim, str(tmp_path / "shim.c"), "-ldl"], check=True)
+    run_script(BOTH, env={"LD_PRELOAD": shim})
