@@ -113,7 +113,7 @@ static double transfer_bytes(const Level& L, const Level& C) {
 // back and smooth again. Above level 0 the first smoothing, x = step D^-1 r, is done already:
 // by the restriction that made r. On small levels each kernel is a chain of dependent loads,
 // so a single piece's kernels look up no row's piece, and a level without tops none of its
-// rows' flags (done is null for a single piece: the iterations stop with it).
+// rows' flags (done is null for a single piece in the device-side loop, which stops with it).
 template <class T>
 static void cycle(Context& ctx, Batch& b, int l, const T* r, T* z, const int32_t* done) {
     Level& L = b.levels[l];
@@ -724,13 +724,15 @@ static int64_t pcg(Context& ctx, Batch& b, const V* rhs, S* x, V* r, V* z, V* p,
     // direction update read directly (no FP64 copy of z is made); rp, the cycle's input,
     // is written by the residual update itself.
     const P* zs = same ? reinterpret_cast<const P*>(z) : zp;
-    // one piece's kernels need no look at its done flag: the loop ends with it
-    const int32_t* done = np == 1 ? nullptr : cg.s.done;
+    // The device-side loop ends with a single piece, whose kernels then need no look at its
+    // done flag; a loop driven from the host runs on to its next look.
+    bool device_loop = false;
+    auto done = [&]() -> const int32_t* { return np == 1 && device_loop ? nullptr : cg.s.done; };
     auto precondition = [&]() {
         if constexpr (same)
-            cycle<V>(ctx, b, 0, r, z, done);
+            cycle<V>(ctx, b, 0, r, z, done());
         else
-            cycle<P>(ctx, b, 0, rp, zp, done);
+            cycle<P>(ctx, b, 0, rp, zp, done());
     };
     SC_CK(cudaMemsetAsync(x, 0, n6 * sizeof(S), st));
     SC_CK(cudaMemcpyAsync(r, rhs, n6 * sizeof(V), cudaMemcpyDeviceToDevice, st));
@@ -758,14 +760,13 @@ static int64_t pcg(Context& ctx, Batch& b, const V* rhs, S* x, V* r, V* z, V* p,
     // iterations one launch of the device-side loop runs at most between looks at the done
     // count (and at the time limit)
     const uint32_t chunk = 32;
-    bool device_loop = false;
     auto body = [&]() {
         if (L.matrix_free) {
-            stencil_apply<V>(ctx, b, p, ap, nullptr, done);
+            stencil_apply<V>(ctx, b, p, ap, nullptr, done());
         } else {
             ProfScope ps(ctx, fam_of<V>(SC_FAM_SPMV64), spmv_bytes<V>(L, 2));
             spmv<V>(ctx, SPMV_Y, L.n, L.rowptr.get(), L.col.get(), VAL<V>(L), p, nullptr, ap, nullptr, nullptr,
-                    np == 1 ? nullptr : L.piece.get(), nullptr, done, L.nnzb);
+                    np == 1 ? nullptr : L.piece.get(), nullptr, done(), L.nnzb);
         }
         if (L.nchunks <= 0) return;  // no parts: every piece is done
         const unsigned grid = red_grid(L.nchunks);

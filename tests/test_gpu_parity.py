@@ -486,3 +486,22 @@ def test_reductions_with_empty_and_tiny_pieces(solver, precision):
         u_ref, _ = lat.motions(loads, tol=1e-12)
         assert info["status"] == sc.OK and info["residual"] <= 1e-8 * 1.0001
         assert rel(u, u_ref) < DISP_TOL
+
+
+def test_finished_piece_costs_nothing_more(solver):
+    """A solve driven from the host (here: its kernels are being timed) looks at the done count
+    every four iterations. A piece stopped after the first of them must not go through the
+    other three in full: the same launches as for four iterations, in well under their time
+    (two preconditioner applications in full instead of five, the rest returning at once)."""
+    st, k = piece(96, 1)
+    ms = {}
+    for iterations in (1, 4, 1, 4):  # the first two warm up
+        solver.profile(1 << sc.FAM_STENCIL32)
+        try:
+            _, info = solver.solve_grid(st, k, sc.options(max_iter=iterations, tol=1e-8, precision=sc.MIXED))
+            ms[iterations] = solver.profile_read()["stencil32"]
+        finally:
+            solver.profile(0)
+        assert info["status"] == sc.MAXITER and info["iterations"] == iterations
+    assert ms[1]["launches"] == ms[4]["launches"] > 0
+    assert ms[1]["ms"] < 0.75 * ms[4]["ms"]
