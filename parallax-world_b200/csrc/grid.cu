@@ -990,8 +990,9 @@ void level0_down(Context& ctx, const Batch& b, const T* r, T* x, T* left, T* t, 
     launch_stencil<T, ST_RES_JAC>(ctx, b, x, r, left, t, nullptr, skip, done, 4);
     launch_stencil<T, ST_RES_W>(ctx, b, t, left, u, nullptr, L.step.get(), skip, done, 3);
     {
+        const double jac = xc ? (double)sizeof(T) * 42.0 * (double)C.n : 0.0;  // the next level's smoothing
         ProfScope ps(ctx, sizeof(T) == 8 ? SC_FAM_TRANSFER64 : SC_FAM_TRANSFER32, vb + (double)sizeof(T) * 3 * L.n +
-                     (double)sizeof(T) * 6 * C.n);
+                     (double)sizeof(T) * 6 * C.n + jac);
         const T* rv = sizeof(T) == 8 ? (const T*)L.mf_r.get() : (const T*)L.mf_r32.get();
         k_p0t<T><<<grid_for(C.n, 128), 128, 0, ctx.stream>>>(C.n, L.mem_off.get(), L.mem.get(), rv, u, rc,
                                                              b.npieces == 1 ? nullptr : C.piece.get(), done,

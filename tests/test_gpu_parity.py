@@ -505,3 +505,29 @@ def test_finished_piece_costs_nothing_more(solver):
         assert info["status"] == sc.MAXITER and info["iterations"] == iterations
     assert ms[1]["launches"] == ms[4]["launches"] > 0
     assert ms[1]["ms"] < 0.75 * ms[4]["ms"]
+
+
+def test_transfer_bytes_of_a_three_level_piece(solver):
+    """The transfer family's bytes where level 0 is matrix-free. With s bytes a value, n parts at
+    level 0, c and t at the two above and q blocks in level 1's P, a V-cycle's four transfers
+    need: P0' and with it level 1's first smoothing s (9 n + 6 c + 42 c), P0 s (9 n + 6 c) + 4 n,
+    P' s (36 q + 6 c + 6 t), P s (36 q + 12 c + 6 t). q is a whole number of at least a block a
+    row, the same in both precisions."""
+    st, k = piece(0, 3, shape=(15, 14, 13))
+    blocks = []
+    for precision, name in ((sc.FP64, "transfer64"), (sc.MIXED, "transfer32")):
+        solver.profile((1 << sc.FAM_TRANSFER64) | (1 << sc.FAM_TRANSFER32))
+        try:
+            _, info = solver.solve_grid(st, k, sc.options(max_iter=5000, tol=1e-8, precision=precision))
+            got = solver.profile_read()[name]
+        finally:
+            solver.profile(0)
+        n, c, t = info["parts"]
+        s = 8 if precision == sc.FP64 else 4
+        assert got["launches"] % 4 == 0
+        a_cycle = got["bytes"] / (got["launches"] // 4)
+        q, rest = divmod(a_cycle - 4 * n - s * (18 * n + 12 * c + 42 * c + 18 * c + 12 * t), 72 * s)
+        assert c % 12 != 0  # else q would be whole without the smoothing's 42 c too
+        assert rest == 0 and c <= q <= c * t
+        blocks.append(q)
+    assert blocks[0] == blocks[1]
