@@ -1,4 +1,9 @@
 """Shared test helpers: synthetic pieces, their oracle lattices and loads."""
+import os
+import subprocess
+import sys
+import textwrap
+
 import numpy as np
 
 import statics_cuda as sc
@@ -30,3 +35,14 @@ def rel(a, b):
 def lattice_dict(ex, level=0):
     return dict(x=ex["x"], held=ex["held"], around=ex["around"], bi=ex["bi"], bj=ex["bj"], p=ex["p"], n=ex["n"],
                 a=ex["a"], d=ex["d"], e=ex["e"], g=ex["g"], level=level)
+
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+def run_script(script, *args, env=None):
+    """`script` in a process of its own (its end ends its device context too)."""
+    paths = [ROOT, os.path.join(ROOT, "parallax-world_b200"), os.path.join(ROOT, "tests"), os.environ.get("PYTHONPATH", "")]
+    done = subprocess.run([sys.executable, "-c", textwrap.dedent(script), *args], capture_output=True, text=True,
+                          timeout=600, env=dict(os.environ, PYTHONPATH=os.pathsep.join(filter(None, paths)), **(env or {})))
+    assert done.returncode == 0, done.stderr[-2000:]

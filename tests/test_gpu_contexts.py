@@ -1,26 +1,14 @@
 """What a process keeps beside a solver context must hold for every device, context and thread:
 kernels' shared-memory limits, which the runtime keeps a device context (one a device)."""
-import os
 import subprocess
-import sys
-import textwrap
 
 import pytest
 
 import statics_cuda as sc
 
+from helpers import run_script
+
 pytestmark = pytest.mark.gpu
-
-ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-
-
-def run_script(script, *args, env=None):
-    """`script` in a process of its own (its end ends its device context too)."""
-    paths = [ROOT, os.path.join(ROOT, "parallax-world_b200"), os.path.join(ROOT, "tests")]
-    done = subprocess.run([sys.executable, "-c", textwrap.dedent(script), *args], capture_output=True, text=True,
-                          timeout=600, env=dict(os.environ, PYTHONPATH=os.pathsep.join(paths), **(env or {})))
-    assert done.returncode == 0, done.stderr[-2000:]
-
 
 TWICE = """
     import ctypes, sys
