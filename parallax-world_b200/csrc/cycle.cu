@@ -134,7 +134,6 @@ static void cycle(Context& ctx, Batch& b, int l, const T* r, T* z, const int32_t
         const int32_t* skip = L.top_h.empty() ? nullptr : L.top_of_part.get();
         T* x = VX<T>(L).get();
         T* left = VL<T>(L).get();
-        bool mf = l == 0 && L.matrix_free;
         double vb = (double)sizeof(T) * 6.0 * (double)L.n;
         // x = step D^-1 r (bodies.rs:386), and any further sweeps
         if (l == 0) {
@@ -142,9 +141,7 @@ static void cycle(Context& ctx, Batch& b, int l, const T* r, T* z, const int32_t
             jacobi<T>(ctx, L.n, INV<T>(L), r, x, L.step.get(), piece, skip, done);
         }
         for (int sweep = 1; sweep < b.sweeps; sweep++) {
-            if (mf) {
-                level0_smooth<T>(ctx, b, r, x, left, done);
-            } else {
+            {
                 ProfScope ps(ctx, fam_of<T>(SC_FAM_SPMV64), spmv_bytes<T>(L, 3) + vb + 36.0 * sizeof(T) * L.n);
                 spmv<T>(ctx, SPMV_RES_SMOOTH, L.n, L.rowptr.get(), L.col.get(), VAL<T>(L), x, r, left, INV<T>(L),
                         L.step.get(), piece, skip, done, L.nnzb);
@@ -152,9 +149,7 @@ static void cycle(Context& ctx, Batch& b, int l, const T* r, T* z, const int32_t
             SC_CK(cudaMemcpyAsync(x, left, 6 * L.n * sizeof(T), cudaMemcpyDeviceToDevice, ctx.stream));
         }
         // left = r - K x (bodies.rs:387)
-        if (mf) {
-            stencil_residual<T>(ctx, b, x, r, left, skip, done);
-        } else {
+        {
             ProfScope ps(ctx, fam_of<T>(SC_FAM_SPMV64), spmv_bytes<T>(L, 3));
             spmv<T>(ctx, SPMV_RES, L.n, L.rowptr.get(), L.col.get(), VAL<T>(L), x, r, left, nullptr, nullptr,
                     piece, skip, done, L.nnzb);
@@ -176,20 +171,14 @@ static void cycle(Context& ctx, Batch& b, int l, const T* r, T* z, const int32_t
         }
         // z = x + step D^-1 (r - K x) (bodies.rs:396-401), after any further sweeps
         for (int sweep = 1; sweep < b.sweeps; sweep++) {
-            if (mf) {
-                level0_smooth<T>(ctx, b, r, x, left, done);
-            } else {
+            {
                 ProfScope ps(ctx, fam_of<T>(SC_FAM_SPMV64), spmv_bytes<T>(L, 3) + vb + 36.0 * sizeof(T) * L.n);
                 spmv<T>(ctx, SPMV_RES_SMOOTH, L.n, L.rowptr.get(), L.col.get(), VAL<T>(L), x, r, left, INV<T>(L),
                         L.step.get(), piece, skip, done, L.nnzb);
             }
             SC_CK(cudaMemcpyAsync(x, left, 6 * L.n * sizeof(T), cudaMemcpyDeviceToDevice, ctx.stream));
         }
-        if (mf) {
-            stencil_residual<T>(ctx, b, x, r, left, skip, done);
-            ProfScope ps(ctx, fam_of<T>(SC_FAM_SMOOTH64), 3 * vb + 36.0 * sizeof(T) * L.n);
-            jacobi_add<T>(ctx, L.n, INV<T>(L), left, x, z, L.step.get(), piece, skip, done);
-        } else {
+        {
             ProfScope ps(ctx, fam_of<T>(SC_FAM_SPMV64), spmv_bytes<T>(L, 3) + vb + 36.0 * sizeof(T) * L.n);
             spmv<T>(ctx, SPMV_RES_SMOOTH, L.n, L.rowptr.get(), L.col.get(), VAL<T>(L), x, r, z, INV<T>(L),
                     L.step.get(), piece, skip, done, L.nnzb);
@@ -845,7 +834,6 @@ static int64_t pcg(Context& ctx, Batch& b, const V* rhs, S* x, V* r, V* z, V* p,
         // individual kernels (profiling) launches them one by one instead.
         bool use_graph = ctx.prof.mask == 0 && graphs_enabled();
         if (use_graph) {
-            ensure_partial(ctx, L);
             // first choice: the iterations loop on the device, a graph whose conditional
             // WHILE node replays the iteration until every piece is done (or `chunk` ran)
             const int64_t l0 = g_launches.load();

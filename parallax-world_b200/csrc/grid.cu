@@ -959,8 +959,6 @@ void stencil_residual(Context& ctx, const Batch& b, const T* x, const T* r, T* y
 }
 template void stencil_residual<double>(Context&, const Batch&, const double*, const double*, double*, const int32_t*,
                                        const int32_t*);
-template void stencil_residual<float>(Context&, const Batch&, const float*, const float*, float*, const int32_t*,
-                                      const int32_t*);
 
 // Level 0's half of a V-cycle on the way up (bodies.rs:386-390), matrix-free:
 //   x = w D^-1 r;  left = r - K x;  t = D^-1 left;  u = left - w K t;  rc = P0' u

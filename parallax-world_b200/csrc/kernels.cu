@@ -354,30 +354,6 @@ __global__ void k_jacobi(int64_t n, const T* __restrict__ inv, const T* __restri
     st6<T>(x + 6 * k, o);
 }
 
-template <class T>
-__global__ void k_jacobi_add(int64_t n, const T* __restrict__ inv, const T* __restrict__ left, const T* __restrict__ x,
-                             T* __restrict__ z, const double* __restrict__ step, const int32_t* __restrict__ piece,
-                             const int32_t* __restrict__ skip_row, const int32_t* __restrict__ done) {
-    int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    if (skip_row && skip_row[k]) return;
-    int p = piece ? piece[k] : 0;
-    if (done && done[p]) return;
-    T lv[6], xv[6], o[6];
-    ld6<T>(left + 6 * k, lv);
-    ld6<T>(x + 6 * k, xv);
-    T st = (T)step[p];
-    const T* d = inv + 36 * k;
-#pragma unroll
-    for (int i = 0; i < 6; i++) {
-        T s = T(0);
-#pragma unroll
-        for (int c = 0; c < 6; c++) s = fma(d[6 * i + c], lv[c], s);
-        o[i] = xv[i] + st * s;
-    }
-    st6<T>(z + 6 * k, o);
-}
-
 // z_i = sum over j of A[j][i] r_j in the order of j, FP64, for the 32 rows i from i0 on. What
 // bounds it is that chain and the loads it waits for (a warp alone gets one load in some 55
 // cycles), so 32 rows are a block whose eight warps bring TOP_TILE values of j to shared
@@ -544,14 +520,6 @@ void jacobi(Context& ctx, int64_t n, const T* inv, const T* r, T* x, const doubl
 }
 
 template <class T>
-void jacobi_add(Context& ctx, int64_t n, const T* inv, const T* left, const T* x, T* z, const double* step,
-                const int32_t* piece, const int32_t* skip_row, const int32_t* done) {
-    if (n <= 0) return;
-    k_jacobi_add<T><<<grid_for(n, 256), 256, 0, ctx.stream>>>(n, inv, left, x, z, step, piece, skip_row, done);
-    SC_LAUNCH_CK();
-}
-
-template <class T>
 void top_solve(Context& ctx, const Level& L, const T* r, T* z, const int32_t* done) {
     if (L.top_h.empty()) return;
     int64_t maxn = 0;
@@ -628,8 +596,6 @@ void seg_dot(Context& ctx, const Level& L, const double* a, const double* b, dou
                           const T*, const double*, const int32_t*, const int32_t*, const int32_t*, int64_t, T*);   \
     template void jacobi<T>(Context&, int64_t, const T*, const T*, T*, const double*, const int32_t*,              \
                             const int32_t*, const int32_t*);                                                       \
-    template void jacobi_add<T>(Context&, int64_t, const T*, const T*, const T*, T*, const double*, const int32_t*, \
-                                const int32_t*, const int32_t*);                                                   \
     template void top_solve<T>(Context&, const Level&, const T*, T*, const int32_t*);                             \
     template void seg_dot_t<T>(Context&, const Level&, const T*, const T*, double*);
 SC_INST(double)

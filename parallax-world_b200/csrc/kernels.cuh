@@ -238,10 +238,6 @@ void spmv(Context& ctx, int mode, int64_t nrows, const int64_t* rowptr, const in
 template <class T>
 void jacobi(Context& ctx, int64_t n, const T* inv, const T* r, T* x, const double* step, const int32_t* piece,
             const int32_t* skip_row, const int32_t* done);
-// z = x + step D^-1 left (the post-smoothing step, bodies.rs:396-401)
-template <class T>
-void jacobi_add(Context& ctx, int64_t n, const T* inv, const T* left, const T* x, T* z, const double* step,
-                const int32_t* piece, const int32_t* skip_row, const int32_t* done);
 template <class T>
 void top_solve(Context& ctx, const Level& L, const T* r, T* z, const int32_t* done);
 // out[p] = sum over piece p's parts of a.b (6 values a part), deterministic.
