@@ -512,18 +512,17 @@ __device__ __forceinline__ int own_entry(uint32_t c) {
 // five blocks would spill), three in FP64 (shared memory allows three).
 template <class T, int MODE, int TH>
 constexpr int brick_min_blocks() {
-    return TH > BRICK_THREADS ? 1 : sizeof(T) == 8 ? 3 : (MODE == ST_RES_JAC || MODE == ST_PROLONG || MODE == ST_SMOOTH) ? 4 : 5;
+    constexpr bool factor = MODE == ST_RES_JAC || MODE == ST_PROLONG || MODE == ST_SMOOTH;
+    return TH > BRICK_THREADS ? 1 : sizeof(T) == 8 ? 3 : factor ? 4 : 5;
 }
 
 // Level 0 applied over bricks, one thread block a brick (see the file's head). The same
 // epilogues as grid.cu's k_stencil: y = Kx, r - Kx, ... (ST_* in level0.cuh).
 template <class T, int MODE, int TH>
-__global__ void __launch_bounds__(TH, brick_min_blocks<T, MODE, TH>()) k_brick_stencil(BrickView v, const T* __restrict__ x,
-                                                                 const T* __restrict__ r, T* __restrict__ y,
-                                                                 T* __restrict__ y2, T s,
-                                                                 const double* __restrict__ step,
-                                                                 const int32_t* __restrict__ skip_row,
-                                                                 const int32_t* __restrict__ done) {
+__global__ void __launch_bounds__(TH, brick_min_blocks<T, MODE, TH>())
+    k_brick_stencil(BrickView v, const T* __restrict__ x, const T* __restrict__ r, T* __restrict__ y,
+                    T* __restrict__ y2, T s, const double* __restrict__ step, const int32_t* __restrict__ skip_row,
+                    const int32_t* __restrict__ done) {
     extern __shared__ __align__(16) unsigned char brick_sm[];
     T* box = reinterpret_cast<T*>(brick_sm);
     float* kbox = reinterpret_cast<float*>(box + 6 * NBOX);
@@ -956,8 +955,8 @@ void brick_stencil(Context& ctx, const Batch& b, const T* x, const T* r, T* y, T
     constexpr size_t smem = brick_smem<T>();
     auto go = [&](auto kernel, int threads) {
         ctx.shared_most(kernel, smem);
-        kernel<<<(unsigned)K.n_bricks, threads, smem, ctx.stream>>>(view_of(K), x, r, y, y2, (T)b.grid.s, step, skip_row,
-                                                                   done);
+        kernel<<<(unsigned)K.n_bricks, threads, smem, ctx.stream>>>(view_of(K), x, r, y, y2, (T)b.grid.s, step,
+                                                                   skip_row, done);
         SC_LAUNCH_CK();
     };
     if (K.n_bricks <= BRICK_FEW)

@@ -362,14 +362,15 @@ __global__ void __launch_bounds__(RED_LANES) k_dots_beta(Chunks ch, CgScalars s,
     atomicAdd(s.ndone, 1);
 }
 
-// x += alpha p, p = z + beta p (bodies.rs:357-369), eight blocks a chunk. On a device-side loop (count not
-// null) it also sets the loop's condition: go on while a piece is not done and fewer than
-// `chunk` iterations ran since the launch (count is zeroed before each launch; any value it
-// holds ends the loop within chunk + 1 iterations).
+// x += alpha p, p = z + beta p (bodies.rs:357-369), eight blocks a chunk. On a device-side
+// loop (count not null) it also sets the loop's condition: go on while a piece is not done and
+// fewer than `chunk` iterations ran since the launch (count is zeroed before each launch; any
+// value it holds ends the loop within chunk + 1 iterations).
 template <class Z>
 __global__ void __launch_bounds__(256) k_update_xp(Chunks ch, CgScalars s, double* __restrict__ x,
-                                                   double* __restrict__ p, const Z* __restrict__ z, cudaGraphConditionalHandle h, int np,
-                                                  uint32_t* __restrict__ count, uint32_t chunk) {
+                                                   double* __restrict__ p, const Z* __restrict__ z,
+                                                   cudaGraphConditionalHandle h, int np,
+                                                   uint32_t* __restrict__ count, uint32_t chunk) {
     if (count && blockIdx.x == 0 && threadIdx.x == 0) {
         const uint32_t n = *count + 1u;
         *count = n;

@@ -964,7 +964,8 @@ template void stencil_residual<double>(Context&, const Batch&, const double*, co
 //   x = w D^-1 r;  left = r - K x;  t = D^-1 left;  u = left - w K t;  rc = P0' u
 // (P' = P0' (I - w K D^-1), P = (I - w D^-1 K) P0, bodies.rs:238-247).
 template <class T>
-void level0_down(Context& ctx, const Batch& b, const T* r, T* x, T* left, T* t, T* u, T* rc, T* xc, const int32_t* done) {
+void level0_down(Context& ctx, const Batch& b, const T* r, T* x, T* left, T* t, T* u, T* rc, T* xc,
+                 const int32_t* done) {
     const Grid0& g = b.grid;
     const Level& L = b.levels[0];
     const Level& C = b.levels[1];
@@ -992,9 +993,9 @@ void level0_down(Context& ctx, const Batch& b, const T* r, T* x, T* left, T* t, 
         ProfScope ps(ctx, sizeof(T) == 8 ? SC_FAM_TRANSFER64 : SC_FAM_TRANSFER32, vb + (double)sizeof(T) * 3 * L.n +
                      (double)sizeof(T) * 6 * C.n + jac);
         const T* rv = sizeof(T) == 8 ? (const T*)L.mf_r.get() : (const T*)L.mf_r32.get();
+        const T* inv = sizeof(T) == 8 ? (const T*)C.inv.get() : (const T*)C.inv32.get();
         k_p0t<T><<<grid_for(C.n, 128), 128, 0, ctx.stream>>>(C.n, L.mem_off.get(), L.mem.get(), rv, u, rc,
-                                                             b.npieces == 1 ? nullptr : C.piece.get(), done,
-                                                             sizeof(T) == 8 ? (const T*)C.inv.get() : (const T*)C.inv32.get(),
+                                                             b.npieces == 1 ? nullptr : C.piece.get(), done, inv,
                                                              C.step.get(), xc);
         SC_LAUNCH_CK();
     }
@@ -1026,7 +1027,8 @@ void level0_up(Context& ctx, const Batch& b, const T* r, T* x, T* e, const T* zc
 template <class T>
 void level0_smooth(Context& ctx, const Batch& b, const T* r, const T* x, T* z, const int32_t* done) {
     const Level& L = b.levels[0];
-    launch_stencil<T, ST_SMOOTH>(ctx, b, x, r, z, nullptr, L.step.get(), L.top_h.empty() ? nullptr : L.top_of_part.get(), done, 3);
+    const int32_t* skip = L.top_h.empty() ? nullptr : L.top_of_part.get();
+    launch_stencil<T, ST_SMOOTH>(ctx, b, x, r, z, nullptr, L.step.get(), skip, done, 3);
 }
 template void level0_smooth<double>(Context&, const Batch&, const double*, const double*, double*, const int32_t*);
 template void level0_smooth<float>(Context&, const Batch&, const float*, const float*, float*, const int32_t*);

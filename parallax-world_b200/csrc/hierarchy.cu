@@ -601,10 +601,10 @@ __global__ void __launch_bounds__(32 * KP0_WARPS) k_kp0(int64_t n, K0View k0, co
                 who &= who - 1u;
                 const TB* bb = B + 36 * (int64_t)entry[w][s][e] + c;
                 double bc[6];
-    #pragma unroll
+#pragma unroll
                 for (int j = 0; j < 6; j++) bc[j] = (double)bb[6 * j];
                 const double2* A = reinterpret_cast<const double2*>(blocks[w] + 36 * e);
-    #pragma unroll
+#pragma unroll
                 for (int r = 0; r < 6; r++) {
                     const double2 a0 = A[3 * r], a1 = A[3 * r + 1], a2 = A[3 * r + 2];
                     double v = 0.0;
@@ -618,7 +618,7 @@ __global__ void __launch_bounds__(32 * KP0_WARPS) k_kp0(int64_t n, K0View k0, co
                 }
                 if (!who) {
                     TO* o = out + 36 * (q0 + s) + c;
-    #pragma unroll
+#pragma unroll
                     for (int r = 0; r < 6; r++) {
                         o[6 * r] = (TO)acc[r];
                         acc[r] = 0.0;

@@ -189,10 +189,9 @@ struct BEntry {
 // the registers are capped at three blocks an SM: the setup of a 128^3 piece spends 62.9 ms
 // here, for 69.4 with 8-byte accesses, and 66.4 without the cap.
 template <int MODE, int TH, bool AREG>
-__global__ void __launch_bounds__(TH, TH != RP_THREADS ? 9 : AREG ? 2 : 3) k_rows_fill(int64_t nrows, RowArgs a, const int64_t* __restrict__ first,
-                                                           const int64_t* __restrict__ crow,
-                                                           int32_t* __restrict__ ccol, double* __restrict__ cval,
-                                                           int S, int nwmax, int meta) {
+__global__ void __launch_bounds__(TH, TH != RP_THREADS ? 9 : AREG ? 2 : 3)
+    k_rows_fill(int64_t nrows, RowArgs a, const int64_t* __restrict__ first, const int64_t* __restrict__ crow,
+                int32_t* __restrict__ ccol, double* __restrict__ cval, int S, int nwmax, int meta) {
     extern __shared__ __align__(16) double smem[];
     constexpr int NG = TH / 6;  // groups of six threads
     __shared__ typename MetaScan<TH>::TempStorage scan;

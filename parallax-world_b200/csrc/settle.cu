@@ -172,8 +172,7 @@ void drop_unheld(Context& c, const DeviceLattice& D, const uint8_t* alive, uint8
 }
 
 // the motions under the weights, the bonds' forces and their use of the bonds' strengths, for
-// the given alive /
-// gone flags (device); the solve's status
+// the given alive and gone flags (device); the solve's status
 sc_status round_used(Context& c, const sc_lattice& L, const DeviceLattice& D, const uint8_t* alive_d,
                      const uint8_t* gone_d, const sc_options& opt, double* used_d, sc_solve_info* info, double& work) {
     cudaStream_t st = c.stream;
