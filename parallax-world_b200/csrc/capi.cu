@@ -395,6 +395,7 @@ sc_status sc_create(int32_t device, sc_context** out) {
     auto* ctx = new sc_context;
     ctx->c.device = device;
     sc_status s = guarded(ctx, [&] {
+        SC_CK(cudaDeviceGetAttribute(&ctx->c.sms, cudaDevAttrMultiProcessorCount, device));
         SC_CK(cudaStreamCreateWithFlags(&ctx->c.stream, cudaStreamNonBlocking));
         cudaMemPool_t pool;
         SC_CK(cudaDeviceGetDefaultMemPool(&pool, device));

@@ -1009,11 +1009,10 @@ void measure_on_device(Context& ctx, CellBatch& cb, int64_t fine_bonds, double s
     ocount.alloc((size_t)ncells, st, &ctx.mem);
     const size_t smem = sizeof(CellSmem);
     SC_CK(cudaFuncSetAttribute(k_gather_cells, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int sms = 0, per = 0;
-    SC_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx.device));
+    int per = 0;
     SC_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_gather_cells, GF_THREADS, smem));
     require(per > 0, SC_CUDA, "the cell measurement does not fit on an SM");
-    const int grid = std::min(ncells, sms * per);
+    const int grid = std::min(ncells, ctx.sms * per);
     scratch.alloc((size_t)grid * GF_MAXM * GF_MAXB * 3, st, &ctx.mem);
     CellBatchView v{};
     v.ncells = ncells;

@@ -1387,7 +1387,7 @@ static bool coarsen(Context& ctx, Batch& b, int l, int octree_level, const sc_op
     const K0View k0 = k0_view(b, F);
     const bool virt = k0.desc != nullptr;  // level-0 blocks made from the cell template
     if (virt)
-        k_num_P<true><<<std::min(grid_for(n, 8), 148u * 5u), 256, 0, st>>>(
+        k_num_P<true><<<std::min(grid_for(n, 8), ctx.sms * 5u), 256, 0, st>>>(
             n, F.rowptr.get(), F.col.get(), nullptr, k0, F.up.get(), rvec.get(), F.inv.get(), F.step.get(),
             F.piece.get(), F.prow.get(), F.pcol.get(), F.pval.get());
     else
@@ -1480,7 +1480,7 @@ static bool coarsen(Context& ctx, Batch& b, int l, int octree_level, const sc_op
         kcnt.alloc(n + 1, st, ms);
         kprow.alloc(n + 1, st, ms);
         SC_CK(cudaMemsetAsync(kcnt.get() + n, 0, sizeof(int64_t), st));
-        const unsigned nb = std::min(grid_for(n, KP0_WARPS), 148u * 40u);
+        const unsigned nb = std::min(grid_for(n, KP0_WARPS), ctx.sms * 40u);
         k_kp0<false, double, double><<<nb, 32 * KP0_WARPS, 0, st>>>(n, k0, F.rowptr.get(), F.col.get(), F.prow.get(),
                                                                    F.pcol.get(), F.up.get(), kcnt.get(), nullptr,
                                                                    nullptr, nullptr, nullptr);

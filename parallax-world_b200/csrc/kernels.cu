@@ -464,14 +464,8 @@ void launch_split(Context& ctx, int mode, int64_t nrows, const int64_t* rowptr, 
 // Warps a row: half a warp (0) where rows average under 12 blocks; one, unless the rows
 // are too few to fill the device twice over and each warp would still stream 16 or more
 // blocks (doubling up to 32).
-static int warps_per_row(int64_t nrows, int64_t nnz) {
-    static const int sms = [] {  // once (thread-safe)
-        int dev = 0, v = 0;
-        SC_CK(cudaGetDevice(&dev));
-        SC_CK(cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev));
-        return v;
-    }();
-    const int64_t target = (int64_t)sms * 64;  // two waves of 32 warps an SM
+static int warps_per_row(const Context& ctx, int64_t nrows, int64_t nnz) {
+    const int64_t target = (int64_t)ctx.sms * 64;  // two waves of 32 warps an SM
     const int64_t avg = nnz / std::max<int64_t>(nrows, 1);
     if (avg < 12) return 0;
     int w = 1;
@@ -484,7 +478,7 @@ void spmv(Context& ctx, int mode, int64_t nrows, const int64_t* rowptr, const in
           const T* r, T* y, const T* inv, const double* step, const int32_t* piece, const int32_t* skip_row,
           const int32_t* done, int64_t nnz, T* y2) {
     if (nrows <= 0) return;
-    const int wpr = nnz > 0 ? warps_per_row(nrows, nnz) : 1;
+    const int wpr = nnz > 0 ? warps_per_row(ctx, nrows, nnz) : 1;
     auto split = [&](auto launch) {
         launch(ctx, mode, nrows, rowptr, col, val, x, r, y, inv, step, piece, skip_row, done, y2);
     };

@@ -70,7 +70,8 @@ struct Chunks {
     uint32_t* arrived = nullptr;           // SPLIT: per chunk, warps that arrived (zero between kernels)
     uint32_t* ticket = nullptr;            // per piece, chunks that arrived (zero between kernels)
 };
-// A block a chunk fills the device from about four blocks an SM on.
+// A block a chunk fills the device from about four blocks an SM on (148 of them; where the
+// line lies changes no sum's order).
 constexpr int64_t RED_WHOLE = 592;
 inline bool red_split(int64_t nchunks) { return nchunks < RED_WHOLE; }
 inline unsigned red_grid(int64_t nchunks) { return (unsigned)(red_split(nchunks) ? 8 * nchunks : nchunks); }

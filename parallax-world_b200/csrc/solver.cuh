@@ -287,6 +287,7 @@ struct ProfScope {
 
 struct Context {
     int device = 0;
+    int sms = 0;  // the device's SMs
     Profiler prof;
     cudaStream_t stream = nullptr;
     MemStats mem;
