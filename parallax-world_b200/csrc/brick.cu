@@ -58,9 +58,9 @@ constexpr int NNB = 13;                             // the brick and the twelve 
 constexpr int HKX = BY * BZ, HKY = BX * BZ, HKZ = BX * BY, HK = HKX + HKY + HKZ;  // halo cells
 // Threads a brick: 256, two parts a thread in turn, where several bricks share an SM; 512
 // where the bricks are no more than the SMs, and a brick's own time, not their throughput, is
-// what a stencil takes. The iterations, 256 and 512 threads: 8^3 (2 bricks) 2.86 and 2.85 ms,
-// 16^3 (16) 5.73 and 5.61, 24^3 (54) 6.38 and 6.23, 32^3 (122) 8.64 and 8.45 in FP64; mixed
-// 2.46 and 2.42, 4.57 and 4.47, 5.13 and 4.98, 6.03 and 5.85.
+// what a stencil takes. The iterations, 256 and 512 threads: 8^3 (at most 2 bricks) 2.86 and 2.85
+// ms, 16^3 (16) 5.73 and 5.61, 24^3 (54) 6.38 and 6.23, 32^3 (128) 8.64 and 8.45 in FP64;
+// mixed 2.46 and 2.42, 4.57 and 4.47, 5.13 and 4.98, 6.03 and 5.85.
 constexpr int BRICK_THREADS = 256, BRICK_THREADS_FEW = 512;
 static_assert(NSLOT < 4096, "slot indices take 12 bits (halo_table)");
 static_assert(BRICK_THREADS >= BCELLS, "the k box is filled a cell a thread");
